@@ -27,11 +27,13 @@
 // fPre of the PSM update.  The FP32 form collides two cells per thread in packed
 // f32x2 arithmetic (collide_segment_pairs) and recomputes the particle surface
 // velocity of its solid cells from the owner particle's row of the float table
-// (no per-cell velocity field); the FP64 form one cell per thread in double,
-// BGK and solid correction in one pass (collide_cell_fp64; with a body force
-// collide_cell), with the velocity setValues stored.  The same
+// (no per-cell velocity field); the FP64 form one cell per thread, BGK and solid
+// correction in one pass in 64-bit fixed point (cell_fixed.h; a cell outside its range
+// in double, collide_cell_fp64; with a body force collide_cell in double), with the
+// velocity setValues stored.  The same
 // kernel steps many independent domains in one launch (batch mode).
 #include "lbdem_internal.h"
+#include "cell_fixed.h"
 
 #include <cstddef>
 #include <type_traits>
@@ -659,9 +661,15 @@ template <typename T>
 __device__ __forceinline__ void arm_terms(T dx, T dy, T dz, const Geom& g, T Fx, T Fy, T Fz, T (&v)[6]) {
     const int nx = g.nx, ny = g.ny, nz = g.nz;
     const int hx = nx / 2, hy = ny / 2, hz = nz / 2;
-    if (dx > T(hx)) dx -= T(nx); else if (dx < T(-hx)) dx += T(nx);
-    if (dy > T(hy)) dy -= T(ny); else if (dy < T(-hy)) dy += T(ny);
-    if (dz > T(hz)) dz -= T(nz); else if (dz < T(-hz)) dz += T(nz);
+    // doubles are compared as integers (same order for a non-negative bound), off the
+    // FP64 pipe
+    auto above = [](T d, int h) -> bool {
+        if constexpr (sizeof(T) == 8) return __double_as_longlong(d) > __double_as_longlong((double)h);
+        else return d > T(h);
+    };
+    if (above(dx, hx)) dx -= T(nx); else if (above(-dx, hx)) dx += T(nx);
+    if (above(dy, hy)) dy -= T(ny); else if (above(-dy, hy)) dy += T(ny);
+    if (above(dz, hz)) dz -= T(nz); else if (above(-dz, hz)) dz += T(nz);
     v[0] = Fx; v[1] = Fy; v[2] = Fz;
     v[3] = dy * Fz - dz * Fy;
     v[4] = -dx * Fz + dz * Fx;
@@ -864,6 +872,8 @@ struct alignas(16) WarpStage {
     unsigned long long lead[2];   // unaligned rows: lead elements of row i at bits 2i, voxel row at bits 38,
                                   // surface-velocity row d at bits 40 + 2d
     unsigned long long bar[2];
+    // stages shared by two warps: buffer b read by both; its halo elements in place
+    unsigned long long empty[2], halo[2];
 };
 
 static_assert(sizeof(WarpStage<float, true>) % 16 == 0 && sizeof(WarpStage<float, false>) % 16 == 0 &&
@@ -875,12 +885,12 @@ static_assert(offsetof(WarpStage<float>, vox) % 16 == 0 && offsetof(WarpStage<fl
 
 // The per-CTA tables behind the warps' stages.
 template <typename T, bool STAGE_UP>
-__device__ __forceinline__ unsigned char* cta_tables() {
+__device__ __forceinline__ unsigned char* cta_tables(int stages = WARPS) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
-    return smem_raw + WARPS * sizeof(WarpStage<T, STAGE_UP>);
+    return smem_raw + stages * sizeof(WarpStage<T, STAGE_UP>);
 }
 
-__device__ __forceinline__ constexpr int row_slot(int dx, int dy) { return 3 * (dx + 1) + dy + 1; }
+__host__ __device__ constexpr int row_slot(int dx, int dy) { return 3 * (dx + 1) + dy + 1; }
 
 __device__ __forceinline__ uint32_t smem_addr(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
 
@@ -890,6 +900,9 @@ __device__ __forceinline__ void mbar_init(unsigned long long* bar, uint32_t coun
 __device__ __forceinline__ void mbar_arrive_expect_tx(unsigned long long* bar, uint32_t bytes) {
     asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smem_addr(bar)), "r"(bytes)
                  : "memory");
+}
+__device__ __forceinline__ void mbar_arrive(unsigned long long* bar) {
+    asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_addr(bar)) : "memory");
 }
 __device__ __forceinline__ bool mbar_try_wait(unsigned long long* bar, uint32_t parity) {
     uint32_t ok;
@@ -1075,6 +1088,7 @@ __device__ __forceinline__ T issue_segment(const CollideArgs<T>& a, WarpStage<T,
         }
     }
     const uint32_t total = __reduce_add_sync(FULL, bytes + bytes2);
+    __syncwarp();   // the lanes' geometry writes come before lane 0's arrival
     if (lane == 0) mbar_arrive_expect_tx(&st.bar[b], total);
     __syncwarp();
     if (bytes) bulk_g2s(dst, src, bytes, &st.bar[b]);
@@ -1517,12 +1531,167 @@ __device__ __forceinline__ void collide_segment_pairs(const CollideArgs<float>& 
     }
 }
 
+// ---------------------------------------------------------------------------
+// FP64 form without a body force: one staged cell (lane's cell j of the segment in
+// buffer b), evaluated in fixed point (cell_fixed.h) from the stage and stored.
+// The loop bodies cover the three direction pairs of one axis and run three times
+// (the axes are cycled in between), over values kept in the stage: fully unrolled
+// the update is 5000 instructions, and the warps, each at another place of it, then
+// wait for the instruction cache 80 % of the time.
+// Target row slots of direction q of the three cycles, four bits each.
+__host__ __device__ constexpr unsigned slot_bits(int q) {
+    unsigned v = 0;
+    for (int t = 0; t < 3; ++t) {
+        const int i = fixed::dir_of(t, q);
+        v |= (unsigned)row_slot(cx(i), cy(i)) << (4 * t);
+    }
+    return v;
+}
+
+template <bool ODD, bool PER, bool MIS, bool STAGE_UP>
+struct StagedCell {
+    static constexpr int ROW = WarpStage<double, STAGE_UP>::W;
+    WarpStage<double, STAGE_UP>& st;
+    double* base;         // cell j of direction 0's staged row, without the row's lead
+    double* fo;           // output populations
+    const double* upf;    // surface-velocity field (read directly where it is not staged)
+    unsigned N;           // cells (19 N doubles fit the memory, so N < 2^32)
+    int b, z;
+    size_t c;
+    int zm, zp;           // z - 1 and z + 1 (wrapped; -1 beyond a wall)
+    uint32_t srcrow;
+    unsigned long long lead;
+
+    // the staged value of direction i (c_z = cz), the cell's own place in the stage
+    __device__ __forceinline__ double* at(int i, int cz) const {
+        int off = i * ROW;
+        if (ODD) off -= (PER || ((srcrow >> i) & 1u)) ? cz : 0;
+        if (MIS) off += (int)((lead >> (2 * i)) & 3u);
+        return base + off;
+    }
+    __device__ __forceinline__ double up(int d, int j) const {
+        if (!STAGE_UP) return __ldg(upf + (size_t)d * N + c);
+        const int m = MIS ? (int)((lead >> (40 + 2 * d)) & 3u) : 0;
+        return st.up[b][d][m + j];
+    }
+    // where the post-collision value of direction i (opposite o, target row slot rs) goes
+    __device__ __forceinline__ double* slot(int i, int o, int rs, int cz) const {
+        if (!ODD) return fo + c + (unsigned long long)(unsigned)o * N;
+        const long long r = st.row[b][rs];
+        const int zd = pick(cz, zm, z, zp);
+        if (PER || (r >= 0 && zd >= 0)) return fo + (unsigned long long)(unsigned)i * N + (size_t)(r + zd);
+        return fo + c + (unsigned long long)(unsigned)o * N;
+    }
+};
+
+// The double routine for a cell outside the fixed-point range, out of line.
+template <bool ODD, bool PER, bool MIS, bool STAGE_UP>
+__device__ __noinline__ void collide_cell_double(StagedCell<ODD, PER, MIS, STAGE_UP> s, double omega, double B,
+                                                 double u0, double u1, double u2, double (&F)[3]) {
+    double f[Q];
+#pragma unroll
+    for (int i = 0; i < Q; ++i) f[i] = *s.at(i, cz(i));
+    collide_cell_fp64<true>(f, omega, B, u0, u1, u2, F[0], F[1], F[2]);
+    s.fo[s.c] = f[0];
+#pragma unroll
+    for (int i = 1; i < Q; ++i) *s.slot(i, opp(i), row_slot(cx(i), cy(i)), cz(i)) = f[i];
+}
+
+template <bool ODD, bool PER, bool MIS, bool STAGE_UP>
+__device__ __forceinline__ void collide_cell_staged(const CollideArgs<double>& a, WarpStage<double, STAGE_UP>& st,
+                                                    int b, int j, int z0, uint32_t srcrow, unsigned long long lead,
+                                                    uint32_t w, bool solid, double (&F)[3]) {
+    using fixed::i64;
+    const Geom& g = a.g;
+    const int z = z0 + j;
+    const StagedCell<ODD, PER, MIS, STAGE_UP> s{st,
+                                                &st.f[b][0][WarpStage<double>::V + j],
+                                                a.fo,
+                                                a.up,
+                                                (unsigned)g.N,
+                                                b,
+                                                z,
+                                                (size_t)st.row[b][row_slot(0, 0)] + z,
+                                                wrap_minus(z, g.nz, PER ? 1 : g.per[2]),
+                                                wrap_plus(z, g.nz, PER ? 1 : g.per[2]),
+                                                srcrow,
+                                                lead};
+    // the cell's unit
+    double* const p0 = s.at(0, 0);
+    int e = __double2hiint(*p0) & 0x7ff00000;
+#pragma unroll
+    for (int i = 1; i < Q; ++i) e = max(e, __double2hiint(*s.at(i, cz(i))) & 0x7ff00000);
+    e >>= 20;
+    double B = 0.0, u0 = 0.0, u1 = 0.0, u2 = 0.0;
+    const int n = min((int)(w & VOX_NMASK), 125);
+    if (n > 0) {
+        B = __ldg(a.btab + n);
+        u0 = s.up(0, j);
+        u1 = s.up(1, j);
+        u2 = s.up(2, j);
+        e = fixed::cell_exponent_up(e, u0, u1, u2);
+    }
+    if (!fixed::fits(e)) {
+        collide_cell_double<ODD, PER, MIS, STAGE_UP>(s, a.omega, B, u0, u1, u2, F);
+        return;
+    }
+    e = max(e, fixed::EMAX_LO);
+    // populations in units (back into the stage), and their sums
+    const i64 X0 = fixed::to_fixed<4>(*p0, e);
+    fixed::Sums sum{X0, {0, 0, 0}};
+    // direction q of cycle a, as in fixed::dir_of, with its c_z and target row slot
+    auto dir = [](int q, int a, int dg) { return q < 2 ? (q == 0 ? 10 : 1) + a : (q == 2 ? 13 : q == 3 ? 4 : q == 4 ? 14 : 5) + dg; };
+    auto dir_z = [](int q, int a) {
+        const int zc = q < 2 ? (a == 2 ? 1 : 0) : (a > 0 ? 1 : 0);
+        return q == 0 || q == 2 || q == 5 ? zc : -zc;
+    };
+    auto dir_row = [](int q, int a) -> int {   // four bits per cycle
+        constexpr unsigned rows[6] = {slot_bits(0), slot_bits(1), slot_bits(2), slot_bits(3), slot_bits(4), slot_bits(5)};
+        return (int)((rows[q] >> (4 * a)) & 15u);
+    };
+#pragma unroll 1
+    for (int t = 0, dg = 0; t < 3; dg = t == 0 ? 4 : 2, ++t) {
+        i64 x[6];
+#pragma unroll
+        for (int q = 0; q < 6; ++q) {
+            double* p = s.at(dir(q, t, dg), dir_z(q, t));
+            x[q] = fixed::to_fixed<4>(*p, e);
+            *reinterpret_cast<i64*>(p) = x[q];
+        }
+        fixed::add_three(sum, x, t == 2);
+    }
+    fixed::Cell cell = fixed::cell_setup(solid, sum.rb, sum.j[0], sum.j[1], sum.j[2], e,
+                                          fixed::relax_of(a.omega), B, u0, u1, u2, F);
+    a.fo[s.c] = fixed::update_rest(solid, cell, X0, e);
+#pragma unroll 1
+    for (int t = 0, dg = 0; t < 3; dg = t == 0 ? 4 : 2, ++t) {
+        const fixed::Three eq = fixed::three_of(cell.eq, t == 2);
+        fixed::Three df{};
+        if (solid) df = fixed::three_of(cell.df, t == 2);
+        fixed::update_three(
+            solid, cell, eq, df,
+            [&](int q) { return *reinterpret_cast<const i64*>(s.at(dir(q, t, dg), dir_z(q, t))); }, e,
+            [&](int q, double v) { *s.slot(dir(q, t, dg), dir(q ^ 1, t, dg), dir_row(q, t), dir_z(q, t)) = v; });
+        fixed::cycle(cell.eq);
+        if (solid) fixed::cycle(cell.df);
+    }
+}
+
+// Warps per stage.  The FP64 form without a body force gives each segment to two
+// warps, one 32-cell pass each: the stages of 8 warps fill the SM's shared memory, and
+// with two warps per scheduler the integer chains of a cell left half of the issue
+// slots empty.  The two take the longer (solid) pass in turn and do not wait for
+// each other at the end of a segment: a buffer is handed back through the stage's
+// `empty` barrier, so the warp with the shorter pass goes on to the next segment.
+template <typename T, bool FORCE>
+__host__ __device__ constexpr int stage_warps() { return sizeof(T) == 8 && !FORCE ? 2 : 1; }
+
 // PER: every axis periodic (no wall cases; shifts and neighbour rows are fixed).
 // MIS: rows not 16-byte aligned (see issue_segment).
 // BATCH: segments of many domains, numbered domain after domain (seg0[d] is
 // the first segment of domain d); every domain has its own CollideArgs.
 template <typename T, bool ODD, bool FORCE, bool PER, bool MIS, bool BATCH>
-__global__ void __launch_bounds__(COLLIDE_BLOCK, sizeof(T) == 4 ? 4 : 2)
+__global__ void __launch_bounds__(COLLIDE_BLOCK, sizeof(T) == 4 ? 4 : 2 * stage_warps<T, FORCE>())
 k_collide_staged(const CollideArgs<T> a1, long long nseg, const CollideArgs<T>* __restrict__ dargs,
                  const int* __restrict__ seg0, int ndom) {
     constexpr int V = WarpStage<T>::V;
@@ -1536,15 +1705,27 @@ k_collide_staged(const CollideArgs<T> a1, long long nseg, const CollideArgs<T>* 
     extern __shared__ __align__(16) unsigned char smem_raw[];
     const int lane = threadIdx.x & 31;
     const int warp = threadIdx.x >> 5;
-    WarpStage<T, STAGE_UP>& st = reinterpret_cast<WarpStage<T, STAGE_UP>*>(smem_raw)[warp];
+    // SW warps share a stage: warp `sub` of group `group`
+    constexpr int SW = stage_warps<T, FORCE>();
+    constexpr int GROUPS = WARPS / SW;
+    const int group = warp / SW, sub = warp % SW;
+    WarpStage<T, STAGE_UP>& st = reinterpret_cast<WarpStage<T, STAGE_UP>*>(smem_raw)[group];
     __shared__ unsigned long long probe[WARPS];   // the test hook's barrier (never completes)
     if (lane == 0) {
-        mbar_init(&st.bar[0], 1);
-        mbar_init(&st.bar[1], 1);
+        if (sub == 0) {
+            mbar_init(&st.bar[0], 1);
+            mbar_init(&st.bar[1], 1);
+            if (SW > 1)
+                for (int q = 0; q < 2; ++q) {
+                    mbar_init(&st.empty[q], SW);
+                    mbar_init(&st.halo[q], 1);
+                }
+        }
         mbar_init(&probe[warp], 1);
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
-    __syncwarp();
+    if (SW > 1) __syncthreads();
+    else __syncwarp();
     bool smap_ok = false;   // the CTA holds a copy of the tag -> slot map (FP32, single lattice)
     if constexpr (smem_tagmap<T, BATCH>()) {
         int* m = reinterpret_cast<int*>(cta_tables<T, STAGE_UP>());
@@ -1560,16 +1741,16 @@ k_collide_staged(const CollideArgs<T> a1, long long nseg, const CollideArgs<T>* 
     }
     const int* sseg0 = nullptr;   // batch: the CTA's copy of seg0 (ndom <= SEG0_SMEM)
     if constexpr (BATCH) {
-        int* m = reinterpret_cast<int*>(cta_tables<T, STAGE_UP>());
+        int* m = reinterpret_cast<int*>(cta_tables<T, STAGE_UP>(GROUPS));
         if (ndom <= SEG0_SMEM) {
             for (int k = threadIdx.x; k < ndom; k += blockDim.x) m[k] = __ldg(seg0 + k);
             sseg0 = m;
         }
         __syncthreads();   // every warp of the CTA reaches it (before any leaves)
     }
-    const long long stride = (long long)gridDim.x * WARPS;
-    long long seg = (long long)blockIdx.x * WARPS + warp;
-    if (seg >= nseg) return;
+    const long long stride = (long long)gridDim.x * GROUPS;
+    long long seg = (long long)blockIdx.x * GROUPS + group;
+    if (seg >= nseg) return;   // both warps of a shared stage
     auto issue = [&](int buf, long long sg) -> T {
         if constexpr (LSU) {
             issue_segment_lsu<T, ODD, PER, STAGE_UP>(a1, st, buf, sg);
@@ -1595,14 +1776,27 @@ k_collide_staged(const CollideArgs<T> a1, long long nseg, const CollideArgs<T>* 
         }
         return issue_segment<T, ODD, MIS, STAGE_UP>(a1, st, buf, sg, 0);
     };
-    T hcur = issue(0, seg);
+    // segment k of the stage (buffer b = k & 1) is issued by warp k % SW, one segment
+    // ahead; with two warps the same warp takes its first (solid) pass
+    T hcur = T(0);
+    if (sub == 0) hcur = issue(0, seg);
     uint32_t phase = 0;   // bit b: parity expected next on buffer b
+    uint32_t ephase = 0;  // the same for the `empty` barriers
     bool first = true;
     int b = 0;
     for (; seg < nseg; seg += stride, b ^= 1) {
         const long long next = seg + stride;
+        const bool lead_warp = SW == 1 || sub == b;
         T hnext = T(0);
-        if (next < nseg) hnext = issue(b ^ 1, next);
+        bool ok = true;
+        if (next < nseg && (SW == 1 || !lead_warp)) {
+            // both warps have left the buffer's last segment (none before the first two)
+            if (SW > 1 && !first) {
+                ok = mbar_wait(&st.empty[b ^ 1], (ephase >> (b ^ 1)) & 1u);
+                ephase ^= 1u << (b ^ 1);
+            }
+            if (SW == 1 || __all_sync(FULL, ok)) hnext = issue(b ^ 1, next);
+        }
         if constexpr (LSU) {
             // this thread's copies of the current segment (all groups but the newest)
             if (next < nseg) cp_wait<1>();
@@ -1610,18 +1804,17 @@ k_collide_staged(const CollideArgs<T> a1, long long nseg, const CollideArgs<T>* 
             __syncwarp();   // and every other lane's
         } else {
             const uint32_t pb = (phase >> b) & 1u;
-            bool ok;
             if (!BATCH && a1.probe_timeout && first) {
                 // test hook: wait on a barrier nothing arrives on, as for a copy that never lands
                 ok = mbar_wait(&probe[warp], 0u, PROBE_WAIT);
-            } else {
+            } else if (ok) {
                 ok = mbar_wait(&st.bar[b], pb);
             }
             phase ^= 1u << b;
             first = false;
             if (__any_sync(FULL, !ok)) {
-                // a copy did not land: report, let this warp's copies in flight land
-                // (both buffers, bounded), leave
+                // a copy did not land (or the stage's other warp has left): report, let the
+                // stage's copies in flight land (both buffers, bounded), leave
                 if (lane == 0) atomicOr(BATCH ? dargs[0].err : a1.err, 0x20u);   // LBDEM_DEVERR_TIMEOUT
                 mbar_wait(&st.bar[b], pb);
                 if (next < nseg) mbar_wait(&st.bar[b ^ 1], (phase >> (b ^ 1)) & 1u);
@@ -1637,7 +1830,7 @@ k_collide_staged(const CollideArgs<T> a1, long long nseg, const CollideArgs<T>* 
         const size_t own = (size_t)st.row[b][row_slot(0, 0)];
         const unsigned long long lead = MIS ? st.lead[b] : 0ull;
         if (MIS && ODD) {
-            if (lane < 10) {
+            if (lane < 10 && lead_warp) {
                 const int i = zdir(lane);
                 if (st.row[b][row_slot(-cx(i), -cy(i))] >= 0) {
                     const int m = (int)((lead >> (2 * i)) & 3u);
@@ -1650,7 +1843,7 @@ k_collide_staged(const CollideArgs<T> a1, long long nseg, const CollideArgs<T>* 
         // Odd phase with walls along z, aligned rows: the halo element of an edge
         // cell is its own slot i (half-way bounce-back).
         if (!MIS && ODD && !PER && !g.per[2] && (z0 == 0 || z0 + len == g.nz)) {
-            if (lane < 10) {
+            if (lane < 10 && lead_warp) {
                 const int i = zdir(lane);
                 if (st.row[b][row_slot(-cx(i), -cy(i))] >= 0) {
                     if (cz(i) > 0 && z0 == 0) st.f[b][i][V - 1] = Fin[(size_t)i * N + own];
@@ -1658,6 +1851,19 @@ k_collide_staged(const CollideArgs<T> a1, long long nseg, const CollideArgs<T>* 
                 }
             }
             __syncwarp();
+        }
+        if constexpr (SW > 1 && ODD && !PER) {
+            // the other warp's cells read the halo elements that the lead warp put in place
+            if (lead_warp) {
+                if (lane == 0) mbar_arrive(&st.halo[b]);
+            } else {
+                ok = mbar_wait(&st.halo[b], (phase >> b & 1u) ^ 1u);   // phase was flipped above
+            }
+            if (__any_sync(FULL, !ok)) {
+                if (lane == 0) atomicOr(BATCH ? dargs[0].err : a1.err, 0x20u);   // LBDEM_DEVERR_TIMEOUT
+                if (next < nseg) mbar_wait(&st.bar[b ^ 1], (phase >> (b ^ 1)) & 1u);
+                return;
+            }
         }
         uint32_t srcrow = 0;   // bit i: source row of direction i lies inside the lattice
         if (ODD && !PER) {
@@ -1674,7 +1880,7 @@ k_collide_staged(const CollideArgs<T> a1, long long nseg, const CollideArgs<T>* 
             // double atomics.  The segment's solid cells are taken first (pass 0
             // holds as many of them as fit): a pass whose warp holds a solid cell
             // runs the solid terms for every lane, so gathering them leaves more
-            // passes on the BGK-only path.  A cell's result does not depend on
+            // passes on the fluid path.  A cell's result does not depend on
             // its pass.
             static_assert(SEGW == 64, "two passes of 32 cells per segment");
             const int vlead = MIS ? (int)((lead >> 38) & 3u) : 0;
@@ -1687,14 +1893,26 @@ k_collide_staged(const CollideArgs<T> a1, long long nseg, const CollideArgs<T>* 
             const int ns0 = __popc(sol0), ns = ns0 + __popc(sol1);
             const int nf0 = __popc(flu0), nf = nf0 + __popc(flu1);
 #pragma unroll 1
-            for (int p = 0; p < 2; ++p) {
+            for (int p = lead_warp ? 0 : 1; p < (lead_warp ? (SW > 1 ? 1 : 2) : 2); ++p) {
                 const int slot = 32 * p + lane;
                 int j = -1;   // the cell this lane takes in pass p
                 if (slot < ns) j = slot < ns0 ? nth_bit(sol0, slot) : 32 + nth_bit(sol1, slot - ns0);
                 else if (slot - ns < nf) j = slot - ns < nf0 ? nth_bit(flu0, slot - ns) : 32 + nth_bit(flu1, slot - ns - nf0);
                 const bool any_solid = ns > 32 * p;   // warp-uniform
                 T v[6] = {T(0), T(0), T(0), T(0), T(0), T(0)};
-                if (j >= 0) {
+                if constexpr (!FORCE) {
+                    if (j >= 0) {
+                        const uint32_t w = st.vox[b][vlead + j];
+                        T Fc[3];
+                        collide_cell_staged<ODD, PER, MIS, STAGE_UP>(a, st, b, j, z0, srcrow, lead, w, any_solid, Fc);
+                        const size_t c = own + z0 + j;
+                        if (a.cf) { a.cf[c] = Fc[0]; a.cf[N + c] = Fc[1]; a.cf[2 * N + c] = Fc[2]; }
+                        if (any_solid) {
+                            const int key = cell_force_terms(a, w, sx, sy, z0 + j, Fc[0], Fc[1], Fc[2], v);
+                            if (key >= 0) add_cell_force(a, key, v);
+                        }
+                    }
+                } else if (j >= 0) {
                     const uint32_t w = st.vox[b][vlead + j];
                     const int z = z0 + j;
                     const size_t c = own + z;
@@ -1714,18 +1932,7 @@ k_collide_staged(const CollideArgs<T> a1, long long nseg, const CollideArgs<T>* 
                         const int m = MIS ? (int)((lead >> (40 + 2 * d)) & 3u) : 0;
                         return st.up[b][d][m + j];
                     };
-                    if constexpr (!FORCE) {
-                        const int n = min((int)(w & VOX_NMASK), 125);
-                        if (any_solid) {
-                            const bool s = n > 0;   // a fluid cell's velocity slot is not read
-                            collide_cell_fp64<true>(f, a.omega, __ldg(a.btab + n), s ? upv(0) : T(0),
-                                                    s ? upv(1) : T(0), s ? upv(2) : T(0), Fx, Fy, Fz);
-                        } else {
-                            collide_cell_fp64<false>(f, a.omega, T(0), T(0), T(0), T(0), Fx, Fy, Fz);
-                        }
-                    } else {
-                        collide_cell<T, FORCE>(a, f, w, [&](int i) { return at(i); }, upv, Fx, Fy, Fz);
-                    }
+                    collide_cell<T, FORCE>(a, f, w, [&](int i) { return at(i); }, upv, Fx, Fy, Fz);
                     if (!ODD) {
 #pragma unroll
                         for (int i = 0; i < Q; ++i) F[(size_t)opp(i) * N + c] = f[i];
@@ -1747,7 +1954,11 @@ k_collide_staged(const CollideArgs<T> a1, long long nseg, const CollideArgs<T>* 
                 }
             }
         }
-        __syncwarp();   // buffer b is free for the segment after next
+        // buffer b is free for the segment after next; writes into it (halo elements,
+        // populations in units) come before the copies that reuse it
+        if constexpr (!LSU) asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+        __syncwarp();
+        if (SW > 1 && lane == 0) mbar_arrive(&st.empty[b]);
         hcur = hnext;
     }
 }
@@ -1755,8 +1966,9 @@ k_collide_staged(const CollideArgs<T> a1, long long nseg, const CollideArgs<T>* 
 template <typename T, bool ODD, bool FORCE, bool PER, bool MIS, bool BATCH>
 cudaError_t launch_staged(const CollideArgs<T>& a, long long nseg, const CollideArgs<T>* dargs,
                           const int* seg0, int ndom, int blocks_per_sm, cudaStream_t s) {
+    constexpr int GROUPS = WARPS / stage_warps<T, FORCE>();   // stages (segments in work) per block
     constexpr size_t smem =
-        WARPS * sizeof(WarpStage<T, stage_up<T, BATCH>()>) + tagmap_bytes<T, BATCH>() + seg0_bytes<BATCH>();
+        GROUPS * sizeof(WarpStage<T, stage_up<T, BATCH>()>) + tagmap_bytes<T, BATCH>() + seg0_bytes<BATCH>();
     if (nseg >= (1LL << 31)) return cudaErrorInvalidValue;   // segment indices are split in 32 bits
     // per device: (resident blocks per SM << 16) | SM count, 0 until first use there
     static std::atomic<int> shape[LBDEM_MAX_DEVICES];
@@ -1783,7 +1995,7 @@ cudaError_t launch_staged(const CollideArgs<T>& a, long long nseg, const Collide
     if (nseg <= 0) return cudaSuccess;
     const int use = (blocks_per_sm > 0 && blocks_per_sm < per_sm) ? blocks_per_sm : per_sm;
     const long long want = (long long)sms * use;
-    const long long blocks = (nseg + WARPS - 1) / WARPS;
+    const long long blocks = (nseg + GROUPS - 1) / GROUPS;
     const unsigned grid = (unsigned)(blocks < want ? blocks : want);
     k_collide_staged<T, ODD, FORCE, PER, MIS, BATCH><<<grid, COLLIDE_BLOCK, smem, s>>>(a, nseg, dargs, seg0, ndom);
     return cudaGetLastError();
