@@ -332,6 +332,9 @@ __device__ __forceinline__ int slice_count_resolve(float dxf, float dyf, float d
 constexpr int VOX_WARPS = 8;                        // warps per block
 constexpr int VOX_THREADS = 32 * VOX_WARPS;
 constexpr int VOX_STAGE = 32;                       // sphere records staged at a time
+// A tile's sphere count and, above it, the arrivals of its warps (at most 8).
+constexpr int TILE_CNT_BITS = 28;
+constexpr unsigned TILE_CNT_MASK = (1u << TILE_CNT_BITS) - 1u;
 constexpr int TOFF_SMEM = 512;                      // batch: domains whose first tiles a CTA keeps
 constexpr uint32_t SETTER_ZERO = 0xffffffffu;       // the cell was set to zero (setToZero)
 constexpr uint32_t SETTER_KEEP = 0xfffffffeu;       // the cell keeps its state (and velocity)
@@ -372,14 +375,14 @@ __device__ __forceinline__ void fold_cell(WarpVox<INIT_VEL>& S, int l, uint32_t 
     if (INIT_VEL && n == 125u) S.defv[l] = S.setter[l];
 }
 
-// Steps 1-3 above for sphere m (float record q in shared memory) on the tile at
-// (X0, Y0, Z0).  Inlined at both sphere sources (an out-of-line routine measured
+// Steps 1-3 above for sphere m (float record q in shared memory) on the x-planes
+// xa..xb of the tile at (X0, Y0, Z0).  Inlined at both sphere sources (an out-of-line routine measured
 // 5 % slower: the call's register saves and restores).
 template <bool INIT_VEL>
 __device__ __forceinline__ void apply_sphere(WarpVox<INIT_VEL>& S, const SphereFast& q, int m,
-                                          const SphereDev* __restrict__ sph, int X0, int Y0, int Z0) {
+                                          const SphereDev* __restrict__ sph, int X0, int Y0, int Z0, int xa, int xb) {
     const int lane = threadIdx.x & 31;
-    const int bx0 = max(q.lo[0] - X0, 0), bx1 = min(q.hi[0] - X0, TILE - 1);
+    const int bx0 = max(q.lo[0] - X0, xa), bx1 = min(q.hi[0] - X0, xb);
     const int by0 = max(q.lo[1] - Y0, 0), by1 = min(q.hi[1] - Y0, TILE - 1);
     const int bz0 = max(q.lo[2] - Z0, 0), bz1 = min(q.hi[2] - Z0, TILE - 1);
     if (bx0 > bx1 || by0 > by1 || bz0 > bz1) return;
@@ -550,7 +553,8 @@ __device__ __forceinline__ void setter_velocity(uint32_t code, const SphereDev* 
     }
 }
 
-// One tile by one warp.  up == nullptr: no surface-velocity field is kept.
+// The x-planes xa..xb of one tile by one warp (parts warps take the tile's slabs).
+// up == nullptr: no surface-velocity field is kept.
 // INIT_VEL: defineVelocity (src/ibCompositeDynamics3D.hh:118-127) with the
 // velocity a fully covered cell holds right after the last sphere covering it.
 template <typename T, bool INIT_VEL>
@@ -558,7 +562,8 @@ __device__ __forceinline__ void voxelize_tile(WarpVox<INIT_VEL>& S, int t, const
                                               const SphereFast* __restrict__ fast, int nsph,
                                               int* __restrict__ tile_cnt, const int* __restrict__ bins,
                                               uint32_t* __restrict__ vox, T* __restrict__ up, T* __restrict__ f,
-                                              int phase, const Geom& g, const OwnerTable& ot) {
+                                              int phase, const Geom& g, const OwnerTable& ot, int xa, int xb,
+                                              int parts) {
     const int lane = threadIdx.x & 31;
     const int tny = tiles_along(g.ny), tnz = tiles_along(g.nz);
     const int tx = t / (tny * tnz);
@@ -569,7 +574,7 @@ __device__ __forceinline__ void voxelize_tile(WarpVox<INIT_VEL>& S, int t, const
     // The tile's count, both bin slots of the lane (read whatever the count; the
     // slots past it are ignored) and its 16 voxel words are independent loads,
     // issued together so that the tile waits for one memory latency, not four.
-    const int cnt = tile_cnt[t];
+    const int cnt = *(volatile int*)(tile_cnt + t) & TILE_CNT_MASK;
     const int a0 = bins[(size_t)t * TILE_BIN + lane];
     const int b0 = bins[(size_t)t * TILE_BIN + lane + 32];
     // cell state; a lane's cells share z and, per plane half, the row
@@ -579,7 +584,7 @@ __device__ __forceinline__ void voxelize_tile(WarpVox<INIT_VEL>& S, int t, const
 #pragma unroll
     for (int j = 0; j < 16; ++j) {
         const int X = X0 + (j >> 1), Y = Y0 + (lane >> 3) + 4 * (j & 1);
-        wv[j] = (zok && X < g.nx && Y < g.ny) ? vox[((size_t)X * g.ny + Y) * g.nz + Z] : 0u;
+        wv[j] = (zok && X < g.nx && Y < g.ny && (j >> 1) >= xa && (j >> 1) <= xb) ? vox[((size_t)X * g.ny + Y) * g.nz + Z] : 0u;
     }
 #pragma unroll
     for (int j = 0; j < 16; ++j) {
@@ -591,8 +596,13 @@ __device__ __forceinline__ void voxelize_tile(WarpVox<INIT_VEL>& S, int t, const
     // the lane's bin entries (list indices)
     int a = (cnt <= TILE_BIN && lane < cnt) ? a0 : INT_MAX;
     int b = (cnt <= TILE_BIN && lane + 32 < cnt) ? b0 : INT_MAX;
-    if (cnt <= 0) return;
-    if (lane == 0) tile_cnt[t] = 0;    // the bins are reused by the next voxelization
+    if (cnt <= 0) return;   // (a listed tile has a sphere)
+    // the bins are reused by the next voxelization: the count is zeroed by the last of
+    // the tile's warps to have read it (arrivals in the bits above TILE_CNT_MASK)
+    if (lane == 0) {
+        if (parts == 1 || atomicAdd((unsigned*)(tile_cnt + t), TILE_CNT_MASK + 1u) >> TILE_CNT_BITS == parts - 1u)
+            tile_cnt[t] = 0;
+    }
     constexpr int W4 = (int)(sizeof(SphereFast) / 16);
     const uint4* src = reinterpret_cast<const uint4*>(fast);
     uint4* dst = reinterpret_cast<uint4*>(S.q);
@@ -611,7 +621,7 @@ __device__ __forceinline__ void voxelize_tile(WarpVox<INIT_VEL>& S, int t, const
                 dst[i] = __ldg(src + (size_t)S.list[base + e] * W4 + (i - W4 * e));
             }
             __syncwarp();
-            for (int k = 0; k < nst; ++k) apply_sphere(S, S.q[k], S.list[base + k], sph, X0, Y0, Z0);
+            for (int k = 0; k < nst; ++k) apply_sphere(S, S.q[k], S.list[base + k], sph, X0, Y0, Z0, xa, xb);
         }
     } else {
         // bin overflow: every sphere whose box reaches the tile, in list order
@@ -631,7 +641,7 @@ __device__ __forceinline__ void voxelize_tile(WarpVox<INIT_VEL>& S, int t, const
                 __syncwarp();
                 if (lane < W4) dst[lane] = __ldg(src + (size_t)m * W4 + lane);
                 __syncwarp();
-                apply_sphere(S, S.q[0], m, sph, X0, Y0, Z0);
+                apply_sphere(S, S.q[0], m, sph, X0, Y0, Z0, xa, xb);
             }
         }
     }
@@ -689,10 +699,33 @@ __device__ __forceinline__ void voxelize_tile(WarpVox<INIT_VEL>& S, int t, const
     }
 }
 
-// Persistent voxelization: warps claim tiles of the work list one at a time
-// (work_n[0] tiles listed, work_n[1] claim counter, work_n[2] finished warps;
-// the last warp to finish zeroes all three for the next voxelization).
+// Persistent voxelization: warps claim items of the work list one at a time
+// (work_n[0] tiles listed, work_n[1] claim counter, work_n[2] finished blocks; the last
+// block to finish zeroes all three for the next voxelization).  A warp's first item is
+// its own number, counted across the blocks first.
+// An item is a tile, or, when the tiles are few for the grid's warps, an x-slab of one
+// (cells are independent): a tile is a serial chain of up to 15 us per sphere shell for
+// one warp, and a short list, or the last round of a longer one, waits for that chain.
+// slab_bits() takes the number of slabs per tile that makes rounds x chain least, with
+// the part of the chain that every slab repeats (tile setup, list, records) a 16th of a
+// tile's: fitted to the cycle times of a 128^3 suspension, 4096 tiles on 3648 warps,
+// 535, 502, 492 us with 1, 2, 4 slabs, and a 96^3 one, 1728 tiles, 65, 60, 67, 73 us
+// with 1, 2, 4, 8.  Longer lists keep whole tiles (256^3: no difference).
 // BATCH: a listed tile belongs to the domain d with toff[d] <= tile.
+__device__ __forceinline__ int slab_bits(int nwork, int warps) {
+    int best = 0, cost = INT_MAX;
+#pragma unroll
+    for (int lp = 0; lp <= 3; ++lp) {
+        const int rounds = min(((nwork << lp) + warps - 1) / warps, 1 << 24);
+        const int c = rounds * (1 + (16 >> lp));
+        if (c < cost) {
+            cost = c;
+            best = lp;
+        }
+    }
+    return nwork < (1 << 24) ? best : 0;   // (longer lists: no slabs, and no overflow above)
+}
+
 template <typename T, bool INIT_VEL, bool BATCH>
 __global__ void __launch_bounds__(VOX_THREADS, INIT_VEL ? 2 : 3)
 k_voxelize(const SphereDev* __restrict__ sph, const SphereFast* __restrict__ fast, int nsph,
@@ -715,17 +748,22 @@ k_voxelize(const SphereDev* __restrict__ sph, const SphereFast* __restrict__ fas
         __syncthreads();   // every thread of the CTA reaches it (before any leaves)
     }
     const int nwork = *(volatile int*)work_n;
-    // the next tile is claimed and its index read while the current one is worked on
-    auto claim = [&]() -> int {
-        int w = 0;
-        if (lane == 0) w = atomicAdd(work_n + 1, 1);
-        w = __shfl_sync(FULL_MASK, w, 0);
-        return w < nwork ? work[w] : -1;
+    const int warps = (int)gridDim.x * VOX_WARPS;
+    const int lp = slab_bits(nwork, warps);
+    const int nitems = nwork << lp;
+    int part = 0;
+    // the next item is claimed and its tile read while the current one is worked on
+    auto item = [&](int w) -> int {
+        part = w & ((1 << lp) - 1);
+        return w < nitems ? work[w >> lp] : -1;
     };
-    int next = claim();
+    int next = item((int)(blockIdx.x + gridDim.x * (threadIdx.x >> 5)));
     while (next >= 0) {
         const int tg = next;
-        next = claim();
+        const int xa = part << (3 - lp), xb = xa + (TILE >> lp) - 1;
+        int w = 0;
+        if (lane == 0) w = atomicAdd(work_n + 1, 1) + warps;
+        next = item(__shfl_sync(FULL_MASK, w, 0));
         if (BATCH) {
             int d;
             if (stoff) {
@@ -743,15 +781,17 @@ k_voxelize(const SphereDev* __restrict__ sph, const SphereFast* __restrict__ fas
             const OwnerTable od{ot.xpf + (size_t)XPF_STRIDE * D.s0, ot.tag2slot + D.tag0, ot.max_tag};
             voxelize_tile<T, INIT_VEL>(S, tg - D.t0, sph + D.s0, fast + D.s0, __ldg(ncur + d), tile_cnt + D.t0,
                                        bins + (size_t)D.t0 * TILE_BIN, vox + D.cell0, up ? up + D.up0 : up,
-                                       f ? f + D.f0 : f, phase, D.g, od);
+                                       f ? f + D.f0 : f, phase, D.g, od, xa, xb, 1 << lp);
         } else {
-            voxelize_tile<T, INIT_VEL>(S, tg, sph, fast, nsph, tile_cnt, bins, vox, up, f, phase, g, ot);
+            voxelize_tile<T, INIT_VEL>(S, tg, sph, fast, nsph, tile_cnt, bins, vox, up, f, phase, g, ot, xa, xb,
+                                       1 << lp);
         }
         __syncwarp();
     }
-    if (lane == 0) {
+    __syncthreads();
+    if (threadIdx.x == 0) {
         __threadfence();
-        if (atomicAdd(work_n + 2, 1) == (int)(gridDim.x * VOX_WARPS) - 1) {
+        if (atomicAdd(work_n + 2, 1) == (int)gridDim.x - 1) {
             work_n[0] = 0;
             work_n[1] = 0;
             work_n[2] = 0;
@@ -811,8 +851,7 @@ cudaError_t launch_vox(const SphereDev* sph, const SphereFast* fast, int n, int*
         blocks = sms * (per_sm > 0 ? per_sm : 1);
         cached[dev].store(blocks, std::memory_order_relaxed);
     }
-    const int need = (ntiles + VOX_WARPS - 1) / VOX_WARPS;
-    const int grid = need < blocks ? need : blocks;
+    const int grid = ntiles < blocks ? ntiles : blocks;   // up to TILE slabs per tile, one per warp
     k_voxelize<T, INIT_VEL, BATCH><<<grid, VOX_THREADS, smem, s>>>(sph, fast, n, tile_cnt, bins, work, work_n, vox, up,
                                                                   f, phase, g, doms, toff, ndom, ncur, ot);
     return cudaGetLastError();
