@@ -14,8 +14,11 @@
 // owns whole cells: it rescales the cell's incoming populations and adds the
 // cell's rhoBar (after the rescale) to the box sum, so the same launch also
 // leaves the averages the next step's rescale needs.  The box sums are
-// deterministic: per-block partial sums, added in block order by the last block
-// of each job.
+// deterministic: per-block partial sums, added in a fixed order by the last block
+// of each job.  A plane is a few thousand cells, so the launch is as long as its chain of
+// memory latencies: one cell per thread, its 19 loads issued together, small blocks
+// (71x67x243 channel: 37 -> 10 us a step; a batch of 1024 boxes is bound by its strided
+// accesses instead, 0.39 ms either way).
 #include "lbdem_internal.h"
 
 namespace lbdem {
@@ -58,16 +61,23 @@ __global__ void __launch_bounds__(PLANE_THREADS)
 
     double acc = 0;
     auto cell = [&](int x, int y, int z) {
+        // all 19 loads before the first store: a store would hold back the loads after it
+        // (they may alias for the compiler), and the pass is as long as its memory latencies
+        size_t s[Q];
+        T v[Q];
+#pragma unroll
+        for (int i = 0; i < Q; ++i) {
+            s[i] = slot_index(i, x, y, z, phase, J.g);
+            v[i] = f[s[i]];
+        }
         T rb = T(0);   // the cell's rhoBar in the lattice type, widened once
 #pragma unroll
         for (int i = 0; i < Q; ++i) {
-            const size_t s = slot_index(i, x, y, z, phase, J.g);
-            T v = f[s];
             if (RESCALE && comp(i, J.dim) == J.dir) {
-                v = rescale_pop<T>(v, wt(i), k);
-                f[s] = v;
+                v[i] = rescale_pop<T>(v[i], wt(i), k);
+                f[s[i]] = v[i];
             }
-            rb += v;
+            rb += v[i];
         }
         acc += (double)rb;
     };
@@ -97,13 +107,20 @@ __global__ void __launch_bounds__(PLANE_THREADS)
         s_last = atomicAdd(&count[blockIdx.y], 1u) == gridDim.x - 1;
     }
     __syncthreads();
-    if (s_last && threadIdx.x == 0) {
+    if (s_last && threadIdx.x < 32) {
+        // two partial sums per lane, then the lanes in a fixed tree: the same sum whichever
+        // block comes last
         __threadfence();
         const volatile double* p = partial + (size_t)blockIdx.y * PLANE_BLOCKS_MAX;
-        double sum = 0;
-        for (unsigned b = 0; b < gridDim.x; ++b) sum += p[b];
-        avg_out[J.write] = 1.0 + sum / (double)ncell;       // fullRho(mean rhoBar)
-        count[blockIdx.y] = 0;
+        static_assert(PLANE_BLOCKS_MAX == 64, "two partial sums per lane");
+        const double a = threadIdx.x < gridDim.x ? p[threadIdx.x] : 0.0;
+        const double b = threadIdx.x + 32 < gridDim.x ? p[threadIdx.x + 32] : 0.0;
+        double sum = a + b;
+        for (int o = 16; o > 0; o >>= 1) sum += __shfl_down_sync(0xffffffffu, sum, o);
+        if (threadIdx.x == 0) {
+            avg_out[J.write] = 1.0 + sum / (double)ncell;       // fullRho(mean rhoBar)
+            count[blockIdx.y] = 0;
+        }
     }
 }
 

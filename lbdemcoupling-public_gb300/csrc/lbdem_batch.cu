@@ -603,7 +603,7 @@ lbdem_status lbdem_batch_create(const lbdem_batch_config* cfg, int32_t ndomains,
                 maxcells = std::max(maxcells, box_cells(box));
             }
         }
-        b->plane_bpj = (int)std::max(1LL, std::min<long long>((maxcells + 2 * PLANE_THREADS - 1) / (2 * PLANE_THREADS),
+        b->plane_bpj = (int)std::max(1LL, std::min<long long>((maxcells + PLANE_THREADS - 1) / PLANE_THREADS,
                                                               PLANE_BLOCKS_MAX));
         TRY(dalloc(b, &b->d_jobs, sizeof(PlaneJob) * b->njobs));
         TRY(dalloc(b, &b->d_pavg, sizeof(double) * 2 * b->njobs));

@@ -235,7 +235,7 @@ long long box_cells(const int32_t* b) {
 }
 
 int plane_blocks(long long cells) {
-    long long b = (cells + 2 * PLANE_THREADS - 1) / (2 * PLANE_THREADS);
+    long long b = (cells + PLANE_THREADS - 1) / PLANE_THREADS;
     return (int)std::max(1LL, std::min<long long>(b, PLANE_BLOCKS_MAX));
 }
 

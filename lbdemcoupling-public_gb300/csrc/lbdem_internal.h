@@ -363,7 +363,7 @@ struct PlaneJob {
     int write;               // average slot receiving this box's average
 };
 constexpr int PLANE_BLOCKS_MAX = 64;    // blocks per job (partial sums per job)
-constexpr int PLANE_THREADS = 256;
+constexpr int PLANE_THREADS = 128;
 
 // jobs: device table; partial: [njobs][PLANE_BLOCKS_MAX]; count: [njobs], zero on
 // entry and left zero; avg_in / avg_out: average slots before / after.  rescale = 0
