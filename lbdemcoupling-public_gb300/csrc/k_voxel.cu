@@ -332,6 +332,7 @@ __device__ __forceinline__ int slice_count_resolve(float dxf, float dyf, float d
 constexpr int VOX_WARPS = 8;                        // warps per block
 constexpr int VOX_THREADS = 32 * VOX_WARPS;
 constexpr int VOX_STAGE = 32;                       // sphere records staged at a time
+constexpr int VOX_SLAB_ROUNDS = 2;
 // A tile's sphere count and, above it, the arrivals of its warps (at most 8).
 constexpr int TILE_CNT_BITS = 28;
 constexpr unsigned TILE_CNT_MASK = (1u << TILE_CNT_BITS) - 1u;
@@ -563,7 +564,7 @@ __device__ __forceinline__ void voxelize_tile(WarpVox<INIT_VEL>& S, int t, const
                                               int* __restrict__ tile_cnt, const int* __restrict__ bins,
                                               uint32_t* __restrict__ vox, T* __restrict__ up, T* __restrict__ f,
                                               int phase, const Geom& g, const OwnerTable& ot, int xa, int xb,
-                                              int parts) {
+                                              unsigned parts) {
     const int lane = threadIdx.x & 31;
     const int tny = tiles_along(g.ny), tnz = tiles_along(g.nz);
     const int tx = t / (tny * tnz);
@@ -574,7 +575,7 @@ __device__ __forceinline__ void voxelize_tile(WarpVox<INIT_VEL>& S, int t, const
     // The tile's count, both bin slots of the lane (read whatever the count; the
     // slots past it are ignored) and its 16 voxel words are independent loads,
     // issued together so that the tile waits for one memory latency, not four.
-    const int cnt = *(volatile int*)(tile_cnt + t) & TILE_CNT_MASK;
+    const int cnt = (int)((unsigned)tile_cnt[t] & TILE_CNT_MASK);
     const int a0 = bins[(size_t)t * TILE_BIN + lane];
     const int b0 = bins[(size_t)t * TILE_BIN + lane + 32];
     // cell state; a lane's cells share z and, per plane half, the row
@@ -701,8 +702,7 @@ __device__ __forceinline__ void voxelize_tile(WarpVox<INIT_VEL>& S, int t, const
 
 // Persistent voxelization: warps claim items of the work list one at a time
 // (work_n[0] tiles listed, work_n[1] claim counter, work_n[2] finished blocks; the last
-// block to finish zeroes all three for the next voxelization).  A warp's first item is
-// its own number, counted across the blocks first.
+// block to finish zeroes all three for the next voxelization).
 // An item is a tile, or, when the tiles are few for the grid's warps, an x-slab of one
 // (cells are independent): a tile is a serial chain of up to 15 us per sphere shell for
 // one warp, and a short list, or the last round of a longer one, waits for that chain.
@@ -710,7 +710,11 @@ __device__ __forceinline__ void voxelize_tile(WarpVox<INIT_VEL>& S, int t, const
 // the part of the chain that every slab repeats (tile setup, list, records) a 16th of a
 // tile's: fitted to the cycle times of a 128^3 suspension, 4096 tiles on 3648 warps,
 // 535, 502, 492 us with 1, 2, 4 slabs, and a 96^3 one, 1728 tiles, 65, 60, 67, 73 us
-// with 1, 2, 4, 8.  Longer lists keep whole tiles (256^3: no difference).
+// with 1, 2, 4, 8.  SLABS false: whole tiles only, for lattices of more than
+// VOX_SLAB_ROUNDS tiles per warp (their lists are long enough as a rule, and the slab
+// bounds cost the kernel 4 % on a 256^3 suspension).
+// A warp's first item is its own number, counted across the blocks first: a short list
+// spreads over the SMs and starts without a claim.
 // BATCH: a listed tile belongs to the domain d with toff[d] <= tile.
 __device__ __forceinline__ int slab_bits(int nwork, int warps) {
     int best = 0, cost = INT_MAX;
@@ -726,7 +730,7 @@ __device__ __forceinline__ int slab_bits(int nwork, int warps) {
     return nwork < (1 << 24) ? best : 0;   // (longer lists: no slabs, and no overflow above)
 }
 
-template <typename T, bool INIT_VEL, bool BATCH>
+template <typename T, bool INIT_VEL, bool BATCH, bool SLABS>
 __global__ void __launch_bounds__(VOX_THREADS, INIT_VEL ? 2 : 3)
 k_voxelize(const SphereDev* __restrict__ sph, const SphereFast* __restrict__ fast, int nsph,
            int* __restrict__ tile_cnt, const int* __restrict__ bins, const int* __restrict__ work,
@@ -749,7 +753,7 @@ k_voxelize(const SphereDev* __restrict__ sph, const SphereFast* __restrict__ fas
     }
     const int nwork = *(volatile int*)work_n;
     const int warps = (int)gridDim.x * VOX_WARPS;
-    const int lp = slab_bits(nwork, warps);
+    const int lp = SLABS ? slab_bits(nwork, warps) : 0;
     const int nitems = nwork << lp;
     int part = 0;
     // the next item is claimed and its tile read while the current one is worked on
@@ -781,10 +785,10 @@ k_voxelize(const SphereDev* __restrict__ sph, const SphereFast* __restrict__ fas
             const OwnerTable od{ot.xpf + (size_t)XPF_STRIDE * D.s0, ot.tag2slot + D.tag0, ot.max_tag};
             voxelize_tile<T, INIT_VEL>(S, tg - D.t0, sph + D.s0, fast + D.s0, __ldg(ncur + d), tile_cnt + D.t0,
                                        bins + (size_t)D.t0 * TILE_BIN, vox + D.cell0, up ? up + D.up0 : up,
-                                       f ? f + D.f0 : f, phase, D.g, od, xa, xb, 1 << lp);
+                                       f ? f + D.f0 : f, phase, D.g, od, xa, xb, 1u << lp);
         } else {
             voxelize_tile<T, INIT_VEL>(S, tg, sph, fast, nsph, tile_cnt, bins, vox, up, f, phase, g, ot, xa, xb,
-                                       1 << lp);
+                                       1u << lp);
         }
         __syncwarp();
     }
@@ -839,21 +843,34 @@ cudaError_t launch_vox(const SphereDev* sph, const SphereFast* fast, int n, int*
     if (dev < 0 || dev >= LBDEM_MAX_DEVICES) return cudaErrorInvalidDevice;
     int blocks = cached[dev].load(std::memory_order_relaxed);
     if (blocks == 0) {
-        int sms = 0, per_sm = 0;
+        int sms = 0, per_sm = 0, per_sm_slabs = 0;
         e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
         if (e == cudaSuccess)
-            e = cudaFuncSetAttribute(k_voxelize<T, INIT_VEL, BATCH>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+            e = cudaFuncSetAttribute(k_voxelize<T, INIT_VEL, BATCH, false>,
+                                     cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        if (e == cudaSuccess)
+            e = cudaFuncSetAttribute(k_voxelize<T, INIT_VEL, BATCH, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                      (int)smem);
         if (e == cudaSuccess)
-            e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_voxelize<T, INIT_VEL, BATCH>, VOX_THREADS,
-                                                              smem);
+            e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_voxelize<T, INIT_VEL, BATCH, false>,
+                                                              VOX_THREADS, smem);
+        if (e == cudaSuccess)
+            e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm_slabs, k_voxelize<T, INIT_VEL, BATCH, true>,
+                                                              VOX_THREADS, smem);
         if (e != cudaSuccess) return e;
+        if (per_sm_slabs < per_sm) per_sm = per_sm_slabs;
         blocks = sms * (per_sm > 0 ? per_sm : 1);
         cached[dev].store(blocks, std::memory_order_relaxed);
     }
     const int grid = ntiles < blocks ? ntiles : blocks;   // up to TILE slabs per tile, one per warp
-    k_voxelize<T, INIT_VEL, BATCH><<<grid, VOX_THREADS, smem, s>>>(sph, fast, n, tile_cnt, bins, work, work_n, vox, up,
-                                                                  f, phase, g, doms, toff, ndom, ncur, ot);
+    if (ntiles <= VOX_SLAB_ROUNDS * blocks * VOX_WARPS)
+        k_voxelize<T, INIT_VEL, BATCH, true><<<grid, VOX_THREADS, smem, s>>>(sph, fast, n, tile_cnt, bins, work, work_n,
+                                                                             vox, up, f, phase, g, doms, toff, ndom,
+                                                                             ncur, ot);
+    else
+        k_voxelize<T, INIT_VEL, BATCH, false><<<grid, VOX_THREADS, smem, s>>>(sph, fast, n, tile_cnt, bins, work,
+                                                                              work_n, vox, up, f, phase, g, doms, toff,
+                                                                              ndom, ncur, ot);
     return cudaGetLastError();
 }
 
