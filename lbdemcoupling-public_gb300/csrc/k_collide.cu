@@ -15,15 +15,15 @@
 // is replaced by the cell itself with the direction reversed: half-way
 // bounce-back.  Periodic axes wrap.
 //
-// One kernel implements the step: persistent CTAs of 128 threads whose warps
-// walk 64-cell z-segments.  The 19 population rows of a segment (plus, in the
+// Lattices with 16-byte aligned rows and the FP64 form: persistent CTAs of 128 threads
+// whose warps walk 64-cell z-segments.  The 19 population rows of a segment (plus, in the
 // odd phase, the halo element of every c_z != 0 direction), the voxel words and
 // (FP64 form, single lattice) the particle surface-velocity rows are staged in
 // shared memory, double-buffered, so the next segment's bytes are in flight while the
 // current one is collided: per-thread 16-byte cp.async with commit groups for
-// FP32 lattices with 16-byte aligned rows, cp.async.bulk on an mbarrier
-// otherwise; rows that are not 16-byte aligned (nz % 4 != 0) are copied in whole
-// 16-byte chunks around the row.  The staged pre-collision values double as
+// the FP32 form, cp.async.bulk on an mbarrier for the FP64 form; rows that are not
+// 16-byte aligned (nz % 4 != 0) are copied in whole 16-byte chunks around the row (FP64),
+// or not staged at all (FP32: k_collide_direct, which also steps FP32 batches).  The staged pre-collision values double as
 // fPre of the PSM update.  The FP32 form collides two cells per thread in packed
 // f32x2 arithmetic (collide_segment_pairs) and recomputes the particle surface
 // velocity of its solid cells from the owner particle's row of the float table
@@ -650,7 +650,6 @@ __device__ __forceinline__ double widen(float x) {
     const uint32_t ed = e == 0xffu ? 0x7ffu : e + 896u;   // rebias 127 -> 1023
     return __hiloint2double((int)(s | (ed << 20) | (m >> 3)), (int)(m << 29));
 }
-__device__ __forceinline__ double widen(double x) { return x; }
 
 // Per-cell force and torque of a solid cell (SumForceTorque3D,
 // src/ibProcessors3D.hh:203-263): particle slot of the owner tag and the
@@ -831,6 +830,8 @@ __device__ __forceinline__ int pick(int c, int m, int v, int p) { return c < 0 ?
 // over SEGW-cell z-segments (no block-wide barriers, so a warp with solid
 // cells does not hold up the others).
 constexpr int WARPS = COLLIDE_BLOCK / 32;    // warps per CTA
+constexpr int DIRECT_BLOCK = 128;              // threads per CTA of k_collide_direct
+constexpr int DIRECT_BLOCKS_PER_SM = 4;
 // Per-CTA tables in dynamic shared memory behind the warps' stages.
 // FP32 form, single lattice: a copy of the tag -> slot map when the tags fit below
 // TAGMAP_SMEM - 1, holding -1 for a tag with no particle in the list and for every entry
@@ -838,17 +839,11 @@ constexpr int WARPS = COLLIDE_BLOCK / 32;    // warps per CTA
 // min(tag, TAGMAP_SMEM - 1) with no tests between the cell's voxel word and the owner's
 // table row; then B(n) (128 floats).
 constexpr int TAGMAP_SMEM = 2048;
-template <typename T, bool BATCH>
-__host__ __device__ constexpr bool smem_tagmap() { return sizeof(T) == 4 && !BATCH; }
-template <typename T, bool BATCH>
-__host__ __device__ constexpr size_t tagmap_bytes() {
-    return smem_tagmap<T, BATCH>() ? sizeof(int) * TAGMAP_SMEM + sizeof(float) * 128 : 0;
-}
+constexpr size_t TAGMAP_BYTES = sizeof(int) * TAGMAP_SMEM + sizeof(float) * 128;
 // Batch mode: each CTA keeps the first segment of every domain in shared memory when
 // there are at most SEG0_SMEM domains (the per-segment domain search reads it there).
 constexpr int SEG0_SMEM = 2048;
-template <bool BATCH>
-__host__ __device__ constexpr size_t seg0_bytes() { return BATCH ? sizeof(int) * SEG0_SMEM : 0; }
+constexpr size_t SEG0_BYTES = sizeof(int) * SEG0_SMEM;
 constexpr int SEGW = COLLIDE_SEGW;          // cells per warp segment (2 per lane)
 constexpr int WAIT_LIMIT = 1 << 22;         // bounded mbarrier wait (iterations of try_wait)
 constexpr int PROBE_WAIT = 64;              // the timeout test hook's wait (iterations)
@@ -872,8 +867,6 @@ struct alignas(16) WarpStage {
     unsigned long long lead[2];   // unaligned rows: lead elements of row i at bits 2i, voxel row at bits 38,
                                   // surface-velocity row d at bits 40 + 2d
     unsigned long long bar[2];
-    // stages shared by two warps: buffer b read by both; its halo elements in place
-    unsigned long long empty[2], halo[2];
 };
 
 static_assert(sizeof(WarpStage<float, true>) % 16 == 0 && sizeof(WarpStage<float, false>) % 16 == 0 &&
@@ -883,12 +876,8 @@ static_assert(offsetof(WarpStage<float>, vox) % 16 == 0 && offsetof(WarpStage<fl
                   offsetof(WarpStage<double>, vox) % 16 == 0 && offsetof(WarpStage<double>, up) % 16 == 0,
               "bulk-copy destinations on 16-byte boundaries");
 
-// The per-CTA tables behind the warps' stages.
-template <typename T, bool STAGE_UP>
-__device__ __forceinline__ unsigned char* cta_tables(int stages = WARPS) {
-    extern __shared__ __align__(16) unsigned char smem_raw[];
-    return smem_raw + stages * sizeof(WarpStage<T, STAGE_UP>);
-}
+// Where the FP32 form's per-CTA tables lie: behind the warps' stages.
+constexpr size_t STAGED_TABLES = WARPS * sizeof(WarpStage<float, false>);
 
 __host__ __device__ constexpr int row_slot(int dx, int dy) { return 3 * (dx + 1) + dy + 1; }
 
@@ -1208,79 +1197,217 @@ __device__ __forceinline__ void issue_segment_lsu(const CollideArgs<T>& a, WarpS
     cp_commit();
 }
 
-// Force and torque of a segment that is a whole z-periodic row (per-cell arms),
-// kept out of line: the bench lattices never take it.
-__device__ __noinline__ void whole_row_forces(const CollideArgs<float>& a, uint32_t w0, uint32_t w1, bool v0, bool v1,
-                                              int sx, int sy, int za, int zb, float2 fx, float2 fy, float2 fz) {
-    float va[6] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f}, vb[6] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
-    const int ka = v0 ? cell_force_terms(a, w0, sx, sy, za, fx.x, fy.x, fz.x, va) : -1;
-    const int kb = v1 ? cell_force_terms(a, w1, sx, sy, zb, fx.y, fy.y, fz.y, vb) : -1;
-    if (__all_sync(FULL, ka < 0 || kb < 0 || ka == kb)) {
-        const int key = ka >= 0 ? ka : kb;
-#pragma unroll
-        for (int q = 0; q < 6; ++q) va[q] += vb[q];
-        reduce_forces(a, key, va);
-    } else {
-        reduce_forces(a, ka, va);
-        reduce_forces(a, kb, vb);
+// The FP32 form's per-CTA tables (see TAGMAP_SMEM), OFF bytes into dynamic shared
+// memory; NO_TABLES: none, B(n) and the map are read from global memory.  (Addressed from
+// the array itself: through a stored pointer the compiler takes generic loads.)
+constexpr size_t NO_TABLES = ~(size_t)0;
+template <size_t OFF>
+struct PairTables {
+    bool map;   // the tags fit the copy of the map
+    __device__ __forceinline__ static int* base() {
+        extern __shared__ __align__(16) unsigned char smem_raw[];
+        return reinterpret_cast<int*>(smem_raw + OFF);
     }
+    __device__ __forceinline__ static float* btab() { return reinterpret_cast<float*>(base() + TAGMAP_SMEM); }
+    // Filled by the CTA's threads (TAGMAP_BYTES); the caller synchronizes.
+    __device__ __forceinline__ void load(const CollideArgs<float>& a) {
+        map = a.max_tag < TAGMAP_SMEM - 1;
+        if (map)
+            for (int k = threadIdx.x; k < TAGMAP_SMEM; k += blockDim.x) {
+                const int v = k <= a.max_tag ? __ldg(a.tag2slot + k) : -1;
+                base()[k] = (v >= 0 && v < a.nslot) ? v : -1;
+            }
+        for (int k = threadIdx.x; k < 126; k += blockDim.x) btab()[k] = __ldg(a.btab + k);
+    }
+};
+// What the collision of a lane's two cells leaves for the force sums: the momentum
+// exchange, the owners' slots (-1: none) and the centre part of the table row that the
+// velocity lookup read (slot vslot).
+struct PairForce {
+    F2 Fx, Fy, Fz;
+    int s0, s1, vslot;
+    bool unmapped;   // a solid cell whose tag names no particle (reported, left out of the sums)
+    float4 rh;
+    float rl0, rl1;
+};
+
+// Collision of a lane's two cells (x, ya, za) and (x, yb, zb) with the voxel words w0,
+// w1 (0 for a lane slot without a cell): f in, f out, for k_collide_direct.  The same
+// operations as in collide_segment_pairs, so a cell gets the same bits in both.
+// BGK runs for every cell, the fully covered ones included (their solid correction with
+// B = 1 returns fPre + bb up to rounding), so that a cell's result does not depend on the
+// cell it is paired with; the solid terms run in warps that hold a solid cell.  Must be
+// reached by all 32 lanes.
+template <bool FORCE, size_t OFF>
+__device__ __forceinline__ void collide_pair(const CollideArgs<float>& a, const Geom& g, const PairTables<OFF>& tb,
+                                             F2 (&f)[Q], uint32_t w0, uint32_t w1, int x, int ya, int za, int yb,
+                                             int zb, PairForce& o) {
+    const int n0 = min((int)(w0 & VOX_NMASK), 125), n1 = min((int)(w1 & VOX_NMASK), 125);
+    const F2 B = OFF != NO_TABLES ? pk(tb.btab()[n0], tb.btab()[n1]) : pk(__ldg(a.btab + n0), __ldg(a.btab + n1));
+    const Mom2 m = moments2(f);
+    o.Fx = o.Fy = o.Fz = bc(0.f);
+    o.s0 = o.s1 = o.vslot = -1;
+    o.unmapped = false;
+    o.rh = make_float4(0.f, 0.f, 0.f, 0.f);
+    o.rl0 = o.rl1 = 0.f;
+    // owner slots (from the CTA's shared copy of the map when it has one)
+    auto owner = [&](uint32_t w) -> int {
+        const int tag = (int)(w >> VOX_NBITS);
+        if (OFF != NO_TABLES && tb.map) return tb.base()[min(tag, TAGMAP_SMEM - 1)];
+        // global map: an unconditional load at the clamped tag, tested afterwards
+        const int slot = __ldg(a.tag2slot + min(tag, a.max_tag));
+        return (tag <= a.max_tag && slot >= 0 && slot < a.nslot) ? slot : -1;
+    };
+    o.s0 = n0 > 0 ? owner(w0) : -1;
+    o.s1 = n1 > 0 ? owner(w1) : -1;
+    // particle surface velocity of the lane's solid cells, recomputed from the owner
+    // particle's row of the float table (one row when both cells belong to the same
+    // particle); every lane of the warp loads a row (slot 0 for a lane without a solid
+    // cell, whose velocities stay zero): no branch ahead of the load
+    F2 u0 = bc(0.f), u1 = bc(0.f), u2 = bc(0.f);
+    auto solid_velocity = [&]() {
+        float ua[3] = {0.f, 0.f, 0.f}, ub[3] = {0.f, 0.f, 0.f};
+        const int sl = o.s0 >= 0 ? o.s0 : o.s1;
+        {
+            const TableRow r = load_row(a.xpf, max(sl, 0));
+            o.rh = r.a;
+            o.rl0 = r.b.x;
+            o.rl1 = r.b.y;
+            o.vslot = sl;
+            const RowPart rp = row_part(r, x, ya, g);
+            if (o.s0 >= 0) cell_part(r, rp, za, g, ua[0], ua[1], ua[2]);
+            if (sl >= 0 && o.s1 == sl) {
+                if (yb != ya) cell_part(r, row_part(r, x, yb, g), zb, g, ub[0], ub[1], ub[2]);
+                else cell_part(r, rp, zb, g, ub[0], ub[1], ub[2]);
+            }
+        }
+        if (o.s1 >= 0 && o.s1 != sl) row_velocity(load_row(a.xpf, o.s1), x, yb, zb, g, ub[0], ub[1], ub[2]);
+        u0 = pk(ua[0], ub[0]);
+        u1 = pk(ua[1], ub[1]);
+        u2 = pk(ua[2], ub[2]);
+    };
+    // FORCE: the solid correction's momentum is the BGK post-collision one, j + rho g,
+    // for the cells that ran BGK
+    auto hsol = [&]() -> F2 {
+        return pk(n0 < 125 ? 1.f : 0.f, n1 < 125 ? 1.f : 0.f) * (bc(1.f) + m.rhoBar);
+    };
+    if (__any_sync(FULL, n0 > 0 || n1 > 0)) {   // one pass
+        solid_velocity();
+        if constexpr (FORCE)
+            bgk_psm2<FORCE>(f, m, a.omega, a.g3[0], a.g3[1], a.g3[2], hsol(), u0, u1, u2, B, o.Fx, o.Fy, o.Fz);
+        else
+            collide_g2<true>(f, m, a.omega, u0, u1, u2, B, o.Fx, o.Fy, o.Fz);
+    } else {
+        if constexpr (FORCE) bgk2<FORCE>(f, m, a.omega, a.g3[0], a.g3[1], a.g3[2]);
+        else collide_g2<false>(f, m, a.omega, u0, u1, u2, B, o.Fx, o.Fy, o.Fz);
+    }
+    o.unmapped = (n0 > 0 && o.s0 < 0) || (n1 > 0 && o.s1 < 0);
 }
 
-// FP32 compute pass over one staged segment, two cells per lane in packed
-// pairs.  Aligned rows (!MIS): lane l takes the adjacent cells j = 2 l, 2 l + 1,
+// Force and torque of a lane's two cells with per-cell arms (cells of one owner may lie in
+// several rows, or wrap around a periodic row), reduced over the warp per run of equal
+// owner; v0, v1: the lane slots that hold a cell.  Must be reached by all 32 lanes.
+__device__ __forceinline__ void forces_by_cell(const CollideArgs<float>& a, const Geom& g, const PairForce& o,
+                                               int x, int ya, int za, int yb, int zb) {
+    if (o.unmapped) atomicOr(a.err, 0x8u);   // LBDEM_DEVERR_UNMAPPED_TAG
+    const int ka = o.s0, kb = o.s1;
+    if (!__any_sync(FULL, ka >= 0 || kb >= 0)) return;
+    const float2 fx = upk(o.Fx), fy = upk(o.Fy), fz = upk(o.Fz);
+    auto terms = [&](int slot, int y, int z, float cfx, float cfy, float cfz, float (&v)[6]) {
+        float4 h = o.rh;
+        float lx = o.rl0, lz = o.rl1;
+        if (slot != o.vslot) {
+            const float4* p = reinterpret_cast<const float4*>(a.xpf + (size_t)slot * XPF_STRIDE);
+            h = __ldg(p);
+            const float4 l = __ldg(p + 1);
+            lx = l.x;
+            lz = l.y;
+        }
+        // centre = hi + lo in float: (x - hi) - lo is the arm to ~1 ulp
+        arm_terms(((float)x - h.x) - h.w, ((float)y - h.y) - lx, ((float)z - h.z) - lz, g, cfx, cfy, cfz, v);
+    };
+    float va[6] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f}, vb[6] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+    if (ka >= 0) terms(ka, ya, za, fx.x, fy.x, fz.x, va);
+    if (kb >= 0) terms(kb, yb, zb, fx.y, fy.y, fz.y, vb);
+    const bool one = __all_sync(FULL, ka < 0 || kb < 0 || ka == kb);   // one reduction for both cells
+    if (one) {
+#pragma unroll
+        for (int q = 0; q < 6; ++q) va[q] += vb[q];
+    }
+#pragma unroll 1
+    for (int pass = 0; pass < (one ? 1 : 2); ++pass) {   // a single reduction site, as below
+        float v[6];
+#pragma unroll
+        for (int q = 0; q < 6; ++q) v[q] = pass == 0 ? va[q] : vb[q];
+        reduce_forces(a, pass == 0 ? (one && ka < 0 ? kb : ka) : kb, v);
+    }
+}
+// Force and torque of the two cells of a lane in one row segment, reduced per run of
+// equal owner (finish_run), arms from the segment's middle point zc; the two cells go
+// through one warp reduction when their owners agree.  Must be reached by all 32 lanes.
+__device__ __forceinline__ void forces_by_run(const CollideArgs<float>& a, const PairForce& o, int x, int y, int zc,
+                                              int za, int zb) {
+    if (o.unmapped) atomicOr(a.err, 0x8u);   // LBDEM_DEVERR_UNMAPPED_TAG
+    const int ka = o.s0, kb = o.s1;
+    if (!__any_sync(FULL, ka >= 0 || kb >= 0)) return;
+    const float2 fx = upk(o.Fx), fy = upk(o.Fy), fz = upk(o.Fz);
+    const float da = (float)(za - zc), db = (float)(zb - zc);
+    float va[5] = {fx.x, fy.x, fz.x, -da * fy.x, da * fx.x};
+    float vb[5] = {fx.y, fy.y, fz.y, -db * fy.y, db * fx.y};
+#pragma unroll
+    for (int q = 0; q < 5; ++q) {
+        if (ka < 0) va[q] = 0.f;
+        if (kb < 0) vb[q] = 0.f;
+    }
+    const bool one = __all_sync(FULL, ka < 0 || kb < 0 || ka == kb);   // one reduction for both cells
+    if (one) {
+#pragma unroll
+        for (int q = 0; q < 5; ++q) va[q] += vb[q];
+    }
+    // a single reduction site (the batch kernels' loop bodies are large enough for
+    // instruction-cache misses to cost more than the loop)
+#pragma unroll 1
+    for (int pass = 0; pass < (one ? 1 : 2); ++pass) {
+        float v[5];
+#pragma unroll
+        for (int q = 0; q < 5; ++q) v[q] = pass == 0 ? va[q] : vb[q];
+        const bool second = pass == 1 || (one && ka < 0);   // the run's cells are the b cells
+        reduce_runs(a, second ? kb : ka, v, second ? zb : za, x, y, zc, o.rh, o.rl0, o.rl1, o.vslot);
+    }
+}
+// forces_by_cell out of line, for the rare segments of the row kernels.
+__device__ __noinline__ void forces_by_cell_far(const CollideArgs<float>& a, PairForce o, int x, int y, int za,
+                                                int zb) {
+    forces_by_cell(a, a.g, o, x, y, za, y, zb);
+}
+
+// FP32 compute pass over one staged segment of a lattice with 16-byte aligned rows, two
+// cells per lane in packed pairs: lane l takes the adjacent cells j = 2 l, 2 l + 1,
 // whose staged values and destination slots are 8-byte aligned pairs, so loads
 // and stores are 64-bit (in the odd phase the c_z != 0 directions land one slot
-// over and are moved one lane over with a shuffle).  Unaligned rows (MIS): lane
-// l takes j = l and l + 32 (32-bit accesses, conflict-free and coalesced).
+// over and are moved one lane over with a shuffle).
 // Force and torque are reduced per run of equal owner (reduce_runs); the two
 // cells of a lane go through one warp reduction when their owners agree.
-// FLAT (even phase of the FP32 batch): the segment is 64 cells of an x-plane
-// taken in memory order across its z-rows (a.g is the plane view, see
-// CollideArgs); a solid cell's true (y, z) is recovered from its index in the
-// plane, and force and torque take per-cell arms (a run may cross rows).  The
-// even phase touches only the cell's own slots, so a cell's populations do
-// not depend on how the cells are grouped into segments.  FOLD (batch): one
-// force-reduction site instead of three (the batch kernels' loop bodies miss the
-// instruction cache).
-template <bool ODD, bool FORCE, bool PER, bool MIS, bool STAGE_UP, bool FLAT = false, bool FOLD = false>
+template <bool ODD, bool FORCE, bool PER, bool STAGE_UP>
 __device__ __forceinline__ void collide_segment_pairs(const CollideArgs<float>& a, WarpStage<float, STAGE_UP>& st,
                                                       int b, int sx, int sy, int z0, int len, uint32_t srcrow,
-                                                      unsigned long long lead, bool smap_ok, bool sbtab_ok) {
-    static_assert(!FLAT || (!ODD && MIS), "plane segments: even phase, unaligned-row staging");
+                                                      const PairTables<STAGED_TABLES>& tb) {
     constexpr int V = WarpStage<float>::V;
-    constexpr bool ADJ = !MIS;
     const int lane = threadIdx.x & 31;
     const Geom& g = a.g;
     const size_t N = g.N;
     float* F = a.fo;
     const size_t own = (size_t)st.row[b][row_slot(0, 0)];
-    const int j0 = ADJ ? 2 * lane : lane, j1 = ADJ ? j0 + 1 : lane + 32;
+    const int j0 = 2 * lane, j1 = j0 + 1;
     const bool v0 = j0 < len, v1 = j1 < len;
     const int za = z0 + j0, zb = z0 + j1;
     const size_t ca = own + za, cb = own + zb;
-    // the cells' true geometry and coordinates (y, z) (FLAT: from the plane index;
-    // otherwise gt is g itself, not a copy that would hold its fields in registers)
-    Geom gflat;
-    if constexpr (FLAT) {
-        gflat = g;
-        gflat.ny = a.flat_ny;
-        gflat.nz = a.flat_nz;
-    }
-    const Geom& gt = FLAT ? gflat : g;
-    int ya = sy, yb = sy, zta = za, ztb = zb;
-    if constexpr (FLAT) {
-        ya = (int)fast_div((unsigned)za, a.dnz);
-        yb = (int)fast_div((unsigned)zb, a.dnz);
-        zta = za - ya * a.flat_nz;
-        ztb = zb - yb * a.flat_nz;
-    }
 
     // staged values of direction i for the lane's two cells
     auto at2 = [&](int i) -> F2 {
         const int shift = (ODD && cz(i) != 0 && (PER || ((srcrow >> i) & 1u))) ? cz(i) : 0;
-        const int m = MIS ? (int)((lead >> (2 * i)) & 3u) : 0;
-        const float* p = &st.f[b][i][V + m - shift];
-        if (ADJ && (shift & 1) == 0) {
+        const float* p = &st.f[b][i][V - shift];
+        if ((shift & 1) == 0) {
             const float2 t = *reinterpret_cast<const float2*>(p + j0);
             return pk(t.x, t.y);
         }
@@ -1289,12 +1416,9 @@ __device__ __forceinline__ void collide_segment_pairs(const CollideArgs<float>& 
     F2 f[Q];
 #pragma unroll
     for (int i = 0; i < Q; ++i) f[i] = at2(i);
-    const int vlead = MIS ? (int)((lead >> 38) & 3u) : 0;
-    const uint32_t w0 = v0 ? st.vox[b][vlead + j0] : 0u, w1 = v1 ? st.vox[b][vlead + j1] : 0u;
+    const uint32_t w0 = v0 ? st.vox[b][j0] : 0u, w1 = v1 ? st.vox[b][j1] : 0u;
     const int n0 = min((int)(w0 & VOX_NMASK), 125), n1 = min((int)(w1 & VOX_NMASK), 125);
-    const int* smap = reinterpret_cast<const int*>(cta_tables<float, STAGE_UP>());
-    const float* sbtab = reinterpret_cast<const float*>(smap + TAGMAP_SMEM);
-    const F2 B = sbtab_ok ? pk(sbtab[n0], sbtab[n1]) : pk(__ldg(a.btab + n0), __ldg(a.btab + n1));
+    const F2 B = pk(tb.btab()[n0], tb.btab()[n1]);
 
     // BGK runs for every cell, the fully covered ones included (their solid
     // correction with B = 1 returns fPre + bb up to rounding), so that a cell's
@@ -1308,7 +1432,7 @@ __device__ __forceinline__ void collide_segment_pairs(const CollideArgs<float>& 
     // owner slots (from the CTA's shared copy of the map when it has one)
     auto owner = [&](uint32_t w) -> int {
         const int tag = (int)(w >> VOX_NBITS);
-        if (smap_ok) return smap[min(tag, TAGMAP_SMEM - 1)];
+        if (tb.map) return tb.base()[min(tag, TAGMAP_SMEM - 1)];
         // global map: an unconditional load at the clamped tag, tested afterwards
         const int slot = __ldg(a.tag2slot + min(tag, a.max_tag));
         return (tag <= a.max_tag && slot >= 0 && slot < a.nslot) ? slot : -1;
@@ -1328,14 +1452,11 @@ __device__ __forceinline__ void collide_segment_pairs(const CollideArgs<float>& 
             // cell, whose velocities stay zero): no branch ahead of the load
             const TableRow r = load_row(a.xpf, max(sl, 0));
             vrh = r.a; vrl0 = r.b.x; vrl1 = r.b.y; vslot = sl;
-            const RowPart rp = row_part(r, sx, ya, gt);
-            if (s0 >= 0) cell_part(r, rp, zta, gt, ua[0], ua[1], ua[2]);
-            if (sl >= 0 && s1 == sl) {
-                if (FLAT && yb != ya) cell_part(r, row_part(r, sx, yb, gt), ztb, gt, ub[0], ub[1], ub[2]);
-                else cell_part(r, rp, ztb, gt, ub[0], ub[1], ub[2]);
-            }
+            const RowPart rp = row_part(r, sx, sy, g);
+            if (s0 >= 0) cell_part(r, rp, za, g, ua[0], ua[1], ua[2]);
+            if (sl >= 0 && s1 == sl) cell_part(r, rp, zb, g, ub[0], ub[1], ub[2]);
         }
-        if (s1 >= 0 && s1 != sl) row_velocity(load_row(a.xpf, s1), sx, yb, ztb, gt, ub[0], ub[1], ub[2]);
+        if (s1 >= 0 && s1 != sl) row_velocity(load_row(a.xpf, s1), sx, sy, zb, g, ub[0], ub[1], ub[2]);
 #pragma unroll
         for (int d = 0; d < 3; ++d) up[d] = pk(ua[d], ub[d]);
     };
@@ -1352,12 +1473,6 @@ __device__ __forceinline__ void collide_segment_pairs(const CollideArgs<float>& 
         } else {
             collide_g2<false>(f, m, a.omega, up[0], up[1], up[2], B, Fx, Fy, Fz);
         }
-    } else if constexpr (MIS) {
-        if (__any_sync(FULL, n0 > 0 || n1 > 0)) {   // one pass; a no-op for the lanes' fluid cells
-            if (n0 > 0 || n1 > 0) solid_velocity();
-            bgk_psm2<FORCE>(f, m, a.omega, a.g3[0], a.g3[1], a.g3[2], hsol(), up[0], up[1], up[2], B, Fx, Fy, Fz);
-        } else
-            bgk2<FORCE>(f, m, a.omega, a.g3[0], a.g3[1], a.g3[2]);
     } else {
         bgk2<FORCE>(f, m, a.omega, a.g3[0], a.g3[1], a.g3[2]);
         if (n0 > 0 || n1 > 0) {
@@ -1365,16 +1480,15 @@ __device__ __forceinline__ void collide_segment_pairs(const CollideArgs<float>& 
             const F2 sjx = fma2(hs, bc(a.g3[0]), m.jx), sjy = fma2(hs, bc(a.g3[1]), m.jy),
                      sjz = fma2(hs, bc(a.g3[2]), m.jz);
             solid_velocity();
-            if (FORCE) psm2(f, m.rhoBar, sjx, sjy, sjz, m.invRho, up[0], up[1], up[2], B, at2, Fx, Fy, Fz);
-            else psm2(f, m.rhoBar, m.jx, m.jy, m.jz, m.invRho, up[0], up[1], up[2], B, at2, Fx, Fy, Fz);
+            psm2(f, m.rhoBar, sjx, sjy, sjz, m.invRho, up[0], up[1], up[2], B, at2, Fx, Fy, Fz);
         }
     }
 
-    // Stores.  put(off, x, y, vx, vy): values x, y into slots off, off + 1 (ADJ:
-    // one 64-bit store when both are valid and the pair is aligned).
+    // Stores.  put(off, x, y, vx, vy): values x, y into slots off, off + 1 (one 64-bit
+    // store when both are valid and the pair is aligned).
     auto put = [&](size_t off, float x, float y, bool vx, bool vy) {
         // aligned rows only (the launcher sends arrays that are not 16-byte aligned
-        // to the unaligned-row path): an even slot offset is an 8-byte aligned pair
+        // to k_collide_direct): an even slot offset is an 8-byte aligned pair
         if (vx && vy) {
             *reinterpret_cast<float2*>(F + off) = make_float2(x, y);
         } else {
@@ -1385,14 +1499,9 @@ __device__ __forceinline__ void collide_segment_pairs(const CollideArgs<float>& 
     // the lane's two cells into slots (i, base + j0) and (i, base + j1)
     auto put_cells = [&](size_t base, F2 v) {
         const float2 t = upk(v);
-        if (ADJ) {
-            // aligned rows: segments hold a multiple of 4 cells, so both cells of a pair
-            // are valid together, and every pair of slots is 8-byte aligned
-            if (v0) *reinterpret_cast<float2*>(F + base + j0) = t;
-        } else {
-            if (v0) F[base + j0] = t.x;
-            if (v1) F[base + j1] = t.y;
-        }
+        // segments hold a multiple of 4 cells, so both cells of a pair are valid together,
+        // and every pair of slots is 8-byte aligned
+        if (v0) *reinterpret_cast<float2*>(F + base + j0) = t;
     };
     if (!ODD) {
 #pragma unroll
@@ -1414,29 +1523,17 @@ __device__ __forceinline__ void collide_segment_pairs(const CollideArgs<float>& 
             }
             // c_z != 0: each cell to slot z + c_z (wrapped, or bounced back at a z wall)
             const float2 t = upk(f[i]);
-            if (ADJ) {
-                // slots (j0, j0 + 1) of this lane receive cells (j0 - 1, j0) (c_z = +1)
-                // or (j0 + 1, j0 + 2) (c_z = -1), one lane over; the cell whose slot
-                // lies outside the segment (je) is stored on its own
-                if (cz(i) > 0) put(dst + z0 + j0, __shfl_up_sync(FULL, t.y, 1), t.x, lane > 0 && v0, v1);
-                else put(dst + z0 + j0, t.y, __shfl_down_sync(FULL, t.x, 1), v1, j0 + 2 < len);
-                const int je = cz(i) > 0 ? len - 1 : 0;
-                const int ze = z0 + je;
-                const int zd = cz(i) > 0 ? wrap_plus(ze, g.nz, per_z) : wrap_minus(ze, g.nz, per_z);
-                const size_t eoff = (PER || zd >= 0) ? dst + zd : (size_t)opp(i) * N + own + ze;
-                const float ev = (je & 1) ? t.y : t.x;
-                if (lane == (je >> 1)) F[eoff] = ev;
-            } else {
-#pragma unroll
-                for (int h = 0; h < 2; ++h) {
-                    if (h == 0 ? !v0 : !v1) continue;
-                    const int zz = h == 0 ? za : zb;
-                    const int zd = cz(i) > 0 ? wrap_plus(zz, g.nz, per_z) : wrap_minus(zz, g.nz, per_z);
-                    const float val = h == 0 ? t.x : t.y;
-                    if (PER || zd >= 0) F[dst + zd] = val;
-                    else F[(size_t)opp(i) * N + own + zz] = val;
-                }
-            }
+            // slots (j0, j0 + 1) of this lane receive cells (j0 - 1, j0) (c_z = +1)
+            // or (j0 + 1, j0 + 2) (c_z = -1), one lane over; the cell whose slot
+            // lies outside the segment (je) is stored on its own
+            if (cz(i) > 0) put(dst + z0 + j0, __shfl_up_sync(FULL, t.y, 1), t.x, lane > 0 && v0, v1);
+            else put(dst + z0 + j0, t.y, __shfl_down_sync(FULL, t.x, 1), v1, j0 + 2 < len);
+            const int je = cz(i) > 0 ? len - 1 : 0;
+            const int ze = z0 + je;
+            const int zd = cz(i) > 0 ? wrap_plus(ze, g.nz, per_z) : wrap_minus(ze, g.nz, per_z);
+            const size_t eoff = (PER || zd >= 0) ? dst + zd : (size_t)opp(i) * N + own + ze;
+            const float ev = (je & 1) ? t.y : t.x;
+            if (lane == (je >> 1)) F[eoff] = ev;
         }
     }
 
@@ -1445,50 +1542,11 @@ __device__ __forceinline__ void collide_segment_pairs(const CollideArgs<float>& 
         if (v0) { a.cf[ca] = fx.x; a.cf[N + ca] = fy.x; a.cf[2 * N + ca] = fz.x; }
         if (v1) { a.cf[cb] = fx.y; a.cf[N + cb] = fy.y; a.cf[2 * N + cb] = fz.y; }
     }
-    if constexpr (FLAT) {
-        // per-cell arms (a run of one owner may cross rows here), keyed by the owner
-        // slots of the velocity lookup; the arm reads the centre from the table row
-        // that lookup kept (a second owner in the lane reads its own row)
-        if ((v0 && n0 > 0 && s0 < 0) || (v1 && n1 > 0 && s1 < 0)) atomicOr(a.err, 0x8u);   // LBDEM_DEVERR_UNMAPPED_TAG
-        const int ka = v0 ? s0 : -1;
-        const int kb = v1 ? s1 : -1;
-        if (!__any_sync(FULL, ka >= 0 || kb >= 0)) return;
-        auto terms = [&](int slot, int y, int z, float cfx, float cfy, float cfz, float (&v)[6]) {
-            float4 h = vrh;
-            float lx = vrl0, lz = vrl1;
-            if (slot != vslot) {
-                const float4* p = reinterpret_cast<const float4*>(a.xpf + (size_t)slot * XPF_STRIDE);
-                h = __ldg(p);
-                const float4 l = __ldg(p + 1);
-                lx = l.x;
-                lz = l.y;
-            }
-            // centre = hi + lo in float: (x - hi) - lo is the arm to ~1 ulp
-            arm_terms(((float)sx - h.x) - h.w, ((float)y - h.y) - lx, ((float)z - h.z) - lz, gt, cfx, cfy, cfz, v);
-        };
-        float va[6] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f}, vb[6] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
-        if (ka >= 0) terms(ka, ya, zta, fx.x, fy.x, fz.x, va);
-        if (kb >= 0) terms(kb, yb, ztb, fx.y, fy.y, fz.y, vb);
-        const bool one = __all_sync(FULL, ka < 0 || kb < 0 || ka == kb);   // one reduction for both cells
-        if (one) {
-#pragma unroll
-            for (int q = 0; q < 6; ++q) va[q] += vb[q];
-        }
-        // a single reduction site: this kernel's loop body is large enough for
-        // instruction-cache misses to cost more than the loop
-#pragma unroll 1
-        for (int pass = 0; pass < (one ? 1 : 2); ++pass) {
-            float v[6];
-#pragma unroll
-            for (int q = 0; q < 6; ++q) v[q] = pass == 0 ? va[q] : vb[q];
-            reduce_forces(a, pass == 0 ? (one && ka < 0 ? kb : ka) : kb, v);
-        }
-        return;
-    }
     if ((PER || g.per[2]) && len == g.nz) {
         // the segment is a whole z-periodic row: a particle's chord may wrap
         // around inside it, so the arms are taken per cell
-        whole_row_forces(a, w0, w1, v0, v1, sx, sy, za, zb, fx, fy, fz);
+        forces_by_cell_far(a, PairForce{Fx, Fy, Fz, s0, s1, vslot, (n0 > 0 && s0 < 0) || (n1 > 0 && s1 < 0), vrh, vrl0, vrl1},
+                           sx, sy, za, zb);
         return;
     }
     // runs of equal owner, arms from the segment's middle point zc
@@ -1506,21 +1564,7 @@ __device__ __forceinline__ void collide_segment_pairs(const CollideArgs<float>& 
         if (ka < 0) va[q] = 0.f;
         if (kb < 0) vb[q] = 0.f;
     }
-    if constexpr (FOLD) {
-        const bool one = __all_sync(FULL, ka < 0 || kb < 0 || ka == kb);   // one reduction for both cells
-        if (one) {
-#pragma unroll
-            for (int q = 0; q < 5; ++q) va[q] += vb[q];
-        }
-#pragma unroll 1
-        for (int pass = 0; pass < (one ? 1 : 2); ++pass) {
-            float v[5];
-#pragma unroll
-            for (int q = 0; q < 5; ++q) v[q] = pass == 0 ? va[q] : vb[q];
-            const bool second = pass == 1 || (one && ka < 0);   // the run's cells are the b cells
-            reduce_runs(a, second ? kb : ka, v, second ? zb : za, sx, sy, zc, vrh, vrl0, vrl1, vslot);
-        }
-    } else if (__all_sync(FULL, ka < 0 || kb < 0 || ka == kb)) {
+    if (__all_sync(FULL, ka < 0 || kb < 0 || ka == kb)) {
         const int key = ka >= 0 ? ka : kb;
 #pragma unroll
         for (int q = 0; q < 5; ++q) va[q] += vb[q];
@@ -1528,6 +1572,206 @@ __device__ __forceinline__ void collide_segment_pairs(const CollideArgs<float>& 
     } else {
         reduce_runs(a, ka, va, za, sx, sy, zc, vrh, vrl0, vrl1, vslot);
         reduce_runs(a, kb, vb, zb, sx, sy, zc, vrh, vrl0, vrl1, vslot);
+    }
+}
+
+// ---------------------------------------------------------------------------
+// FP32 form without staging: lattices whose rows are not 16-byte aligned, and
+// every batch.  Lane l takes the cells l and l + 32 of a 64-cell segment and reads and
+// writes global memory directly: every access is a coalesced 32-bit one whatever its
+// alignment, and a cell's source and target slots follow from its own index and its six
+// neighbours' displacements, so a segment needs no set-up.  (Staged, such rows cost a
+// bulk copy per row with its own lead, and halo elements put in place by hand: even / odd
+// phase of a 71x67x243 channel 34.8 / 54.7 us staged, 32.4 / 35.5 us here = 82 / 75 % of
+// the copy bandwidth; of 512 batched channels, 75.6 M cells, 2.80 / 5.27 and 2.61 /
+// 3.40 ms.)  16 warps per SM at 128 registers; 20 or 24 spill and are slower.
+// A segment lies in a z-row, or, in the even phase of a batch, which touches only each
+// cell's own slots, in an x-plane across its z-rows (the plane view: the lanes are filled
+// whatever the row length; force and torque then take per-cell arms).
+struct DirectCell {
+    unsigned own;      // index in the domain, also of its voxel word
+    int y, z;
+    unsigned dz[2];    // displacement of the neighbour at z - 1, z + 1 (wrapped)
+    unsigned wall;     // bit 0..5: no neighbour at x - 1, x + 1, y - 1, y + 1, z - 1, z + 1
+};
+// The walls that stand between a cell and its neighbour at (-cx, -cy, -cz).
+__host__ __device__ constexpr unsigned wall_bits(int i) {
+    return (cx(i) > 0 ? 1u : cx(i) < 0 ? 2u : 0u) | (cy(i) > 0 ? 4u : cy(i) < 0 ? 8u : 0u) |
+           (cz(i) > 0 ? 16u : cz(i) < 0 ? 32u : 0u);
+}
+// Slot that direction I of the cell is read from (odd phase): slot opp I of the
+// neighbour at x - c_I, or the cell's own slot I beyond a wall.  The value that streams
+// along I goes to the slot of opp I: in the AA pattern a cell reads and writes the same
+// slots.  dx, dy: displacements of the rows at x - 1, x + 1 and y - 1, y + 1; indices are
+// modulo 2^32.
+template <bool WALLS, int I>
+__device__ __forceinline__ float* direct_slot(float* F, unsigned N, const DirectCell& c, const unsigned (&dx)[2],
+                                              const unsigned (&dy)[2]) {
+    unsigned idx = c.own;
+    if constexpr (cz(I) != 0) idx += c.dz[cz(I) > 0 ? 0 : 1];
+    unsigned d = 0;
+    if constexpr (cx(I) != 0) d += dx[cx(I) > 0 ? 0 : 1];
+    if constexpr (cy(I) != 0) d += dy[cy(I) > 0 ? 0 : 1];
+    float* p = F + (unsigned long long)opp(I) * N + (idx + d);
+    if (WALLS && (c.wall & wall_bits(I))) p = F + (unsigned long long)I * N + c.own;
+    return p;
+}
+
+template <bool ODD, bool FORCE, bool BATCH>
+__global__ void __launch_bounds__(DIRECT_BLOCK, DIRECT_BLOCKS_PER_SM)
+k_collide_direct(const CollideArgs<float> a1, long long nseg, const CollideArgs<float>* __restrict__ dargs,
+                 const int* __restrict__ seg0, int ndom) {
+    constexpr bool PLANE = BATCH && !ODD;
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    const int lane = threadIdx.x & 31;
+    PairTables<BATCH ? NO_TABLES : 0> tb{false};
+    const int* sseg0 = nullptr;   // batch: the CTA's copy of seg0 (ndom <= SEG0_SMEM)
+    if constexpr (BATCH) {
+        int* m = reinterpret_cast<int*>(smem_raw);
+        if (ndom <= SEG0_SMEM) {
+            for (int k = threadIdx.x; k < ndom; k += blockDim.x) m[k] = __ldg(seg0 + k);
+            sseg0 = m;
+        }
+    } else {
+        tb.load(a1);
+        if (a1.probe_timeout) {
+            // test hook: every warp meets a wait that runs out (as in k_collide_staged), reports
+            // it and leaves; this kernel has no waits of its own
+            __shared__ unsigned long long probe[DIRECT_BLOCK / 32];
+            if (lane == 0) mbar_init(&probe[threadIdx.x >> 5], 1);
+            __syncthreads();
+            if (!mbar_wait(&probe[threadIdx.x >> 5], 0u, PROBE_WAIT) && lane == 0) atomicOr(a1.err, 0x20u);
+            return;
+        }
+    }
+    __syncthreads();
+    const unsigned warps = gridDim.x * (DIRECT_BLOCK / 32);
+    for (unsigned seg = blockIdx.x * (DIRECT_BLOCK / 32) + (threadIdx.x >> 5); seg < (unsigned)nseg; seg += warps) {
+        int d = 0, first = 0;
+        if constexpr (BATCH) {
+            if (sseg0) {
+                int lo = 0, hi = ndom - 1;
+                while (lo < hi) {
+                    const int mid = (lo + hi + 1) >> 1;
+                    if (sseg0[mid] <= (int)seg) lo = mid;
+                    else hi = mid - 1;
+                }
+                d = lo;
+                first = sseg0[d];
+            } else {
+                d = find_domain(seg0, ndom, (int)seg);
+                first = __ldg(seg0 + d);
+            }
+        }
+        const CollideArgs<float>& a = BATCH ? dargs[d] : a1;
+        // PLANE: a.g is the plane view (one row of ny nz cells per x), g the domain itself
+        Geom g = a.g;
+        if (PLANE) {
+            g.ny = a.flat_ny;
+            g.nz = a.flat_nz;
+        }
+        const unsigned N = (unsigned)g.N;   // 19 N floats fit the memory, so N < 2^32
+        const unsigned sg = seg - (unsigned)first;
+        const unsigned row = fast_div(sg, a.dz);
+        const int z0 = (int)(sg - row * a.dz.d) * SEGW;
+        const int x = (int)fast_div(row, a.dy);
+        const int y = (int)(row - (unsigned)x * a.dy.d);
+        const unsigned rowbase = row * (unsigned)a.g.nz;
+        float* F = a.fo;
+        const float* Fin = a.f;
+        const unsigned unz = (unsigned)g.nz, xs = (unsigned)g.ny * unz;
+        const unsigned dx[2] = {x > 0 ? 0u - xs : (unsigned)(g.nx - 1) * xs,
+                                x < g.nx - 1 ? xs : 0u - (unsigned)(g.nx - 1) * xs};
+        const unsigned dy[2] = {y > 0 ? 0u - unz : xs - unz, y < g.ny - 1 ? unz : unz - xs};
+        unsigned wall = 0u;
+        if (ODD) {
+            if (!g.per[0]) wall |= (x == 0 ? 1u : 0u) | (x == g.nx - 1 ? 2u : 0u);
+            if (!g.per[1]) wall |= (y == 0 ? 4u : 0u) | (y == g.ny - 1 ? 8u : 0u);
+        }
+        DirectCell c[2];
+        bool valid[2];
+        uint32_t w[2];
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+            const int p = z0 + lane + 32 * h;
+            valid[h] = p < a.g.nz;
+            const int pc = valid[h] ? p : a.g.nz - 1;   // a lane slot past the row reads its last cell
+            DirectCell& q = c[h];
+            q.own = rowbase + (unsigned)pc;
+            w[h] = a.vox[q.own];
+            q.y = y;
+            q.z = pc;
+            if (PLANE) {
+                q.y = (int)fast_div((unsigned)pc, a.dnz);
+                q.z = pc - q.y * g.nz;
+            }
+            if (ODD) {
+                const bool lo = pc == 0, hi = pc == g.nz - 1;
+                q.dz[0] = lo ? unz - 1u : ~0u;
+                q.dz[1] = hi ? 1u - unz : 1u;
+                q.wall = wall;
+                if (!g.per[2]) q.wall |= (lo ? 16u : 0u) | (hi ? 32u : 0u);
+            }
+        }
+        F2 f[Q];
+        bool walls = false;
+        if constexpr (!ODD) {
+#pragma unroll
+            for (int i = 0; i < Q; ++i) {
+                const float* r = Fin + (unsigned long long)i * N;
+                f[i] = pk(r[c[0].own], r[c[1].own]);
+            }
+        } else {
+            walls = __any_sync(FULL, (c[0].wall | c[1].wall) != 0u);
+            float* R = const_cast<float*>(Fin);
+            auto load = [&](auto wc) {
+                constexpr bool WALLS = decltype(wc)::value;
+                unroll_seq(std::make_integer_sequence<int, Q>{}, [&](auto ic) {
+                    constexpr int i = decltype(ic)::value;
+                    f[i] = pk(*direct_slot<WALLS, i>(R, N, c[0], dx, dy), *direct_slot<WALLS, i>(R, N, c[1], dx, dy));
+                });
+            };
+            if (walls) load(std::true_type{});
+            else load(std::false_type{});
+        }
+        PairForce o;
+        collide_pair<FORCE>(a, g, tb, f, valid[0] ? w[0] : 0u, valid[1] ? w[1] : 0u, x, c[0].y, c[0].z, c[1].y, c[1].z,
+                            o);
+        if constexpr (!ODD) {
+#pragma unroll
+            for (int i = 0; i < Q; ++i) {
+                float* r = F + (unsigned long long)opp(i) * N;
+                const float2 t = upk(f[i]);
+                if (valid[0]) r[c[0].own] = t.x;
+                if (valid[1]) r[c[1].own] = t.y;
+            }
+        } else {
+            auto store = [&](auto wc) {
+                constexpr bool WALLS = decltype(wc)::value;
+                unroll_seq(std::make_integer_sequence<int, Q>{}, [&](auto ic) {
+                    constexpr int i = decltype(ic)::value;
+                    const float2 t = upk(f[i]);
+                    if (valid[0]) *direct_slot<WALLS, opp(i)>(F, N, c[0], dx, dy) = t.x;
+                    if (valid[1]) *direct_slot<WALLS, opp(i)>(F, N, c[1], dx, dy) = t.y;
+                });
+            };
+            if (walls) store(std::true_type{});
+            else store(std::false_type{});
+        }
+        if (a.cf) {
+            const float2 fx = upk(o.Fx), fy = upk(o.Fy), fz = upk(o.Fz);
+            if (valid[0]) { a.cf[c[0].own] = fx.x; a.cf[N + c[0].own] = fy.x; a.cf[2ull * N + c[0].own] = fz.x; }
+            if (valid[1]) { a.cf[c[1].own] = fx.y; a.cf[N + c[1].own] = fy.y; a.cf[2ull * N + c[1].own] = fz.y; }
+        }
+        if (PLANE) {
+            forces_by_cell(a, g, o, x, c[0].y, c[0].z, c[1].y, c[1].z);
+        } else if (g.per[2] && g.nz <= SEGW) {
+            // the segment is a whole z-periodic row: a particle's chord may wrap around inside
+            // it, so the arms are taken per cell
+            forces_by_cell_far(a, o, x, y, z0 + lane, z0 + lane + 32);
+        } else {
+            forces_by_run(a, o, x, y, z0 + SEGW / 2, z0 + lane, z0 + lane + 32);
+        }
     }
 }
 
@@ -1681,8 +1925,7 @@ __device__ __forceinline__ void collide_cell_staged(const CollideArgs<double>& a
 // warps, one 32-cell pass each: the stages of 8 warps fill the SM's shared memory, and
 // with two warps per scheduler the integer chains of a cell left half of the issue
 // slots empty.  The two take the longer (solid) pass in turn and do not wait for
-// each other at the end of a segment: a buffer is handed back through the stage's
-// `empty` barrier, so the warp with the shorter pass goes on to the next segment.
+// each other at the end of a segment: a buffer is handed back through a barrier, so the warp with the shorter pass goes on to the next segment.
 template <typename T, bool FORCE>
 __host__ __device__ constexpr int stage_warps() { return sizeof(T) == 8 && !FORCE ? 2 : 1; }
 
@@ -1711,14 +1954,16 @@ k_collide_staged(const CollideArgs<T> a1, long long nseg, const CollideArgs<T>* 
     const int group = warp / SW, sub = warp % SW;
     WarpStage<T, STAGE_UP>& st = reinterpret_cast<WarpStage<T, STAGE_UP>*>(smem_raw)[group];
     __shared__ unsigned long long probe[WARPS];   // the test hook's barrier (never completes)
+    // a shared stage's barriers: buffer b left by both warps [b]; its halo elements in place [2 + b]
+    __shared__ unsigned long long shared_bar[SW > 1 ? GROUPS : 1][4];
     if (lane == 0) {
         if (sub == 0) {
             mbar_init(&st.bar[0], 1);
             mbar_init(&st.bar[1], 1);
             if (SW > 1)
                 for (int q = 0; q < 2; ++q) {
-                    mbar_init(&st.empty[q], SW);
-                    mbar_init(&st.halo[q], 1);
+                    mbar_init(&shared_bar[group][q], SW);
+                    mbar_init(&shared_bar[group][2 + q], 1);
                 }
         }
         mbar_init(&probe[warp], 1);
@@ -1726,22 +1971,14 @@ k_collide_staged(const CollideArgs<T> a1, long long nseg, const CollideArgs<T>* 
     }
     if (SW > 1) __syncthreads();
     else __syncwarp();
-    bool smap_ok = false;   // the CTA holds a copy of the tag -> slot map (FP32, single lattice)
-    if constexpr (smem_tagmap<T, BATCH>()) {
-        int* m = reinterpret_cast<int*>(cta_tables<T, STAGE_UP>());
-        smap_ok = a1.max_tag < TAGMAP_SMEM - 1;
-        if (smap_ok)
-            for (int k = threadIdx.x; k < TAGMAP_SMEM; k += blockDim.x) {
-                const int v = k <= a1.max_tag ? __ldg(a1.tag2slot + k) : -1;
-                m[k] = (v >= 0 && v < a1.nslot) ? v : -1;
-            }
-        float* sb = reinterpret_cast<float*>(m + TAGMAP_SMEM);
-        for (int k = threadIdx.x; k < 126; k += blockDim.x) sb[k] = __ldg(a1.btab + k);
+    PairTables<STAGED_TABLES> tb{false};
+    if constexpr (sizeof(T) == 4) {
+        tb.load(a1);
         __syncthreads();   // every warp of the CTA reaches it (before any leaves)
     }
     const int* sseg0 = nullptr;   // batch: the CTA's copy of seg0 (ndom <= SEG0_SMEM)
     if constexpr (BATCH) {
-        int* m = reinterpret_cast<int*>(cta_tables<T, STAGE_UP>(GROUPS));
+        int* m = reinterpret_cast<int*>(smem_raw + GROUPS * sizeof(WarpStage<T, STAGE_UP>));
         if (ndom <= SEG0_SMEM) {
             for (int k = threadIdx.x; k < ndom; k += blockDim.x) m[k] = __ldg(seg0 + k);
             sseg0 = m;
@@ -1781,7 +2018,7 @@ k_collide_staged(const CollideArgs<T> a1, long long nseg, const CollideArgs<T>* 
     T hcur = T(0);
     if (sub == 0) hcur = issue(0, seg);
     uint32_t phase = 0;   // bit b: parity expected next on buffer b
-    uint32_t ephase = 0;  // the same for the `empty` barriers
+    uint32_t ephase = 0;  // the same for the barriers that hand a shared buffer back
     bool first = true;
     int b = 0;
     for (; seg < nseg; seg += stride, b ^= 1) {
@@ -1792,7 +2029,7 @@ k_collide_staged(const CollideArgs<T> a1, long long nseg, const CollideArgs<T>* 
         if (next < nseg && (SW == 1 || !lead_warp)) {
             // both warps have left the buffer's last segment (none before the first two)
             if (SW > 1 && !first) {
-                ok = mbar_wait(&st.empty[b ^ 1], (ephase >> (b ^ 1)) & 1u);
+                ok = mbar_wait(&shared_bar[group][b ^ 1], (ephase >> (b ^ 1)) & 1u);
                 ephase ^= 1u << (b ^ 1);
             }
             if (SW == 1 || __all_sync(FULL, ok)) hnext = issue(b ^ 1, next);
@@ -1855,9 +2092,9 @@ k_collide_staged(const CollideArgs<T> a1, long long nseg, const CollideArgs<T>* 
         if constexpr (SW > 1 && ODD && !PER) {
             // the other warp's cells read the halo elements that the lead warp put in place
             if (lead_warp) {
-                if (lane == 0) mbar_arrive(&st.halo[b]);
+                if (lane == 0) mbar_arrive(&shared_bar[group][2 + b]);
             } else {
-                ok = mbar_wait(&st.halo[b], (phase >> b & 1u) ^ 1u);   // phase was flipped above
+                ok = mbar_wait(&shared_bar[group][2 + b], (phase >> b & 1u) ^ 1u);   // phase was flipped above
             }
             if (__any_sync(FULL, !ok)) {
                 if (lane == 0) atomicOr(BATCH ? dargs[0].err : a1.err, 0x20u);   // LBDEM_DEVERR_TIMEOUT
@@ -1872,9 +2109,8 @@ k_collide_staged(const CollideArgs<T> a1, long long nseg, const CollideArgs<T>* 
                 if (cz(i) != 0 && st.row[b][row_slot(-cx(i), -cy(i))] >= 0) srcrow |= 1u << i;
         }
         if constexpr (sizeof(T) == 4) {
-            // FP32 form: packed pairs of cells (batch, even phase: plane segments)
-            collide_segment_pairs<ODD, FORCE, PER, MIS, STAGE_UP, BATCH && !ODD, BATCH>(
-                a, st, b, sx, sy, z0, len, srcrow, lead, smap_ok, smem_tagmap<T, BATCH>());
+            static_assert(LSU, "FP32: aligned rows of a single lattice (others: k_collide_direct)");
+            collide_segment_pairs<ODD, FORCE, PER, STAGE_UP>(a, st, b, sx, sy, z0, len, srcrow, tb);
         } else {
             // FP64 form: one cell per lane at a time; force and torque per cell with
             // double atomics.  The segment's solid cells are taken first (pass 0
@@ -1958,20 +2194,18 @@ k_collide_staged(const CollideArgs<T> a1, long long nseg, const CollideArgs<T>* 
         // populations in units) come before the copies that reuse it
         if constexpr (!LSU) asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
         __syncwarp();
-        if (SW > 1 && lane == 0) mbar_arrive(&st.empty[b]);
+        if (SW > 1 && lane == 0) mbar_arrive(&shared_bar[group][b]);
         hcur = hnext;
     }
 }
 
-template <typename T, bool ODD, bool FORCE, bool PER, bool MIS, bool BATCH>
-cudaError_t launch_staged(const CollideArgs<T>& a, long long nseg, const CollideArgs<T>* dargs,
-                          const int* seg0, int ndom, int blocks_per_sm, cudaStream_t s) {
-    constexpr int GROUPS = WARPS / stage_warps<T, FORCE>();   // stages (segments in work) per block
-    constexpr size_t smem =
-        GROUPS * sizeof(WarpStage<T, stage_up<T, BATCH>()>) + tagmap_bytes<T, BATCH>() + seg0_bytes<BATCH>();
+// A persistent grid of a kernel: as many blocks as fit the device (or blocks_per_sm of
+// them per SM), at most one per `per_block` segments.  `shape` is the kernel's own cache,
+// per device: (resident blocks per SM << 16) | SM count, 0 until first use there.
+template <typename Kernel>
+cudaError_t persistent_grid(Kernel kernel, int threads, size_t smem, std::atomic<int>* shape, long long nseg,
+                            int per_block, int blocks_per_sm, unsigned* grid) {
     if (nseg >= (1LL << 31)) return cudaErrorInvalidValue;   // segment indices are split in 32 bits
-    // per device: (resident blocks per SM << 16) | SM count, 0 until first use there
-    static std::atomic<int> shape[LBDEM_MAX_DEVICES];
     int dev = 0;
     cudaError_t e = cudaGetDevice(&dev);
     if (e != cudaSuccess) return e;
@@ -1981,51 +2215,78 @@ cudaError_t launch_staged(const CollideArgs<T>& a, long long nseg, const Collide
         int sms = 0, per_sm = 0;
         e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
         if (e == cudaSuccess)
-            e = cudaFuncSetAttribute(k_collide_staged<T, ODD, FORCE, PER, MIS, BATCH>,
-                                     cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-        if (e == cudaSuccess)
-            e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_collide_staged<T, ODD, FORCE, PER, MIS, BATCH>,
-                                                              COLLIDE_BLOCK, smem);
+            e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        if (e == cudaSuccess) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, threads, smem);
         if (e != cudaSuccess) return e;
         if (per_sm < 1) per_sm = 1;
         packed = (per_sm << 16) | (sms & 0xffff);
         shape[dev].store(packed, std::memory_order_relaxed);
     }
     const int per_sm = packed >> 16, sms = packed & 0xffff;
-    if (nseg <= 0) return cudaSuccess;
     const int use = (blocks_per_sm > 0 && blocks_per_sm < per_sm) ? blocks_per_sm : per_sm;
     const long long want = (long long)sms * use;
-    const long long blocks = (nseg + GROUPS - 1) / GROUPS;
-    const unsigned grid = (unsigned)(blocks < want ? blocks : want);
+    const long long blocks = (nseg + per_block - 1) / per_block;
+    *grid = (unsigned)(blocks < want ? blocks : want);
+    return cudaSuccess;
+}
+
+template <typename T, bool ODD, bool FORCE, bool PER, bool MIS, bool BATCH>
+cudaError_t launch_staged(const CollideArgs<T>& a, long long nseg, const CollideArgs<T>* dargs,
+                          const int* seg0, int ndom, int blocks_per_sm, cudaStream_t s) {
+    constexpr int GROUPS = WARPS / stage_warps<T, FORCE>();   // stages (segments in work) per block
+    constexpr size_t smem =
+        GROUPS * sizeof(WarpStage<T, stage_up<T, BATCH>()>) + (sizeof(T) == 4 ? TAGMAP_BYTES : 0) +
+        (BATCH ? SEG0_BYTES : 0);
+    static std::atomic<int> shape[LBDEM_MAX_DEVICES];
+    unsigned grid = 0;
+    const cudaError_t e = persistent_grid(k_collide_staged<T, ODD, FORCE, PER, MIS, BATCH>, COLLIDE_BLOCK, smem, shape,
+                                          nseg, GROUPS, blocks_per_sm, &grid);
+    if (e != cudaSuccess || grid == 0) return e;
     k_collide_staged<T, ODD, FORCE, PER, MIS, BATCH><<<grid, COLLIDE_BLOCK, smem, s>>>(a, nseg, dargs, seg0, ndom);
+    return cudaGetLastError();
+}
+
+template <bool ODD, bool FORCE, bool BATCH>
+cudaError_t launch_direct(const CollideArgs<float>& a, long long nseg, const CollideArgs<float>* dargs, const int* seg0,
+                        int ndom, int blocks_per_sm, cudaStream_t s) {
+    constexpr size_t smem = BATCH ? SEG0_BYTES : TAGMAP_BYTES;
+    static std::atomic<int> shape[LBDEM_MAX_DEVICES];
+    unsigned grid = 0;
+    const cudaError_t e = persistent_grid(k_collide_direct<ODD, FORCE, BATCH>, DIRECT_BLOCK, smem, shape, nseg,
+                                          DIRECT_BLOCK / 32, blocks_per_sm, &grid);
+    if (e != cudaSuccess || grid == 0) return e;
+    k_collide_direct<ODD, FORCE, BATCH><<<grid, DIRECT_BLOCK, smem, s>>>(a, nseg, dargs, seg0, ndom);
     return cudaGetLastError();
 }
 
 template <typename T, bool ODD, bool FORCE>
 cudaError_t launch_one(const CollideArgs<T>& args, cudaStream_t s) {
-    const int nzseg = (args.g.nz + SEGW - 1) / SEGW;
     CollideArgs<T> a = args;
+    // Aligned rows: every row start and length 16-byte aligned for population rows
+    // (nz * sizeof(T)) and voxel-word rows (nz * 4), i.e. nz % 4 == 0, and 16-byte
+    // aligned arrays (device allocations are; a caller's out-of-place target that is
+    // not takes the other path)
+    const bool arrays_aligned = (((uintptr_t)a.f | (uintptr_t)a.fo | (uintptr_t)a.vox | (uintptr_t)a.up) & 15u) == 0;
+    const bool aligned = a.g.nz % 4 == 0 && arrays_aligned;
+    const int nzseg = (a.g.nz + SEGW - 1) / SEGW;
     a.dz = div_magic((unsigned)nzseg);
     a.dy = div_magic((unsigned)a.g.ny);
     const long long nseg = (long long)a.g.nx * a.g.ny * nzseg;
-    // Aligned bulk copies need every row start and length 16-byte aligned:
-    // population rows (nz * sizeof(T)) and voxel-word rows (nz * 4), i.e. nz % 4 == 0,
-    // and 16-byte aligned arrays (device allocations are; a caller's out-of-place
-    // target that is not takes the unaligned-row path)
-    const bool arrays_aligned = (((uintptr_t)a.f | (uintptr_t)a.fo | (uintptr_t)a.vox | (uintptr_t)a.up) & 15u) == 0;
-    if (a.g.nz % 4 == 0 && arrays_aligned) {
+    if (aligned) {
         if (a.g.per[0] && a.g.per[1] && a.g.per[2])
             return launch_staged<T, ODD, FORCE, true, false, false>(a, nseg, nullptr, nullptr, 0, 0, s);
         return launch_staged<T, ODD, FORCE, false, false, false>(a, nseg, nullptr, nullptr, 0, 0, s);
     }
-    return launch_staged<T, ODD, FORCE, false, true, false>(a, nseg, nullptr, nullptr, 0, 0, s);
+    if constexpr (sizeof(T) == 8) return launch_staged<T, ODD, FORCE, false, true, false>(a, nseg, nullptr, nullptr, 0, 0, s);
+    else return launch_direct<ODD, FORCE, false>(a, nseg, nullptr, nullptr, 0, 0, s);
 }
 
 template <typename T, bool ODD, bool FORCE>
 cudaError_t launch_batch(const CollideArgs<T>* dargs, const int* seg0, int ndom, long long nseg, int blocks_per_sm,
                          cudaStream_t s) {
     CollideArgs<T> none{};
-    return launch_staged<T, ODD, FORCE, false, true, true>(none, nseg, dargs, seg0, ndom, blocks_per_sm, s);
+    if constexpr (sizeof(T) == 4) return launch_direct<ODD, FORCE, true>(none, nseg, dargs, seg0, ndom, blocks_per_sm, s);
+    else return launch_staged<T, ODD, FORCE, false, true, true>(none, nseg, dargs, seg0, ndom, blocks_per_sm, s);
 }
 
 }  // namespace
