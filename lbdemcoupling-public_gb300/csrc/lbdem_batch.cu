@@ -784,6 +784,7 @@ lbdem_status lbdem_batch_get_field(lbdem_batch* b, int32_t domain, int32_t which
     }
     switch (which) {
         case LBDEM_FIELD_POPULATIONS:
+            populate_host(host_buf, Q * N * b->esz);
             for (int i = 0; i < Q; ++i) {
                 if (b->prec == LBDEM_PREC_FP64)
                     BK(b, launch_pop_gather<double>(fptr<double>(b, domain), (double*)b->scratch, i, phase, v.g, s));
@@ -804,10 +805,12 @@ lbdem_status lbdem_batch_get_field(lbdem_batch* b, int32_t domain, int32_t which
             b->launches += 1;
             const size_t bytes =
                 which == LBDEM_FIELD_SOLID_FRACTION ? N * 8 : which == LBDEM_FIELD_PARTICLE_ID ? N * 4 : N;
+            populate_host(host_buf, bytes);
             BK(b, cudaMemcpyAsync(host_buf, b->scratch, bytes, cudaMemcpyDeviceToHost, s));
             break;
         }
         case LBDEM_FIELD_PARTICLE_VELOCITY:
+            populate_host(host_buf, 3 * N * b->esz);
             if (b->up) {
                 BK(b, cudaMemcpyAsync(host_buf, (char*)b->up + v.up0 * b->esz, 3 * N * b->esz, cudaMemcpyDeviceToHost,
                                       s));
@@ -828,6 +831,7 @@ lbdem_status lbdem_batch_get_field(lbdem_batch* b, int32_t domain, int32_t which
                 BK(b, launch_macro<float>(fptr<float>(b, domain), phase, vel ? nullptr : (double*)b->scratch,
                                           vel ? (double*)b->scratch : nullptr, v.g, s));
             b->launches += 1;
+            populate_host(host_buf, (vel ? 3 : 1) * N * sizeof(double));
             BK(b, cudaMemcpyAsync(host_buf, b->scratch, (vel ? 3 : 1) * N * sizeof(double), cudaMemcpyDeviceToHost, s));
             break;
         }

@@ -3,7 +3,11 @@
 #include "lbdem_gpu.h"
 #include "lbdem_internal.h"
 
+#include <sys/mman.h>
+#include <unistd.h>
+
 #include <algorithm>
+#include <cerrno>
 #include <cmath>
 #include <cstdio>
 #include <cstring>
@@ -16,6 +20,18 @@ using namespace lbdem;
 
 namespace lbdem {
 std::atomic<int> g_alloc_fail_countdown{0};
+
+void populate_host(void* p, size_t bytes) {
+#ifndef MADV_POPULATE_WRITE
+#define MADV_POPULATE_WRITE 23
+#endif
+    const uintptr_t page = (uintptr_t)sysconf(_SC_PAGESIZE);
+    if (bytes < 4 * page) return;   // a few faults cost less than the call is worth
+    const uintptr_t a = (uintptr_t)p & ~(page - 1);
+    const int saved = errno;
+    madvise((void*)a, (uintptr_t)p + bytes - a, MADV_POPULATE_WRITE);
+    errno = saved;
+}
 }
 
 namespace {
@@ -616,6 +632,7 @@ lbdem_status lbdem_get_field(lbdem_handle* h, int32_t which, void* host_buf) {
                 else
                     CK(h, launch_pop_gather<float>((const float*)h->f, (float*)h->scratch, i, phase, h->g, s));
                 h->launches += 1;
+                populate_host((char*)host_buf + (size_t)i * N * h->esz, N * h->esz);
                 CK(h, cudaMemcpyAsync((char*)host_buf + (size_t)i * N * h->esz, h->scratch, N * h->esz,
                                       cudaMemcpyDeviceToHost, s));
             }
@@ -630,10 +647,12 @@ lbdem_status lbdem_get_field(lbdem_handle* h, int32_t which, void* host_buf) {
             CK(h, launch_vox_fields(h->vox, sf, id, ns, h->g, s));
             h->launches += 1;
             const size_t bytes = which == LBDEM_FIELD_SOLID_FRACTION ? N * 8 : which == LBDEM_FIELD_PARTICLE_ID ? N * 4 : N;
+            populate_host(host_buf, bytes);
             CK(h, cudaMemcpyAsync(host_buf, h->scratch, bytes, cudaMemcpyDeviceToHost, s));
             break;
         }
         case LBDEM_FIELD_PARTICLE_VELOCITY:
+            populate_host(host_buf, 3 * N * h->esz);
             if (h->up) {
                 CK(h, cudaMemcpyAsync(host_buf, h->up, 3 * N * h->esz, cudaMemcpyDeviceToHost, s));
             } else {   // FP32 form: recomputed from the owner particles of the current list
@@ -646,6 +665,7 @@ lbdem_status lbdem_get_field(lbdem_handle* h, int32_t which, void* host_buf) {
             break;
         case LBDEM_FIELD_HYDRO_FORCE:
             if (!h->cf) return fail(h, LBDEM_ERR_INVALID_ARG, "get_field: create with LBDEM_FLAG_CELL_FORCE");
+            populate_host(host_buf, 3 * N * h->esz);
             CK(h, cudaMemcpyAsync(host_buf, h->cf, 3 * N * h->esz, cudaMemcpyDeviceToHost, s));
             break;
         case LBDEM_FIELD_DENSITY:
@@ -659,6 +679,7 @@ lbdem_status lbdem_get_field(lbdem_handle* h, int32_t which, void* host_buf) {
                 CK(h, launch_macro<float>((const float*)h->f, phase, vel ? nullptr : (double*)h->scratch,
                                           vel ? (double*)h->scratch : nullptr, h->g, s));
             h->launches += 1;
+            populate_host(host_buf, (vel ? 3 : 1) * N * sizeof(double));
             CK(h, cudaMemcpyAsync(host_buf, h->scratch, (vel ? 3 : 1) * N * sizeof(double), cudaMemcpyDeviceToHost, s));
             break;
         }
@@ -1014,6 +1035,7 @@ lbdem_status lbdem_adjoint_window(lbdem_handle* h, int32_t nsteps, int32_t K, in
     double glob[4];
     CK(h, cudaMemcpyAsync(loss, d_loss, sizeof(double), cudaMemcpyDeviceToHost, s));
     CK(h, cudaMemcpyAsync(glob, d_glob, 4 * sizeof(double), cudaMemcpyDeviceToHost, s));
+    if (grad_f0) populate_host(grad_f0, pop);
     if (n > 0) CK(h, cudaMemcpyAsync(grad_vel, d_gv, nrec * 6 * sizeof(double), cudaMemcpyDeviceToHost, s));
     if (grad_f0) CK(h, cudaMemcpyAsync(grad_f0, lam_in, pop, cudaMemcpyDeviceToHost, s));
     CK(h, cudaMemcpyAsync(h->h_err, h->d_err, sizeof(unsigned), cudaMemcpyDeviceToHost, s));
