@@ -23,12 +23,18 @@
 // 2^-958 are left out too.  A cell outside the range, or with a NaN or infinity,
 // takes the double routine: fits() tells, from the cell's own values alone.
 //
-// The update is the one of collide_cell_fp64 (k_collide.cu), regrouped as
-//   out_i = feq_i + A g_i + B (g_k - Dl_i),   A = (1 - omega)(1 - B),
-//   out_0 = feq_0 + (A + B) g_0 + B Dl_0,
-//   F = B (j - P)
-// (the pair terms of the momentum exchange summed over c_k:
-//  sum_k c_k (f_k - f_i) = j and sum_k 3 t c_k (c_k.(j + P)) = (j + P) / 2).
+// The update (src/ibCompositeDynamics3D.hh:130-203 with the Guo force in the base BGK) is
+// regrouped, with g = f - feq(J), J = j + rho g/2 (g the body force), S = feq + source,
+// j* = j + rho g below full coverage (else j) and P = rho uPart, as
+//   out_k = S_k + A g_k + B (f_i - feq_i(j*) + feq_k(P) - S_k),  A = (1 - omega)(1 - B),
+//   out_0 = S_0 + A g_0 + B (f_0 + feq_0(j*) - feq_0(P) - S_0),
+//   F = B (2 j - j* - P)
+// (the pair terms of the momentum exchange summed over c_k).  S is an equilibrium too: the
+// source's even part is that of the tensor M = pre (u g + g u), its odd part that of the
+// vector pre g, pre = (1 - omega/2) rho.  Without a body force S = feq, J = j* = j, and
+// with Dl = feq - feq(P) the same reads (6 % faster than through S)
+//   out_k = feq_k + A g_k + B (g_i - Dl_k),  out_0 = feq_0 + (A + B) g_0 + B Dl_0,
+//   F = B (j - P).
 #pragma once
 
 #include <cstdint>
@@ -125,9 +131,9 @@ LBDEM_HD i64 mul(const Split& a, const Split& b) {
     return shl((i64)a.h * b.h, 64 - S) + (t >> (S - 32));
 }
 
-// omega's part of a launch: 1 - omega in Q62 (omega in (0, 2)).
+// omega's part of a launch: 1 - omega and 1 - omega/2 in Q62 (omega in (0, 2)).
 struct Relax {
-    Split om1;
+    Split om1, hom;
 };
 LBDEM_HD i64 to_q62(double x) {   // |x| <= 1, exact to 2^-62
     const u64 b = bits_of(x);
@@ -135,7 +141,7 @@ LBDEM_HD i64 to_q62(double x) {   // |x| <= 1, exact to 2^-62
     const i64 s = (i64)b >> 63;
     return (i64)(m ^ (u64)s) - s;
 }
-LBDEM_HD Relax relax_of(double omega) { return Relax{split(to_q62(1.0 - omega))}; }
+LBDEM_HD Relax relax_of(double omega) { return Relax{split(to_q62(1.0 - omega)), split(to_q62(1.0 - 0.5 * omega))}; }
 
 // Symmetric second-order tensor in units: the diagonal (xx, yy, zz) and the mixed
 // entries (xy, yz, zx), each of them one place on when the axes are cycled.
@@ -240,25 +246,63 @@ LBDEM_HD void add_three(Sums& s, const i64 (&x)[6], bool last) {
 
 // What the update of a cell needs besides its populations.
 struct Cell {
-    Parts eq;       // feq
-    Parts df;       // feq - feqS (solid)
-    Split A, A0, B;
+    Parts eq;       // feq(J)
+    Parts fs;       // S (with a body force; else eq is taken)
+    Parts df;       // solid; with a body force feq(P) - feq(j*), odd parts added; else Dl
+    Split A, A0, B; // A0 = A + B (without a body force)
 };
 
 // From the sums of the cell's populations; returns the force in F (solid).
-// emax: cell_exponent() of the cell, at least EMAX_LO.
-LBDEM_HD Cell cell_setup(bool solid, i64 rb, i64 jx, i64 jy, i64 jz, int emax, const Relax& rx, double Bd, double up0,
-                         double up1, double up2, double (&F)[3]) {
+// emax: cell_exponent() of the cell, at least EMAX_LO.  gx, gy, gz: body force (FORCE);
+// full: n = 125.
+template <bool FORCE>
+LBDEM_HD Cell cell_setup(bool solid, const Sums& m, int emax, const Relax& rx, double gx, double gy, double gz,
+                         bool full, double Bd, double up0, double up1, double up2, double (&F)[3]) {
     Cell c;
     // rho = 1 + rhoBar in Q62: a unit is 2^(emax - 1079)
-    const i64 rbq = rb >> imin(1017 - emax, 63);
+    const i64 rbq = m.rb >> imin(1017 - emax, 63);
+    const Split rq = split(rbq);
     const int sh = imin(1018 - emax, 62);        // >= 1
     const i64 half = (i64)1 << (sh - 1);
-    const Split J[3] = {split(jx), split(jy), split(jz)};
-    {
-        const Split inv = split(reciprocal_q61(((i64)1 << 62) + rbq));
+    const Split inv = split(reciprocal_q61(((i64)1 << 62) + rbq));
+    i64 js[3] = {m.j[0], m.j[1], m.j[2]};        // j*
+    Tensor qs;                                   // j* j* / rho
+    if (FORCE) {
+        // rho g, J = j + rho g / 2 and pre g
+        const i64 g[3] = {to_fixed<4 + UP_BITS>(gx, emax), to_fixed<4 + UP_BITS>(gy, emax),
+                          to_fixed<4 + UP_BITS>(gz, emax)};
+        i64 J[3], pg[3];
+        Split JS[3], U[3], W[3];
+#pragma unroll
+        for (int a = 0; a < 3; ++a) {
+            const i64 rg = g[a] + mul<62>(split(g[a]), rq);
+            J[a] = m.j[a] + ((rg + 1) >> 1);
+            pg[a] = mul<62>(split(rg), rx.hom);
+            JS[a] = split(J[a]);
+            U[a] = split(mul<61>(JS[a], inv));
+            W[a] = split(pg[a]);
+            if (!full) js[a] += rg;
+        }
+        const Tensor q = tensor_of(JS, U, sh, half);
+        c.eq = parts_of(m.rb, q, J[0], J[1], J[2]);
+        Tensor s;
+#pragma unroll
+        for (int a = 0; a < 3; ++a) {
+            const int b = (a + 1) % 3;
+            s.d[a] = q.d[a] + ((mul<61>(U[a], W[a]) + (half >> 1)) >> (sh - 1));   // 2 u_a pre g_a
+            s.m[a] = q.m[a] + ((mul<61>(U[a], W[b]) + mul<61>(U[b], W[a]) + half) >> sh);
+        }
+        c.fs = parts_of(m.rb, s, J[0] + pg[0], J[1] + pg[1], J[2] + pg[2]);
+        if (solid) {
+            const Split S[3] = {split(js[0]), split(js[1]), split(js[2])};
+            const Split V[3] = {split(mul<61>(S[0], inv)), split(mul<61>(S[1], inv)), split(mul<61>(S[2], inv))};
+            qs = tensor_of(S, V, sh, half);
+        }
+    } else {
+        const Split J[3] = {split(m.j[0]), split(m.j[1]), split(m.j[2])};
         const Split U[3] = {split(mul<61>(J[0], inv)), split(mul<61>(J[1], inv)), split(mul<61>(J[2], inv))};
-        c.eq = parts_of(rb, tensor_of(J, U, sh, half), jx, jy, jz);
+        qs = tensor_of(J, U, sh, half);
+        c.eq = parts_of(m.rb, qs, m.j[0], m.j[1], m.j[2]);
     }
     c.A = c.A0 = rx.om1;
     c.B = Split{0, 0};
@@ -269,29 +313,30 @@ LBDEM_HD Cell cell_setup(bool solid, i64 rb, i64 jx, i64 jy, i64 jz, int emax, c
         c.B = split(Bq);
         const i64 Aq = (shl(rx.om1.h, 32) + rx.om1.l) - mul<62>(rx.om1, c.B);
         c.A = split(Aq);
-        c.A0 = split(Aq + Bq);
+        if (!FORCE) c.A0 = split(Aq + Bq);
         const i64 u[3] = {to_fixed<4 + UP_BITS>(up0, emax), to_fixed<4 + UP_BITS>(up1, emax),
                           to_fixed<4 + UP_BITS>(up2, emax)};
         const Split U[3] = {split(u[0]), split(u[1]), split(u[2])};
-        const Split rq = split(rbq);
         const i64 P[3] = {u[0] + mul<62>(U[0], rq), u[1] + mul<62>(U[1], rq), u[2] + mul<62>(U[2], rq)};
         const Split PS[3] = {split(P[0]), split(P[1]), split(P[2])};
         Tensor d = tensor_of(PS, U, sh, half);   // P P / rho, P = rho u_p
 #pragma unroll
         for (int a = 0; a < 3; ++a) {
-            d.d[a] = c.eq.q.d[a] - d.d[a];
-            d.m[a] = c.eq.q.m[a] - d.m[a];
+            d.d[a] = FORCE ? d.d[a] - qs.d[a] : qs.d[a] - d.d[a];
+            d.m[a] = FORCE ? d.m[a] - qs.m[a] : qs.m[a] - d.m[a];
         }
-        const i64 v[3] = {jx - P[0], jy - P[1], jz - P[2]};
-        c.df = parts_of(0, d, v[0], v[1], v[2]);
+        const i64 v[3] = {m.j[0] - P[0], m.j[1] - P[1], m.j[2] - P[2]};
+        if (FORCE) c.df = parts_of(0, d, js[0] + P[0], js[1] + P[1], js[2] + P[2]);
+        else c.df = parts_of(0, d, v[0], v[1], v[2]);
 #pragma unroll
-        for (int a = 0; a < 3; ++a) F[a] = to_double(mul<62>(split(v[a]), c.B), emax);
+        for (int a = 0; a < 3; ++a)
+            F[a] = to_double(mul<62>(split(FORCE ? v[a] - (js[a] - m.j[a]) : v[a]), c.B), emax);
     }
     return c;
 }
 
-// eq + a g + b h, both products rounded together.
-LBDEM_HD double relaxed(bool solid, i64 eq, i64 g, const Split& a, i64 h, const Split& b, int emax) {
+// s + a g + b h, both products rounded together.
+LBDEM_HD double relaxed(bool solid, i64 s0, i64 g, const Split& a, i64 h, const Split& b, int emax) {
     const Split gs = split(g);
     i64 t = (i64)gs.h * a.l + ((i64)gs.l * a.h + ((i64)1 << 29));
     i64 s = (i64)gs.h * a.h;
@@ -300,18 +345,28 @@ LBDEM_HD double relaxed(bool solid, i64 eq, i64 g, const Split& a, i64 h, const 
         t = (i64)hs.h * b.l + ((i64)hs.l * b.h + t);
         s = (i64)hs.h * b.h + s;
     }
-    return to_double(eq + shl(s, 2) + (t >> 30), emax);
+    return to_double(s0 + shl(s, 2) + (t >> 30), emax);
 }
+template <bool FORCE>
 LBDEM_HD double update_rest(bool solid, const Cell& c, i64 X0, int emax) {
+    if (FORCE) return relaxed(solid, c.fs.b3, X0 - c.eq.b3, c.A, X0 - c.df.b3 - c.fs.b3, c.B, emax);
     return relaxed(solid, c.eq.b3, X0 - c.eq.b3, c.A0, c.df.b3, c.B, emax);
 }
-// One pair (k, i): populations in units in, doubles out.
-LBDEM_HD void update_pair(bool solid, const Cell& c, i64 C, i64 L, i64 Cd, i64 Ld, i64 Xk, i64 Xi, int emax,
-                          double& fk, double& fi) {
-    const i64 ek = C + L, ei = C - L;
-    const i64 gk = Xk - ek, gi = Xi - ei;
-    fk = relaxed(solid, ek, gk, c.A, gi - (Cd + Ld), c.B, emax);
-    fi = relaxed(solid, ei, gi, c.A, gk - (Cd - Ld), c.B, emax);
+// One pair (k, i): populations in units in, doubles out; feq = C +- L, S = Cs +- Ls (with a
+// body force), the solid parts Cd +- Ld.
+template <bool FORCE>
+LBDEM_HD void update_pair(bool solid, const Cell& c, i64 C, i64 L, i64 Cs, i64 Ls, i64 Cd, i64 Ld, i64 Xk, i64 Xi,
+                          int emax, double& fk, double& fi) {
+    if (!FORCE) {
+        const i64 ek = C + L, ei = C - L;
+        const i64 gk = Xk - ek, gi = Xi - ei;
+        fk = relaxed(solid, ek, gk, c.A, gi - (Cd + Ld), c.B, emax);
+        fi = relaxed(solid, ei, gi, c.A, gk - (Cd - Ld), c.B, emax);
+        return;
+    }
+    const i64 sk = Cs + Ls, si = Cs - Ls;
+    fk = relaxed(solid, sk, Xk - (C + L), c.A, (Xi - sk) + (Cd + Ld), c.B, emax);
+    fi = relaxed(solid, si, Xi - (C - L), c.A, (Xk - si) + (Cd - Ld), c.B, emax);
 }
 
 // The three pairs of the current cycle: X(q) is a population in units, put(q, f) takes
@@ -319,24 +374,31 @@ LBDEM_HD void update_pair(bool solid, const Cell& c, i64 C, i64 L, i64 Cd, i64 L
 // additions: the FP64 pipe is otherwise idle, and 38 additions cost it less time than
 // integer conversions take (128^3 cycle 586, 567, 550, 543 us with none, one, two and
 // all three pairs converted this way).
-template <typename In, typename Out>
-LBDEM_HD void update_three(bool solid, const Cell& c, const Three& e, const Three& d, const In& X, int emax,
-                           const Out& put) {
+template <bool FORCE, typename In, typename Out>
+LBDEM_HD void update_three(bool solid, Cell& c, bool last, const In& X, int emax, const Out& put) {
+    const Three e = three_of(c.eq, last);
+    Three s = e, d{};
+    if (FORCE) s = three_of(c.fs, last);
+    if (solid) d = three_of(c.df, last);
     double fk, fi;
 #pragma unroll
     for (int q = 0; q < 3; ++q) {
-        update_pair(solid, c, e.C[q], e.L[q], d.C[q], d.L[q], X(2 * q), X(2 * q + 1), emax, fk, fi);
+        update_pair<FORCE>(solid, c, e.C[q], e.L[q], s.C[q], s.L[q], d.C[q], d.L[q], X(2 * q), X(2 * q + 1), emax, fk, fi);
         put(2 * q, fk);
         put(2 * q + 1, fi);
     }
+    cycle(c.eq);
+    if (FORCE) cycle(c.fs);
+    if (solid) cycle(c.df);
 }
 
-// One cell with its populations in an array; cell.f[i] of the kernel's loops.
-// solid adds the solid correction with the weight B and the surface velocity
+// One cell with its populations in an array (the kernel runs the same loops over its
+// stage).  solid adds the solid correction with the weight B and the surface velocity
 // (up0, up1, up2); a fluid cell (B = 0, up = 0) gets the same bits either way.
 // emax: cell_exponent() of the same values, fits(emax).
-LBDEM_HD void collide(bool solid, double (&f)[19], int emax, const Relax& rx, double B, double up0, double up1,
-                      double up2, double (&F)[3]) {
+template <bool FORCE>
+LBDEM_HD void collide(bool solid, double (&f)[19], int emax, const Relax& rx, double gx, double gy, double gz,
+                      bool full, double B, double up0, double up1, double up2, double (&F)[3]) {
     emax = imax(emax, EMAX_LO);
     i64 X[19];
 #pragma unroll
@@ -348,16 +410,12 @@ LBDEM_HD void collide(bool solid, double (&f)[19], int emax, const Relax& rx, do
                           X[dir_of(a, 3)], X[dir_of(a, 4)], X[dir_of(a, 5)]};
         add_three(s, x, a == 2);
     }
-    Cell c = cell_setup(solid, s.rb, s.j[0], s.j[1], s.j[2], emax, rx, B, up0, up1, up2, F);
-    f[0] = update_rest(solid, c, X[0], emax);
+    Cell c = cell_setup<FORCE>(solid, s, emax, rx, gx, gy, gz, full, B, up0, up1, up2, F);
+    f[0] = update_rest<FORCE>(solid, c, X[0], emax);
 #pragma unroll
-    for (int a = 0; a < 3; ++a) {
-        const Three e = three_of(c.eq, a == 2), d = three_of(c.df, a == 2);
-        update_three(solid, c, e, d, [&](int q) { return X[dir_of(a, q)]; }, emax,
-                     [&](int q, double v) { f[dir_of(a, q)] = v; });
-        cycle(c.eq);
-        cycle(c.df);
-    }
+    for (int a = 0; a < 3; ++a)
+        update_three<FORCE>(solid, c, a == 2, [&](int q) { return X[dir_of(a, q)]; }, emax,
+                            [&](int q, double v) { f[dir_of(a, q)] = v; });
 }
 
 }  // namespace fixed

@@ -29,7 +29,7 @@
 // velocity of its solid cells from the owner particle's row of the float table
 // (no per-cell velocity field); the FP64 form one cell per thread, BGK and solid
 // correction in one pass in 64-bit fixed point (cell_fixed.h; a cell outside its range
-// in double, collide_cell_fp64; with a body force collide_cell in double), with the
+// in double, collide_cell_fp64 or, with a body force, collide_cell), with the
 // velocity setValues stored.  The same
 // kernel steps many independent domains in one launch (batch mode).
 #include "lbdem_internal.h"
@@ -184,25 +184,20 @@ __device__ __forceinline__ void psm(T (&f)[Q], const Mom<T>& m, T up0, T up1, T 
     }
 }
 
-// Collision of one cell given its pre-collision populations: BGK for every
-// cell below full coverage (src/ibCompositeDynamics3D.hh:139-140), then the
-// solid correction for cells with n > 0.  Written as two convergent blocks so
-// that a warp mixing fluid and solid cells runs the BGK once.  Without a body
-// force BGK conserves rhoBar and j, so the solid correction reuses the
-// pre-collision moments (the reference recomputes them from the post-collision
-// populations, :146-148; the two differ by rounding only); with the Guo force
-// the post-collision moments are recomputed.
-// up(d) returns component d of the cell's particle surface velocity.
-template <typename T, bool FORCE, typename Pre, typename Up>
-__device__ __forceinline__ void collide_cell(const CollideArgs<T>& a, T (&f)[Q], uint32_t w, const Pre& pre,
-                                             const Up& up, T& Fx, T& Fy, T& Fz) {
-    const int n = min((int)(w & VOX_NMASK), 125);
-    Fx = T(0); Fy = T(0); Fz = T(0);
-    Mom<T> m = cell_moments(f);
-    if (n < 125) bgk<T, FORCE>(f, m, a.omega, a.g3[0], a.g3[1], a.g3[2]);
+// Collision of one cell with a body force given its pre-collision populations: BGK for
+// every cell below full coverage (src/ibCompositeDynamics3D.hh:139-140), then the
+// solid correction for cells with n > 0, with the moments of the post-collision
+// populations (:146-148; the Guo force changes the momentum).  pre(i) returns fPre_i.
+template <typename Pre>
+__device__ __forceinline__ void collide_cell(double (&f)[Q], double omega, double gx, double gy, double gz, int n,
+                                             double B, double up0, double up1, double up2, const Pre& pre,
+                                             double (&F)[3]) {
+    F[0] = F[1] = F[2] = 0.0;
+    Mom<double> m = cell_moments(f);
+    if (n < 125) bgk<double, true>(f, m, omega, gx, gy, gz);
     if (n > 0) {
-        if (FORCE && n < 125) m = cell_moments(f);
-        psm<T>(f, m, up(0), up(1), up(2), __ldg(a.btab + n), pre, Fx, Fy, Fz);
+        if (n < 125) m = cell_moments(f);
+        psm<double>(f, m, up0, up1, up2, B, pre, F[0], F[1], F[2]);
     }
 }
 
@@ -1776,7 +1771,7 @@ k_collide_direct(const CollideArgs<float> a1, long long nseg, const CollideArgs<
 }
 
 // ---------------------------------------------------------------------------
-// FP64 form without a body force: one staged cell (lane's cell j of the segment in
+// FP64 form: one staged cell (lane's cell j of the segment in
 // buffer b), evaluated in fixed point (cell_fixed.h) from the stage and stored.
 // The loop bodies cover the three direction pairs of one axis and run three times
 // (the axes are cycled in between), over values kept in the stage: fully unrolled
@@ -1829,19 +1824,21 @@ struct StagedCell {
 };
 
 // The double routine for a cell outside the fixed-point range, out of line.
-template <bool ODD, bool PER, bool MIS, bool STAGE_UP>
-__device__ __noinline__ void collide_cell_double(StagedCell<ODD, PER, MIS, STAGE_UP> s, double omega, double B,
-                                                 double u0, double u1, double u2, double (&F)[3]) {
+template <bool ODD, bool FORCE, bool PER, bool MIS, bool STAGE_UP>
+__device__ __noinline__ void collide_cell_double(StagedCell<ODD, PER, MIS, STAGE_UP> s, double omega, double g0,
+                                                 double g1, double g2, int n, double B, double u0, double u1,
+                                                 double u2, double (&F)[3]) {
     double f[Q];
 #pragma unroll
     for (int i = 0; i < Q; ++i) f[i] = *s.at(i, cz(i));
-    collide_cell_fp64<true>(f, omega, B, u0, u1, u2, F[0], F[1], F[2]);
+    if constexpr (FORCE) collide_cell(f, omega, g0, g1, g2, n, B, u0, u1, u2, [&](int i) { return *s.at(i, cz(i)); }, F);
+    else collide_cell_fp64<true>(f, omega, B, u0, u1, u2, F[0], F[1], F[2]);
     s.fo[s.c] = f[0];
 #pragma unroll
     for (int i = 1; i < Q; ++i) *s.slot(i, opp(i), row_slot(cx(i), cy(i)), cz(i)) = f[i];
 }
 
-template <bool ODD, bool PER, bool MIS, bool STAGE_UP>
+template <bool ODD, bool FORCE, bool PER, bool MIS, bool STAGE_UP>
 __device__ __forceinline__ void collide_cell_staged(const CollideArgs<double>& a, WarpStage<double, STAGE_UP>& st,
                                                     int b, int j, int z0, uint32_t srcrow, unsigned long long lead,
                                                     uint32_t w, bool solid, double (&F)[3]) {
@@ -1875,8 +1872,9 @@ __device__ __forceinline__ void collide_cell_staged(const CollideArgs<double>& a
         u2 = s.up(2, j);
         e = fixed::cell_exponent_up(e, u0, u1, u2);
     }
+    if (FORCE) e = fixed::cell_exponent_up(e, a.g3[0], a.g3[1], a.g3[2]);
     if (!fixed::fits(e)) {
-        collide_cell_double<ODD, PER, MIS, STAGE_UP>(s, a.omega, B, u0, u1, u2, F);
+        collide_cell_double<ODD, FORCE, PER, MIS, STAGE_UP>(s, a.omega, a.g3[0], a.g3[1], a.g3[2], n, B, u0, u1, u2, F);
         return;
     }
     e = max(e, fixed::EMAX_LO);
@@ -1904,37 +1902,32 @@ __device__ __forceinline__ void collide_cell_staged(const CollideArgs<double>& a
         }
         fixed::add_three(sum, x, t == 2);
     }
-    fixed::Cell cell = fixed::cell_setup(solid, sum.rb, sum.j[0], sum.j[1], sum.j[2], e,
-                                          fixed::relax_of(a.omega), B, u0, u1, u2, F);
-    a.fo[s.c] = fixed::update_rest(solid, cell, X0, e);
+    fixed::Cell cell = fixed::cell_setup<FORCE>(solid, sum, e, fixed::relax_of(a.omega), a.g3[0], a.g3[1], a.g3[2],
+                                                n == 125, B, u0, u1, u2, F);
+    a.fo[s.c] = fixed::update_rest<FORCE>(solid, cell, X0, e);
 #pragma unroll 1
     for (int t = 0, dg = 0; t < 3; dg = t == 0 ? 4 : 2, ++t) {
-        const fixed::Three eq = fixed::three_of(cell.eq, t == 2);
-        fixed::Three df{};
-        if (solid) df = fixed::three_of(cell.df, t == 2);
-        fixed::update_three(
-            solid, cell, eq, df,
+        fixed::update_three<FORCE>(
+            solid, cell, t == 2,
             [&](int q) { return *reinterpret_cast<const i64*>(s.at(dir(q, t, dg), dir_z(q, t))); }, e,
             [&](int q, double v) { *s.slot(dir(q, t, dg), dir(q ^ 1, t, dg), dir_row(q, t), dir_z(q, t)) = v; });
-        fixed::cycle(cell.eq);
-        if (solid) fixed::cycle(cell.df);
     }
 }
 
-// Warps per stage.  The FP64 form without a body force gives each segment to two
+// Warps per stage.  The FP64 form gives each segment to two
 // warps, one 32-cell pass each: the stages of 8 warps fill the SM's shared memory, and
 // with two warps per scheduler the integer chains of a cell left half of the issue
 // slots empty.  The two take the longer (solid) pass in turn and do not wait for
 // each other at the end of a segment: a buffer is handed back through a barrier, so the warp with the shorter pass goes on to the next segment.
-template <typename T, bool FORCE>
-__host__ __device__ constexpr int stage_warps() { return sizeof(T) == 8 && !FORCE ? 2 : 1; }
+template <typename T>
+__host__ __device__ constexpr int stage_warps() { return sizeof(T) == 8 ? 2 : 1; }
 
 // PER: every axis periodic (no wall cases; shifts and neighbour rows are fixed).
 // MIS: rows not 16-byte aligned (see issue_segment).
 // BATCH: segments of many domains, numbered domain after domain (seg0[d] is
 // the first segment of domain d); every domain has its own CollideArgs.
 template <typename T, bool ODD, bool FORCE, bool PER, bool MIS, bool BATCH>
-__global__ void __launch_bounds__(COLLIDE_BLOCK, sizeof(T) == 4 ? 4 : 2 * stage_warps<T, FORCE>())
+__global__ void __launch_bounds__(COLLIDE_BLOCK, sizeof(T) == 4 ? 4 : 2 * stage_warps<T>())
 k_collide_staged(const CollideArgs<T> a1, long long nseg, const CollideArgs<T>* __restrict__ dargs,
                  const int* __restrict__ seg0, int ndom) {
     constexpr int V = WarpStage<T>::V;
@@ -1949,7 +1942,7 @@ k_collide_staged(const CollideArgs<T> a1, long long nseg, const CollideArgs<T>* 
     const int lane = threadIdx.x & 31;
     const int warp = threadIdx.x >> 5;
     // SW warps share a stage: warp `sub` of group `group`
-    constexpr int SW = stage_warps<T, FORCE>();
+    constexpr int SW = stage_warps<T>();
     constexpr int GROUPS = WARPS / SW;
     const int group = warp / SW, sub = warp % SW;
     WarpStage<T, STAGE_UP>& st = reinterpret_cast<WarpStage<T, STAGE_UP>*>(smem_raw)[group];
@@ -2063,7 +2056,6 @@ k_collide_staged(const CollideArgs<T> a1, long long nseg, const CollideArgs<T>* 
         const Geom& g = a.g;
         const size_t N = g.N;
         const T* Fin = a.f;   // input populations
-        T* F = a.fo;          // output populations (== a.f in place)
         const size_t own = (size_t)st.row[b][row_slot(0, 0)];
         const unsigned long long lead = MIS ? st.lead[b] : 0ull;
         if (MIS && ODD) {
@@ -2135,58 +2127,17 @@ k_collide_staged(const CollideArgs<T> a1, long long nseg, const CollideArgs<T>* 
                 if (slot < ns) j = slot < ns0 ? nth_bit(sol0, slot) : 32 + nth_bit(sol1, slot - ns0);
                 else if (slot - ns < nf) j = slot - ns < nf0 ? nth_bit(flu0, slot - ns) : 32 + nth_bit(flu1, slot - ns - nf0);
                 const bool any_solid = ns > 32 * p;   // warp-uniform
-                T v[6] = {T(0), T(0), T(0), T(0), T(0), T(0)};
-                if constexpr (!FORCE) {
-                    if (j >= 0) {
-                        const uint32_t w = st.vox[b][vlead + j];
-                        T Fc[3];
-                        collide_cell_staged<ODD, PER, MIS, STAGE_UP>(a, st, b, j, z0, srcrow, lead, w, any_solid, Fc);
-                        const size_t c = own + z0 + j;
-                        if (a.cf) { a.cf[c] = Fc[0]; a.cf[N + c] = Fc[1]; a.cf[2 * N + c] = Fc[2]; }
-                        if (any_solid) {
-                            const int key = cell_force_terms(a, w, sx, sy, z0 + j, Fc[0], Fc[1], Fc[2], v);
-                            if (key >= 0) add_cell_force(a, key, v);
-                        }
-                    }
-                } else if (j >= 0) {
+                if (j >= 0) {
                     const uint32_t w = st.vox[b][vlead + j];
-                    const int z = z0 + j;
-                    const size_t c = own + z;
-                    // smem index of direction i: V + lead_i + j - shift_i, shift_i = c_z,i
-                    // when the source row x - c_i exists (odd phase)
-                    auto at = [&](int i) -> const T& {
-                        const int shift = (ODD && cz(i) != 0 && (PER || ((srcrow >> i) & 1u))) ? cz(i) : 0;
-                        const int m = MIS ? (int)((lead >> (2 * i)) & 3u) : 0;
-                        return st.f[b][i][V + m + j - shift];
-                    };
-                    T f[Q];
-#pragma unroll
-                    for (int i = 0; i < Q; ++i) f[i] = at(i);
-                    T Fx, Fy, Fz;
-                    auto upv = [&](int d) -> T {
-                        if (!STAGE_UP) return __ldg(a.up + (size_t)d * N + c);
-                        const int m = MIS ? (int)((lead >> (40 + 2 * d)) & 3u) : 0;
-                        return st.up[b][d][m + j];
-                    };
-                    collide_cell<T, FORCE>(a, f, w, [&](int i) { return at(i); }, upv, Fx, Fy, Fz);
-                    if (!ODD) {
-#pragma unroll
-                        for (int i = 0; i < Q; ++i) F[(size_t)opp(i) * N + c] = f[i];
-                    } else {
-                        F[c] = f[0];
-                        const int zm = wrap_minus(z, g.nz, PER ? 1 : g.per[2]);
-                        const int zp = wrap_plus(z, g.nz, PER ? 1 : g.per[2]);
-#pragma unroll
-                        for (int i = 1; i < Q; ++i) {
-                            const long long r = st.row[b][row_slot(cx(i), cy(i))];
-                            const int zd = pick(cz(i), zm, z, zp);
-                            if (PER || (r >= 0 && zd >= 0)) F[(size_t)i * N + (size_t)r + zd] = f[i];
-                            else F[(size_t)opp(i) * N + c] = f[i];
-                        }
+                    T Fc[3];
+                    collide_cell_staged<ODD, FORCE, PER, MIS, STAGE_UP>(a, st, b, j, z0, srcrow, lead, w, any_solid, Fc);
+                    const size_t c = own + z0 + j;
+                    if (a.cf) { a.cf[c] = Fc[0]; a.cf[N + c] = Fc[1]; a.cf[2 * N + c] = Fc[2]; }
+                    if (any_solid) {
+                        T v[6] = {T(0), T(0), T(0), T(0), T(0), T(0)};
+                        const int key = cell_force_terms(a, w, sx, sy, z0 + j, Fc[0], Fc[1], Fc[2], v);
+                        if (key >= 0) add_cell_force(a, key, v);
                     }
-                    if (a.cf) { a.cf[c] = Fx; a.cf[N + c] = Fy; a.cf[2 * N + c] = Fz; }
-                    const int key = cell_force_terms(a, w, sx, sy, z, Fx, Fy, Fz, v);
-                    if (key >= 0) add_cell_force(a, key, v);
                 }
             }
         }
@@ -2233,7 +2184,7 @@ cudaError_t persistent_grid(Kernel kernel, int threads, size_t smem, std::atomic
 template <typename T, bool ODD, bool FORCE, bool PER, bool MIS, bool BATCH>
 cudaError_t launch_staged(const CollideArgs<T>& a, long long nseg, const CollideArgs<T>* dargs,
                           const int* seg0, int ndom, int blocks_per_sm, cudaStream_t s) {
-    constexpr int GROUPS = WARPS / stage_warps<T, FORCE>();   // stages (segments in work) per block
+    constexpr int GROUPS = WARPS / stage_warps<T>();   // stages (segments in work) per block
     constexpr size_t smem =
         GROUPS * sizeof(WarpStage<T, stage_up<T, BATCH>()>) + (sizeof(T) == 4 ? TAGMAP_BYTES : 0) +
         (BATCH ? SEG0_BYTES : 0);

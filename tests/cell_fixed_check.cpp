@@ -78,6 +78,61 @@ static void collide(T (&f)[19], T omega, T B, const T (&up)[3], T (&F)[3]) {
     for (int a = 0; a < 3; ++a) F[a] = (B + B) * E[a];
 }
 
+// The update with a body force (k_collide.cu's collide_cell): BGK with the Guo force below
+// full coverage, then the solid correction with the moments of the result, statement by
+// statement (src/ibCompositeDynamics3D.hh:130-203).
+template <typename T>
+static void moments(const T (&f)[19], T& rb, T (&j)[3]) {
+    rb = 0;
+    j[0] = j[1] = j[2] = 0;
+    for (int i = 0; i < 19; ++i) {
+        rb += f[i];
+        if (CX[i]) j[0] += CX[i] * f[i];
+        if (CY[i]) j[1] += CY[i] * f[i];
+        if (CZ[i]) j[2] += CZ[i] * f[i];
+    }
+}
+template <typename T>
+static T feq(int i, T rb, const T (&j)[3]) {
+    const T t = i == 0 ? T(1) / T(3) : (i < 4 || (i > 9 && i < 13)) ? T(1) / T(18) : T(1) / T(36);
+    const T cj = CX[i] * j[0] + CY[i] * j[1] + CZ[i] * j[2];
+    const T jj = j[0] * j[0] + j[1] * j[1] + j[2] * j[2];
+    return t * (rb + T(3) * cj + (T(4.5) * cj * cj - T(1.5) * jj) / (T(1) + rb));
+}
+template <typename T>
+static void collide_force(T (&f)[19], T omega, const T (&g)[3], int n, T B, const T (&up)[3], T (&F)[3]) {
+    T pre[19], rb, j[3];
+    for (int i = 0; i < 19; ++i) pre[i] = f[i];
+    moments(f, rb, j);
+    if (n < 125) {
+        const T rho = T(1) + rb;
+        const T J[3] = {j[0] + T(0.5) * rho * g[0], j[1] + T(0.5) * rho * g[1], j[2] + T(0.5) * rho * g[2]};
+        const T u[3] = {J[0] / rho, J[1] / rho, J[2] / rho};
+        const T ug = u[0] * g[0] + u[1] * g[1] + u[2] * g[2];
+        for (int i = 0; i < 19; ++i) {
+            const T t = i == 0 ? T(1) / T(3) : (i < 4 || (i > 9 && i < 13)) ? T(1) / T(18) : T(1) / T(36);
+            const T cg = CX[i] * g[0] + CY[i] * g[1] + CZ[i] * g[2], cu = CX[i] * u[0] + CY[i] * u[1] + CZ[i] * u[2];
+            f[i] = (T(1) - omega) * f[i] + omega * feq<T>(i, rb, J) +
+                   t * (T(1) - T(0.5) * omega) * rho * (T(3) * (cg - ug) + T(9) * cu * cg);
+        }
+        moments(f, rb, j);
+    }
+    F[0] = F[1] = F[2] = 0;
+    if (n == 0) return;
+    const T P[3] = {up[0] * (T(1) + rb), up[1] * (T(1) + rb), up[2] * (T(1) + rb)};
+    f[0] = pre[0] + (T(1) - B) * (f[0] - pre[0]) + B * (feq<T>(0, rb, j) - feq<T>(0, rb, P));
+    for (int i = 1; i < 10; ++i) {
+        const int o = i + 9;
+        const T bb = B * ((pre[o] - feq<T>(o, rb, j)) - (pre[i] - feq<T>(i, rb, P)));
+        const T bo = B * ((pre[i] - feq<T>(i, rb, j)) - (pre[o] - feq<T>(o, rb, P)));
+        f[i] = pre[i] + (T(1) - B) * (f[i] - pre[i]) + bb;
+        f[o] = pre[o] + (T(1) - B) * (f[o] - pre[o]) + bo;
+        F[0] -= CX[i] * (bb - bo);
+        F[1] -= CY[i] * (bb - bo);
+        F[2] -= CZ[i] * (bb - bo);
+    }
+}
+
 struct Err {
     double mx = 0, sq = 0;
     long n = 0;
@@ -99,13 +154,16 @@ int main(int argc, char** argv) {
         const char* name;
         double rho, u, noise, up;   // density and velocity spread, non-equilibrium part, surface velocity spread
         bool solid;
+        double g;                   // body force spread
     };
     const Kind kinds[] = {
-        {"slow_fluid", 1e-5, 1e-4, 1e-7, 0, false},      {"fluid", 1e-3, 1e-2, 1e-5, 0, false},
-        {"fast_fluid", 1e-2, 5e-2, 1e-3, 0, false},      {"noise", 0, 0, 1e-3, 0, false},
-        {"faint_fluid", 1e-12, 1e-12, 1e-13, 0, false},  {"solid", 1e-3, 1e-2, 1e-5, 1e-2, true},
-        {"slow_solid", 1e-5, 1e-4, 1e-7, 1e-4, true},    {"fast_solid", 1e-2, 5e-2, 1e-3, 5e-2, true},
-        {"resting_bed", 1e-3, 1e-2, 1e-5, 0, true},      {"far_outside", 0.5, 0.3, 1e-2, 0.3, true},
+        {"slow_fluid", 1e-5, 1e-4, 1e-7, 0, false, 0},      {"fluid", 1e-3, 1e-2, 1e-5, 0, false, 0},
+        {"fast_fluid", 1e-2, 5e-2, 1e-3, 0, false, 0},      {"noise", 0, 0, 1e-3, 0, false, 0},
+        {"faint_fluid", 1e-12, 1e-12, 1e-13, 0, false, 0},  {"solid", 1e-3, 1e-2, 1e-5, 1e-2, true, 0},
+        {"slow_solid", 1e-5, 1e-4, 1e-7, 1e-4, true, 0},    {"fast_solid", 1e-2, 5e-2, 1e-3, 5e-2, true, 0},
+        {"resting_bed", 1e-3, 1e-2, 1e-5, 0, true, 0},      {"far_outside", 0.5, 0.3, 1e-2, 0.3, true, 0},
+        {"driven_fluid", 1e-3, 1e-2, 1e-5, 0, false, 1e-6}, {"driven_solid", 1e-3, 1e-2, 1e-5, 1e-2, true, 1e-6},
+        {"pushed_fluid", 1e-3, 1e-2, 1e-5, 0, false, 1e-2}, {"pushed_solid", 1e-3, 1e-2, 1e-5, 1e-2, true, 1e-2},
     };
     for (const Kind& k : kinds) {
         Err fx, db, ffx, fdb;
@@ -123,25 +181,40 @@ int main(int argc, char** argv) {
             const int n = k.solid ? 1 + (int)(U(rng) * 125) : 0;
             const double ooo = 1 / omega - 0.5, sf = n / 125.;
             const double B = n == 0 ? 0.0 : n >= 125 ? 1.0 : sf * ooo / ((1 - sf) + ooo);
+            const double g[3] = {k.g * N(rng), k.g * N(rng), k.g * N(rng)};
             double a[19], b[19], Fa[3] = {0, 0, 0}, Fb[3];
             quad q[19], Fq[3], upq[3] = {up[0], up[1], up[2]};
             for (int i = 0; i < 19; ++i) { a[i] = b[i] = f[i]; q[i] = f[i]; }
             double scale = 0;
             for (int i = 0; i < 19; ++i) scale = std::fmax(scale, std::fabs(f[i]));
+            for (double v : g) scale = std::fmax(scale, std::fabs(v) / 8);
             if (n) scale = std::fmax(scale, std::fmax(std::fabs(up[0]), std::fmax(std::fabs(up[1]), std::fabs(up[2]))) / 8);
-            collide<quad>(q, omega, B, upq, Fq);
-            collide<double>(b, omega, B, up, Fb);
+            const bool force = k.g != 0;
+            const quad gq[3] = {g[0], g[1], g[2]};
+            if (force) {
+                collide_force<quad>(q, omega, gq, n, B, upq, Fq);
+                collide_force<double>(b, omega, g, n, B, up, Fb);
+            } else {
+                collide<quad>(q, omega, B, upq, Fq);
+                collide<double>(b, omega, B, up, Fb);
+            }
+            auto fixed = [&](bool solid, double(&v)[19], int e, double(&F)[3]) {
+                const lbdem::fixed::Relax rx = lbdem::fixed::relax_of(omega);
+                const double w = solid && n ? B : 0.0, a0 = n ? up[0] : 0.0, a1 = n ? up[1] : 0.0, a2 = n ? up[2] : 0.0;
+                if (force) lbdem::fixed::collide<true>(solid, v, e, rx, g[0], g[1], g[2], n == 125, w, a0, a1, a2, F);
+                else lbdem::fixed::collide<false>(solid, v, e, rx, 0, 0, 0, n == 125, w, a0, a1, a2, F);
+            };
             int e = lbdem::fixed::cell_exponent(f);
             if (n) e = lbdem::fixed::cell_exponent_up(e, up[0], up[1], up[2]);
+            if (force) e = lbdem::fixed::cell_exponent_up(e, g[0], g[1], g[2]);
             if (!lbdem::fixed::fits(e)) { ++out; continue; }
-            const lbdem::fixed::Relax rx = lbdem::fixed::relax_of(omega);
             if (n) {
-                lbdem::fixed::collide(true, a, e, rx, B, up[0], up[1], up[2], Fa);
+                fixed(true, a, e, Fa);
             } else {
                 double a2[19], z[3];
                 for (int i = 0; i < 19; ++i) a2[i] = a[i];
-                lbdem::fixed::collide(false, a, e, rx, 0, 0, 0, 0, Fa);
-                lbdem::fixed::collide(true, a2, e, rx, 0, 0, 0, 0, z);
+                fixed(false, a, e, Fa);
+                fixed(true, a2, e, z);
                 bool same = z[0] == 0 && z[1] == 0 && z[2] == 0;
                 for (int i = 0; i < 19; ++i) same = same && std::memcmp(&a[i], &a2[i], 8) == 0;
                 bits += same ? 0 : 1;
@@ -162,7 +235,7 @@ int main(int argc, char** argv) {
     double z[19] = {}, F[3];
     const int e = lbdem::fixed::cell_exponent(z);
     bool zero = lbdem::fixed::fits(e);
-    lbdem::fixed::collide(false, z, e, lbdem::fixed::relax_of(1.7), 0, 0, 0, 0, F);
+    lbdem::fixed::collide<false>(false, z, e, lbdem::fixed::relax_of(1.7), 0, 0, 0, false, 0, 0, 0, 0, F);
     for (double v : z) zero = zero && v == 0.0;
     std::printf("zero %d\n", zero ? 1 : 0);
     // values outside the range are refused

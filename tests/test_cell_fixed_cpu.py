@@ -28,12 +28,13 @@ def test_error_no_larger_than_double(program, seed):
     out = subprocess.run([str(program), "4000", str(seed)], check=True, capture_output=True, text=True).stdout
     lines = [ln.split() for ln in out.splitlines()]
     kinds = [ln for ln in lines if len(ln) == 11]
-    assert len(kinds) == 10
+    assert len(kinds) == 14
     for name, fx, fr, dx, dr, ffx, ffr, fdx, fdr, bits, left_out in kinds:
         if int(left_out) < 3900:
             assert float(fx) <= float(dx) and float(fr) <= float(dr), name
             assert float(ffx) <= float(fdx) and float(ffr) <= float(fdr), name
         assert int(bits) == 0, name
-        if name in ("fluid", "solid", "slow_fluid", "slow_solid", "noise", "faint_fluid", "resting_bed"):
+        if name in ("fluid", "solid", "slow_fluid", "slow_solid", "noise", "faint_fluid", "resting_bed",
+                    "driven_fluid", "driven_solid", "pushed_fluid", "pushed_solid"):
             assert int(left_out) == 0, name
     assert ["zero", "1"] in lines and ["refused", "5"] in lines
