@@ -193,6 +193,20 @@ __global__ void k_prepare_bin(const double* __restrict__ rec, int n, SphereDev* 
     }
 }
 
+// The tables without the bins, one thread per sphere.
+__global__ void k_prepare(const double* __restrict__ rec, int n, SphereDev* __restrict__ sph,
+                          SphereFast* __restrict__ fast, float* __restrict__ xpf, int* __restrict__ tag2slot,
+                          unsigned* __restrict__ err, Geom g, int max_tag, double max_radius,
+                          double* __restrict__ ft_zero, double* __restrict__ rec_copy) {
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= n) return;
+    for (int k = 0; k < 6; ++k) ft_zero[(size_t)k * n + i] = 0.0;
+    const double* p = rec + (size_t)i * REC_STRIDE;
+    for (int k = 0; k < REC_STRIDE; ++k) rec_copy[(size_t)i * REC_STRIDE + k] = p[k];
+    int box[6];
+    prepare_sphere(p, i, i, g, max_tag, max_radius, sph, fast, xpf, tag2slot, err, box);
+}
+
 // Location of population i of cell c in the AA layout (phase = completed steps mod 2).
 template <typename T>
 __device__ __forceinline__ T* pop_slot(T* f, int i, int x, int y, int z, int phase, const Geom& g) {
@@ -813,6 +827,15 @@ cudaError_t launch_prepare_bin(const double* rec, int n, SphereDev* sph, SphereF
     k_prepare_bin<false><<<(n + 7) / 8, 256, 0, s>>>(rec, n, sph, fast, xpf, tag2slot, err, g, max_tag, max_radius,
                                                      nullptr, nullptr, 0, nullptr, ft_zero, rec_copy, tile_cnt, bins,
                                                      work, work_n);
+    return cudaGetLastError();
+}
+
+cudaError_t launch_prepare(const double* rec, int n, SphereDev* sph, SphereFast* fast, float* xpf, int* tag2slot,
+                           unsigned* err, Geom g, int max_tag, double max_radius, double* ft_zero, double* rec_copy,
+                           cudaStream_t s) {
+    if (n <= 0) return cudaSuccess;
+    k_prepare<<<(n + 63) / 64, 64, 0, s>>>(rec, n, sph, fast, xpf, tag2slot, err, g, max_tag, max_radius, ft_zero,
+                                           rec_copy);
     return cudaGetLastError();
 }
 

@@ -99,6 +99,8 @@ struct lbdem_handle {
     size_t dev_bytes = 0;
 
     float adj_fwd_ms = 0.f, adj_bwd_ms = 0.f;
+    void* adj_ws = nullptr;     // adjoint window memory kept for the next window
+    size_t adj_bytes = 0;
 
     int n_cur = 0;
     int64_t step = 0;
@@ -152,7 +154,7 @@ cudaError_t dalloc(lbdem_handle* h, P** p, size_t bytes) {
 void release(lbdem_handle* h) {
     void* dev[] = {h->f, h->vox, h->up, h->cf, h->btab, h->btabf, h->d_rec, h->d_sph, h->d_fast, h->d_xpf, h->d_tag2slot,
                    h->d_tile_cnt, h->d_bins, h->d_work, h->d_work_n, h->d_ft, h->d_err, h->d_mass, h->scratch, h->d_jobs, h->d_pavg,
-                   h->d_ppart, h->d_pcount};
+                   h->d_ppart, h->d_pcount, h->adj_ws};
     for (void* p : dev)
         if (p) cudaFree(p);
     void* host[] = {h->h_rec, h->h_ft, h->h_err, h->h_pavg};
@@ -170,7 +172,17 @@ lbdem_status ensure_scratch(lbdem_handle* h, size_t bytes) {
         h->scratch = nullptr;
         h->scratch_bytes = 0;
     }
-    CK(h, dalloc(h, &h->scratch, bytes));
+    cudaError_t e = dalloc(h, &h->scratch, bytes);
+    if (e == cudaErrorMemoryAllocation && h->adj_ws) {   // give the kept adjoint memory back first
+        cudaGetLastError();
+        cudaStreamSynchronize(h->stream);
+        cudaFree(h->adj_ws);
+        h->dev_bytes -= h->adj_bytes;
+        h->adj_ws = nullptr;
+        h->adj_bytes = 0;
+        e = dalloc(h, &h->scratch, bytes);
+    }
+    CK(h, e);
     h->scratch_bytes = bytes;
     return LBDEM_OK;
 }
@@ -217,6 +229,17 @@ lbdem_status voxelize(lbdem_handle* h, int n, int init_vel, const double* src) {
         if (init_vel) h->pavg_valid = false;
     }
     h->n_cur = n;
+    return LBDEM_OK;
+}
+
+// The tables of n records with the positions, radii and tags of the current list (the
+// voxel words stay), and the force sums zeroed.
+lbdem_status renew_tables(lbdem_handle* h, int n, const double* src) {
+    if (n <= 0) return LBDEM_OK;
+    CK(h, launch_prepare(src, n, h->d_sph, h->d_fast, h->d_xpf, h->d_tag2slot, h->d_err, h->g, h->cfg.max_tag,
+                         h->cfg.max_radius, h->d_ft, h->d_rec, h->stream));
+    h->ft_dirty = false;
+    h->launches += 1;
     return LBDEM_OK;
 }
 
@@ -851,22 +874,43 @@ lbdem_status lbdem_init_profile(lbdem_handle* h, int32_t kind, double rho_hi, do
 
 namespace {
 
-// Device buffers of one adjoint window, released on every exit path.
+// One adjoint window's device memory, in one block that the handle keeps for the next
+// window up to ADJ_KEEP_BYTES (allocating and releasing 2.2 GB took 2 ms of a 10 ms
+// window at 128^3); a larger one is released when the window ends.
+constexpr size_t ADJ_KEEP_BYTES = (size_t)4 << 30;
 struct AdjointBuffers {
-    std::vector<void*> ptrs;
+    lbdem_handle* h;
+    size_t used = 0;
+    explicit AdjointBuffers(lbdem_handle* handle) : h(handle) {}
     ~AdjointBuffers() {
-        for (void* p : ptrs)
-            if (p) cudaFree(p);
+        if (h->adj_bytes > ADJ_KEEP_BYTES) drop();
+    }
+    void drop() {
+        if (h->adj_ws) {
+            cudaStreamSynchronize(h->stream);
+            cudaFree(h->adj_ws);
+            h->dev_bytes -= h->adj_bytes;
+        }
+        h->adj_ws = nullptr;
+        h->adj_bytes = 0;
+    }
+    static size_t rounded(size_t bytes) { return (bytes + 255) / 256 * 256; }
+    cudaError_t reserve(size_t bytes) {
+        if (h->adj_bytes >= bytes) return cudaSuccess;
+        drop();
+        const cudaError_t e = cudaMalloc(&h->adj_ws, bytes);
+        if (e != cudaSuccess) {
+            h->adj_ws = nullptr;
+            return e;
+        }
+        h->adj_bytes = bytes;
+        h->dev_bytes += bytes;
+        return cudaSuccess;
     }
     template <typename P>
-    cudaError_t get(P** p, size_t bytes) {
-        void* q = nullptr;
-        cudaError_t e = cudaMalloc(&q, bytes == 0 ? 16 : bytes);
-        if (e == cudaSuccess) {
-            ptrs.push_back(q);
-            *p = (P*)q;
-        }
-        return e;
+    void get(P** p, size_t bytes) {
+        *p = (P*)((char*)h->adj_ws + used);
+        used += rounded(bytes);
     }
 };
 
@@ -931,18 +975,24 @@ lbdem_status lbdem_adjoint_window(lbdem_handle* h, int32_t nsteps, int32_t K, in
     const size_t pop = (size_t)Q * N * h->esz;
     const int nseg = (nsteps + K - 1) / K;
     const size_t nrec = (size_t)nsteps * n;
-    AdjointBuffers buf;
+    AdjointBuffers buf(h);
     double *d_recs = nullptr, *d_w = nullptr, *d_gv = nullptr, *d_glob = nullptr, *d_loss = nullptr, *d_ft = nullptr;
     unsigned char *ckpt = nullptr, *tape = nullptr, *lam = nullptr;
-    CK(h, buf.get(&d_recs, nrec * REC_STRIDE * sizeof(double)));
-    CK(h, buf.get(&d_w, nrec * 6 * sizeof(double)));
-    CK(h, buf.get(&d_gv, nrec * 6 * sizeof(double)));
-    CK(h, buf.get(&d_glob, 4 * sizeof(double)));
-    CK(h, buf.get(&d_loss, sizeof(double)));
-    CK(h, buf.get(&d_ft, 6 * (size_t)std::max(n, 1) * sizeof(double)));
-    CK(h, buf.get(&ckpt, (size_t)nseg * pop));
-    CK(h, buf.get(&tape, (size_t)K * pop + ALLOC_TAIL));
-    CK(h, buf.get(&lam, 2 * pop));
+    const size_t sizes[9] = {nrec * REC_STRIDE * sizeof(double), nrec * 6 * sizeof(double), nrec * 6 * sizeof(double),
+                             4 * sizeof(double), sizeof(double), 6 * (size_t)std::max(n, 1) * sizeof(double),
+                             (size_t)nseg * pop, (size_t)K * pop + ALLOC_TAIL, 2 * pop};
+    size_t total = 0;
+    for (size_t b : sizes) total += AdjointBuffers::rounded(b);
+    CK(h, buf.reserve(total));
+    buf.get(&d_recs, sizes[0]);
+    buf.get(&d_w, sizes[1]);
+    buf.get(&d_gv, sizes[2]);
+    buf.get(&d_glob, sizes[3]);
+    buf.get(&d_loss, sizes[4]);
+    buf.get(&d_ft, sizes[5]);
+    buf.get(&ckpt, sizes[6]);
+    buf.get(&tape, sizes[7]);
+    buf.get(&lam, sizes[8]);
     EventPair ev;
     for (auto& e : ev.e) CK(h, cudaEventCreate(&e));
     if (n > 0) {
@@ -968,7 +1018,11 @@ lbdem_status lbdem_adjoint_window(lbdem_handle* h, int32_t nsteps, int32_t K, in
     };
     auto voxelize_for = [&](int t) -> lbdem_status {
         if (same_table(vox_t, t)) return LBDEM_OK;
-        const lbdem_status r = lbdem_set_particles_device(h, n, d_recs + (size_t)t * n * REC_STRIDE, 0);
+        const double* src = d_recs + (size_t)t * n * REC_STRIDE;
+        // the FP32 form keeps no surface-velocity field, so a step whose positions are those
+        // of the voxelized list only needs its tables (velocities) renewed
+        const lbdem_status r = vox_t >= 0 && h->prec == LBDEM_PREC_FP32_DEV ? renew_tables(h, n, src)
+                                                                            : lbdem_set_particles_device(h, n, src, 0);
         if (r == LBDEM_OK) vox_t = t;
         return r;
     };

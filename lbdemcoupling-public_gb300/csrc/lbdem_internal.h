@@ -313,6 +313,10 @@ cudaError_t launch_prepare_bin(const double* rec, int n, SphereDev* sph, SphereF
                                int* tag2slot, unsigned* err, Geom g, int max_tag, double max_radius,
                                double* ft_zero, double* rec_copy, int* tile_cnt, int* bins, int* work, int* work_n,
                                cudaStream_t s);
+// The tables and the tag map alone (no tile bins), for a list whose voxel words stand.
+cudaError_t launch_prepare(const double* rec, int n, SphereDev* sph, SphereFast* fast, float* xpf, int* tag2slot,
+                           unsigned* err, Geom g, int max_tag, double max_radius, double* ft_zero, double* rec_copy,
+                           cudaStream_t s);
 // The float table and tag map of the list being voxelized (the prepare launch
 // fills both); used by defineVelocity in the float form, which keeps no
 // surface-velocity field (up == nullptr).
