@@ -67,144 +67,176 @@ __device__ __noinline__ int region_exact(int X, int Y, int Z, const SphereDev& s
 
 __device__ __forceinline__ int tiles_along(int n) { return (n + TILE - 1) / TILE; }
 
+// Where the prepare launches put a sphere list, and what they clear beside it.
+struct SphereTables {
+    SphereDev* sph;
+    SphereFast* fast;
+    float* xpf;
+    int* tag2slot;
+    unsigned* err;
+    double* ft_zero;      // (may be null) 6 n force/torque sums of the coming step, zeroed
+    double* rec_copy;     // (may be null, never overlapping the source) a copy of the records
+};
+
 // Per sphere: bounding box (double -> integer truncation toward zero,
 // src/ibProcessors3D.h:43-45) intersected with the lattice
 // (src/ibDataExchangeWrappers3D.hh:127-133), thresholds, the float split of
 // the centre, and the tag -> lowest list index map (LAMMPS atom->map keeps the
-// owned atom, which precedes its ghost images).  Returns the cell box that the
-// sphere's tiles are binned by (lo > hi: the sphere reaches no cell).
-__device__ __forceinline__ void prepare_sphere(const double* __restrict__ p, int i, int il, const Geom& g,
-                                               int max_tag, double max_radius, SphereDev* __restrict__ sph,
-                                               SphereFast* __restrict__ fast, float* __restrict__ xpf,
-                                               int* __restrict__ tag2slot, unsigned* __restrict__ err, int box[6]) {
-    SphereDev s;
-    SphereFast q;
-    for (int d = 0; d < 3; ++d) { s.x[d] = p[d]; s.v[d] = p[3 + d]; s.w[d] = p[6 + d]; }
-    s.r = p[9];
-    const double tagd = p[10];
-    s.valid = 1;
-    if (!(tagd >= 1.0 && tagd <= (double)max_tag)) {
-        atomicOr(err, 0x4u);  // LBDEM_DEVERR_TAG_RANGE
-        s.valid = 0;
-        s.tag = 0;
-    } else {
-        s.tag = (int)tagd;
+// owned atom, which precedes its ghost images).
+// L lanes (8 or 32) share a sphere: they read its record as one piece, and lanes 0-2
+// take one axis each (GB300's two double lanes per clock make an instruction cost the
+// same for one lane as for 32, so a warp's spheres and axes go through it together).
+// Returns, in lane d < 3 of the sphere, the cell range along axis d that its tiles are
+// binned by, lo > hi in all of them when the sphere reaches no cell.  `on`: the lanes
+// that hold a sphere.  Must be reached by all 32 lanes.
+template <int L>
+__device__ __forceinline__ void prepare_sphere(const double* __restrict__ p, bool on, int i, int il, int n,
+                                               const Geom& g, int max_tag, double max_radius, const SphereTables& t,
+                                               int& blo, int& bhi) {
+    const int lane = threadIdx.x & 31, sub = lane % L, base = lane - sub;
+    double ra = 0.0, rb = 0.0;   // record words sub and (L < 12) L + sub
+    if (on && sub < REC_STRIDE) ra = p[sub];
+    if (L < REC_STRIDE && on && sub < REC_STRIDE - L) rb = p[L + sub];
+    if (on && t.rec_copy) {
+        double* c = t.rec_copy + (size_t)i * REC_STRIDE;
+        if (sub < REC_STRIDE) c[sub] = ra;
+        if (L < REC_STRIDE && sub < REC_STRIDE - L) c[L + sub] = rb;
     }
-    if (!(s.r > 0.0 && s.r <= max_radius)) {
-        atomicOr(err, 0x10u);  // LBDEM_DEVERR_RADIUS
-        s.valid = 0;
+    if (on && t.ft_zero && sub < 6) t.ft_zero[(size_t)sub * n + i] = 0.0;
+    auto word = [&](int k) -> double {
+        const double a = __shfl_sync(FULL_MASK, ra, base + (k % L));
+        if (L >= REC_STRIDE) return a;
+        const double b = __shfl_sync(FULL_MASK, rb, base + (k % L));
+        return k < L ? a : b;
+    };
+    const int d = min(sub, 2);
+    const double x = word(d), v = word(3 + d), w = word(6 + d), r = word(9), tagd = word(10);
+    const int dim = d == 0 ? g.nx : (d == 1 ? g.ny : g.nz);
+    const bool tag_ok = tagd >= 1.0 && tagd <= (double)max_tag;
+    const bool r_ok = r > 0.0 && r <= max_radius;
+    // |x| < 2^24 keeps the integer conversions defined and the float split
+    // accurate; a sphere farther out cannot reach the lattice.
+    const bool x_ok = x > -16777216.0 && x < 16777216.0;
+    float xh = 0.f, xl = 0.f;
+    int lo = 1, hi = 0;
+    if (x_ok) {
+        xh = (float)x;
+        xl = (float)(x - (double)xh);
+        long long l = (long long)(__dsub_rn(__dsub_rn(x, r), 2.0));
+        long long h = (long long)(__dadd_rn(__dadd_rn(x, r), 2.0));
+        if (l < 0) l = 0;
+        if (h > dim - 1) h = dim - 1;
+        lo = (int)(l < (long long)dim ? l : dim);
+        hi = (int)(h > -1 ? h : -1);
     }
-    const int dims[3] = {g.nx, g.ny, g.nz};
-    for (int d = 0; d < 3; ++d) {
-        const double xd = s.x[d];
-        q.xh[d] = 0.f; q.xl[d] = 0.f;
-        // |x| < 2^24 keeps the integer conversions defined and the float split
-        // accurate; a sphere farther out cannot reach the lattice.
-        if (!(xd > -16777216.0 && xd < 16777216.0)) { s.valid = 0; s.lo[d] = 1; s.hi[d] = 0; continue; }
-        q.xh[d] = (float)xd;
-        q.xl[d] = (float)(xd - (double)q.xh[d]);
-        long long lo = (long long)(__dsub_rn(__dsub_rn(xd, s.r), 2.0));
-        long long hi = (long long)(__dadd_rn(__dadd_rn(xd, s.r), 2.0));
-        if (lo < 0) lo = 0;
-        if (hi > dims[d] - 1) hi = dims[d] - 1;
-        s.lo[d] = (int)(lo < (long long)dims[d] ? lo : dims[d]);
-        s.hi[d] = (int)(hi > -1 ? hi : -1);
-        if (s.lo[d] > s.hi[d]) s.valid = 0;
+    const unsigned good = __ballot_sync(FULL_MASK, x_ok && lo <= hi);
+    const bool valid = tag_ok && r_ok && ((good >> base) & 7u) == 7u;
+    blo = on && valid ? lo : 1;
+    bhi = on && valid ? hi : 0;
+    if (!on) return;
+    const int tag = tag_ok ? (int)tagd : 0;
+    SphereDev& s = t.sph[i];
+    SphereFast& q = t.fast[i];
+    float* xp = t.xpf + (size_t)i * XPF_STRIDE;
+    const float vf = (float)v, wf = (float)w;
+    if (sub < 3) {
+        s.x[sub] = x; s.v[sub] = v; s.w[sub] = w;
+        s.lo[sub] = lo; s.hi[sub] = hi;
+        q.xh[sub] = xh; q.xl[sub] = xl;
+        q.lo[sub] = blo; q.hi[sub] = bhi;
+        q.v[sub] = vf; q.w[sub] = wf;
+        xp[sub] = xh; xp[3 + sub] = xl; xp[6 + sub] = vf; xp[9 + sub] = wf; xp[12 + sub] = 0.f;
     }
-    const double rp = __dadd_rn(s.r, SQRT3HALF), rm = __dsub_rn(s.r, SQRT3HALF);
-    s.rp2 = __dmul_rn(rp, rp);
-    s.rm2 = __dmul_rn(rm, rm);
-    s.rsq = __dmul_rn(s.r, s.r);
-    q.rp2 = (float)s.rp2;
-    q.rm2 = (float)s.rm2;
-    q.rsq = (float)s.rsq;
-    const float r4 = (float)s.r + 4.0f;
-    q.margin = ldexpf(r4 * r4, -19);
-    for (int d = 0; d < 3; ++d) {
-        q.lo[d] = s.valid ? s.lo[d] : 1;
-        q.hi[d] = s.valid ? s.hi[d] : 0;
-        q.v[d] = (float)s.v[d];
-        q.w[d] = (float)s.w[d];
-        box[2 * d] = q.lo[d];
-        box[2 * d + 1] = q.hi[d];
+    const double rp = __dadd_rn(r, SQRT3HALF), rm = __dsub_rn(r, SQRT3HALF);
+    const double rp2 = __dmul_rn(rp, rp), rm2 = __dmul_rn(rm, rm), rsq = __dmul_rn(r, r);
+    const float r4 = (float)r + 4.0f;
+    if (sub == 3) {
+        s.r = r; s.rp2 = rp2; s.rm2 = rm2; s.rsq = rsq;
+        s.tag = tag; s.valid = valid ? 1 : 0;
+        q.rp2 = (float)rp2; q.rm2 = (float)rm2; q.rsq = (float)rsq;
+        q.margin = ldexpf(r4 * r4, -19);
+        q.tag = tag; q.pad = 0;
+        xp[15] = 0.f;
+        if (!tag_ok) atomicOr(t.err, 0x4u);  // LBDEM_DEVERR_TAG_RANGE
+        if (!r_ok) atomicOr(t.err, 0x10u);   // LBDEM_DEVERR_RADIUS
+        if (tag >= 1) atomicMin(t.tag2slot + tag, il);
     }
-    q.tag = s.tag;
-    q.pad = 0;
-    sph[i] = s;
-    fast[i] = q;
-    float4* xp = reinterpret_cast<float4*>(xpf + (size_t)i * XPF_STRIDE);
-    xp[0] = make_float4(q.xh[0], q.xh[1], q.xh[2], q.xl[0]);
-    xp[1] = make_float4(q.xl[1], q.xl[2], q.v[0], q.v[1]);
-    xp[2] = make_float4(q.v[2], q.w[0], q.w[1], q.w[2]);
-    xp[3] = make_float4(0.f, 0.f, 0.f, 0.f);
-    if (s.tag >= 1) atomicMin(tag2slot + s.tag, il);
 }
 
-// One warp per sphere: lane 0 prepares the sphere (prepare_sphere), then the
-// lanes stride over the tiles its box overlaps and append the sphere to each
+// A warp prepares 32 / L spheres, then its lanes stride over the tiles that each
+// sphere's box overlaps and append the sphere to each
 // tile's bin (entries past TILE_BIN are dropped; the voxelization of such a
 // tile re-collects its spheres; a tile's bin is rank-sorted there, so the
 // append order does not matter).  The first sphere of a tile also appends the
 // tile to the work list.
 // BATCH: slot i belongs to the domain d with soff[d] <= i; slots past the
 // domain's particle count are skipped; the map stores domain-local slots.
-// ft_zero (may be null): the 6 n force/torque sums of the coming collide-stream
-// step, zeroed here instead of by a separate memset launch.  rec_copy (may be
-// null, never overlapping rec): receives a copy of the n records.
-template <bool BATCH>
-__global__ void k_prepare_bin(const double* __restrict__ rec, int n, SphereDev* __restrict__ sph,
-                              SphereFast* __restrict__ fast, float* __restrict__ xpf, int* __restrict__ tag2slot,
-                              unsigned* __restrict__ err, Geom g, int max_tag, double max_radius,
-                              const DomView* __restrict__ doms, const int* __restrict__ soff, int ndom,
-                              const int* __restrict__ ncur, double* __restrict__ ft_zero,
-                              double* __restrict__ rec_copy, int* __restrict__ tile_cnt, int* __restrict__ bins,
-                              int* __restrict__ work, int* __restrict__ work_n) {
-    const int i = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
+// old: a list whose entries in its own tag map are cleared by the way (map null: none).
+// L = 32, one sphere per warp, is the shorter chain for short lists; L = 8 shares the
+// double instructions of four spheres (PREPARE_WIDE).
+struct OldList {
+    int* map;
+    const double* rec;
+    int n, max_tag;
+};
+template <bool BATCH, int L>
+__global__ void k_prepare_bin(const double* __restrict__ rec, int n, SphereTables t, Geom g, int max_tag,
+                              double max_radius, const DomView* __restrict__ doms, const int* __restrict__ soff,
+                              int ndom, const int* __restrict__ ncur, int* __restrict__ tile_cnt,
+                              int* __restrict__ bins, int* __restrict__ work, int* __restrict__ work_n, OldList old) {
     const int lane = threadIdx.x & 31;
-    if (i >= n) return;   // warp-uniform from here on
-    if (ft_zero && lane < 6) ft_zero[(size_t)lane * n + i] = 0.0;
+    const int i = (blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5)) * (32 / L) + lane / L;
+    if (old.map)
+        for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < old.n; k += gridDim.x * blockDim.x) {
+            const double tagd = old.rec[(size_t)k * REC_STRIDE + 10];
+            if (tagd >= 1.0 && tagd <= (double)old.max_tag) old.map[(int)tagd] = NO_SLOT;
+        }
+    bool on = i < n;
     int il = i, t0 = 0;
     if (BATCH) {
-        const int d = find_domain(soff, ndom, i);
-        il = i - __ldg(soff + d);
-        if (il >= __ldg(ncur + d)) return;
-        g = doms[d].g;
-        tag2slot += doms[d].tag0;
-        t0 = doms[d].t0;
+        if (on) {
+            const int d = find_domain(soff, ndom, i);
+            il = i - __ldg(soff + d);
+            const DomView& D = doms[d];
+            g = D.g;
+            t.tag2slot += D.tag0;
+            t0 = D.t0;
+            if (t.ft_zero && lane % L < 6) t.ft_zero[(size_t)(lane % L) * n + i] = 0.0;   // unused slots too
+            on = il < __ldg(ncur + d);
+        }
     }
-    const double* p = rec + (size_t)i * REC_STRIDE;
-    if (rec_copy && lane < REC_STRIDE) rec_copy[(size_t)i * REC_STRIDE + lane] = p[lane];
-    int box[6] = {1, 0, 1, 0, 1, 0};
-    if (lane == 0) prepare_sphere(p, i, il, g, max_tag, max_radius, sph, fast, xpf, tag2slot, err, box);
+    int blo, bhi;
+    prepare_sphere<L>(rec + (size_t)(on ? i : 0) * REC_STRIDE, on, i, il, n, g, max_tag, max_radius, t, blo, bhi);
+    const int my_tny = tiles_along(g.ny), my_tnz = tiles_along(g.nz);
 #pragma unroll
-    for (int k = 0; k < 6; ++k) box[k] = __shfl_sync(0xffffffffu, box[k], 0);
-    if (box[0] > box[1] || box[2] > box[3] || box[4] > box[5]) return;
-    const int tx0 = box[0] / TILE, ty0 = box[2] / TILE, tz0 = box[4] / TILE;
-    const int ex = box[1] / TILE - tx0 + 1, ey = box[3] / TILE - ty0 + 1, ez = box[5] / TILE - tz0 + 1;
-    const int tny = tiles_along(g.ny), tnz = tiles_along(g.nz);
-    const int total = ex * ey * ez;
-    for (int k = lane; k < total; k += 32) {
-        const int kz = k % ez, kr = k / ez;
-        const int ky = kr % ey, kx = kr / ey;
-        const size_t t = (size_t)t0 + ((size_t)(tx0 + kx) * tny + (ty0 + ky)) * tnz + (tz0 + kz);
-        const int pos = atomicAdd(tile_cnt + t, 1);
-        if (pos == 0) work[atomicAdd(work_n, 1)] = (int)t;
-        if (pos < TILE_BIN) bins[t * TILE_BIN + pos] = il;
+    for (int q = 0; q < 32; q += L) {
+        const int x0 = __shfl_sync(FULL_MASK, blo, q), x1 = __shfl_sync(FULL_MASK, bhi, q);
+        const int y0 = __shfl_sync(FULL_MASK, blo, q + 1), y1 = __shfl_sync(FULL_MASK, bhi, q + 1);
+        const int z0 = __shfl_sync(FULL_MASK, blo, q + 2), z1 = __shfl_sync(FULL_MASK, bhi, q + 2);
+        const int ql = __shfl_sync(FULL_MASK, il, q), qt0 = __shfl_sync(FULL_MASK, t0, q);
+        const int tny = BATCH ? __shfl_sync(FULL_MASK, my_tny, q) : my_tny;
+        const int tnz = BATCH ? __shfl_sync(FULL_MASK, my_tnz, q) : my_tnz;
+        if (x0 > x1) continue;   // warp-uniform: no sphere, or one that reaches no cell
+        const int tx0 = x0 / TILE, ty0 = y0 / TILE, tz0 = z0 / TILE;
+        const int ex = x1 / TILE - tx0 + 1, ey = y1 / TILE - ty0 + 1, ez = z1 / TILE - tz0 + 1;
+        const int total = ex * ey * ez;
+        for (int k = lane; k < total; k += 32) {
+            const int kz = k % ez, kr = k / ez;
+            const int ky = kr % ey, kx = kr / ey;
+            const size_t tile = (size_t)qt0 + ((size_t)(tx0 + kx) * tny + (ty0 + ky)) * tnz + (tz0 + kz);
+            const int pos = atomicAdd(tile_cnt + tile, 1);
+            if (pos == 0) work[atomicAdd(work_n, 1)] = (int)tile;
+            if (pos < TILE_BIN) bins[tile * TILE_BIN + pos] = ql;
+        }
     }
 }
 
-// The tables without the bins, one thread per sphere.
-__global__ void k_prepare(const double* __restrict__ rec, int n, SphereDev* __restrict__ sph,
-                          SphereFast* __restrict__ fast, float* __restrict__ xpf, int* __restrict__ tag2slot,
-                          unsigned* __restrict__ err, Geom g, int max_tag, double max_radius,
-                          double* __restrict__ ft_zero, double* __restrict__ rec_copy) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    for (int k = 0; k < 6; ++k) ft_zero[(size_t)k * n + i] = 0.0;
-    const double* p = rec + (size_t)i * REC_STRIDE;
-    for (int k = 0; k < REC_STRIDE; ++k) rec_copy[(size_t)i * REC_STRIDE + k] = p[k];
-    int box[6];
-    prepare_sphere(p, i, i, g, max_tag, max_radius, sph, fast, xpf, tag2slot, err, box);
+// The tables without the bins.
+__global__ void k_prepare(const double* __restrict__ rec, int n, SphereTables t, Geom g, int max_tag,
+                          double max_radius) {
+    const int i = (blockIdx.x * blockDim.x + threadIdx.x) / 8;
+    int blo, bhi;
+    prepare_sphere<8>(rec + (size_t)(i < n ? i : 0) * REC_STRIDE, i < n, i, i, n, g, max_tag, max_radius, t, blo, bhi);
 }
 
 // Location of population i of cell c in the AA layout (phase = completed steps mod 2).
@@ -819,23 +851,44 @@ k_voxelize(const SphereDev* __restrict__ sph, const SphereFast* __restrict__ fas
 
 }  // namespace
 
+namespace {
+
+// Spheres per warp: one up to PREPARE_WIDE spheres (the launch is then a chain of
+// latencies), four beyond it.  5, 498, 2902, 9535 spheres: 5.8, 7.3, 12.7, 25.4 us with
+// one, 7.6, 10.2, 13.2, 17.1 us with four (6.6, 8.8, 16.5, 40.7 us with one lane
+// preparing a sphere).
+constexpr int PREPARE_WIDE = 4096;
+template <bool BATCH>
+cudaError_t launch_prepare_any(const double* rec, int n, const SphereTables& t, const Geom& g, int max_tag,
+                               double max_radius, const DomView* doms, const int* soff, int ndom, const int* ncur,
+                               int* tile_cnt, int* bins, int* work, int* work_n, const OldList& old, cudaStream_t s) {
+    if (n <= PREPARE_WIDE)
+        k_prepare_bin<BATCH, 32><<<(n + 3) / 4, 128, 0, s>>>(rec, n, t, g, max_tag, max_radius, doms, soff, ndom, ncur,
+                                                             tile_cnt, bins, work, work_n, old);
+    else
+        k_prepare_bin<BATCH, 8><<<(n + 15) / 16, 128, 0, s>>>(rec, n, t, g, max_tag, max_radius, doms, soff, ndom,
+                                                              ncur, tile_cnt, bins, work, work_n, old);
+    return cudaGetLastError();
+}
+
+}  // namespace
+
 cudaError_t launch_prepare_bin(const double* rec, int n, SphereDev* sph, SphereFast* fast, float* xpf,
                                int* tag2slot, unsigned* err, Geom g, int max_tag, double max_radius,
                                double* ft_zero, double* rec_copy, int* tile_cnt, int* bins, int* work, int* work_n,
-                               cudaStream_t s) {
+                               int* old_map, const double* old_rec, int old_n, cudaStream_t s) {
     if (n <= 0) return cudaSuccess;
-    k_prepare_bin<false><<<(n + 7) / 8, 256, 0, s>>>(rec, n, sph, fast, xpf, tag2slot, err, g, max_tag, max_radius,
-                                                     nullptr, nullptr, 0, nullptr, ft_zero, rec_copy, tile_cnt, bins,
-                                                     work, work_n);
-    return cudaGetLastError();
+    return launch_prepare_any<false>(rec, n, SphereTables{sph, fast, xpf, tag2slot, err, ft_zero, rec_copy}, g, max_tag,
+                                     max_radius, nullptr, nullptr, 0, nullptr, tile_cnt, bins, work, work_n,
+                                     OldList{old_map, old_rec, old_n, max_tag}, s);
 }
 
 cudaError_t launch_prepare(const double* rec, int n, SphereDev* sph, SphereFast* fast, float* xpf, int* tag2slot,
                            unsigned* err, Geom g, int max_tag, double max_radius, double* ft_zero, double* rec_copy,
                            cudaStream_t s) {
     if (n <= 0) return cudaSuccess;
-    k_prepare<<<(n + 63) / 64, 64, 0, s>>>(rec, n, sph, fast, xpf, tag2slot, err, g, max_tag, max_radius, ft_zero,
-                                           rec_copy);
+    k_prepare<<<(n + 7) / 8, 64, 0, s>>>(rec, n, SphereTables{sph, fast, xpf, tag2slot, err, ft_zero, rec_copy}, g,
+                                         max_tag, max_radius);
     return cudaGetLastError();
 }
 
@@ -845,10 +898,9 @@ cudaError_t launch_prepare_bin_batch(const double* rec, int nslots, SphereDev* s
                                      double* ft_zero, int* tile_cnt, int* bins, int* work, int* work_n,
                                      cudaStream_t s) {
     if (nslots <= 0) return cudaSuccess;
-    k_prepare_bin<true><<<(nslots + 7) / 8, 256, 0, s>>>(rec, nslots, sph, fast, xpf, tag2slot, err, Geom{}, max_tag,
-                                                         max_radius, doms, soff, ndom, ncur, ft_zero, nullptr,
-                                                         tile_cnt, bins, work, work_n);
-    return cudaGetLastError();
+    return launch_prepare_any<true>(rec, nslots, SphereTables{sph, fast, xpf, tag2slot, err, ft_zero, nullptr}, Geom{},
+                                    max_tag, max_radius, doms, soff, ndom, ncur, tile_cnt, bins, work, work_n,
+                                    OldList{nullptr, nullptr, 0, 0}, s);
 }
 
 namespace {

@@ -43,6 +43,8 @@ cudaError_t halloc(P** p, size_t bytes) {
 }
 }  // namespace
 
+constexpr size_t FT_PAD = 2;   // doubles before the force sums in their allocation (the error word)
+
 struct lbdem_handle {
     lbdem_config cfg{};
     Geom g{};
@@ -61,18 +63,25 @@ struct lbdem_handle {
     float* btabf = nullptr;     // [126] B(n) rounded to float
 
     int cap = 0;
-    double* d_rec = nullptr;    // [cap][12]
+    // particle records [cap][12] and tag map [max_tag + 1], two of each: a new list goes
+    // into the other pair, and its prepare launch clears the entries of the list before it
+    // in that list's map, so no memset of the whole map stands before a voxelization.
+    // The map not in use is clear.
+    double* rec2[2] = {nullptr, nullptr};
+    int* map2[2] = {nullptr, nullptr};
+    int cur = 0;
+    double* d_rec = nullptr;    // rec2[cur]
     SphereDev* d_sph = nullptr; // [cap]
     SphereFast* d_fast = nullptr; // [cap]
     float* d_xpf = nullptr;     // [cap][XPF_STRIDE]
-    int* d_tag2slot = nullptr;  // [max_tag + 1]
+    int* d_tag2slot = nullptr;  // map2[cur]
     int ntiles = 0;
     int* d_tile_cnt = nullptr;  // [ntiles] spheres binned per tile (zero between calls)
     int* d_bins = nullptr;      // [ntiles][TILE_BIN]
     int* d_work = nullptr;      // [ntiles] tiles with spheres (voxelization work list)
     int* d_work_n = nullptr;    // [4] work-list counters (zero between calls)
-    double* d_ft = nullptr;     // [6][cap]
-    unsigned* d_err = nullptr;
+    double* d_ft = nullptr;     // [6][cap], FT_PAD doubles into an allocation that starts with
+    unsigned* d_err = nullptr;  // the error word, so that one copy brings both back
     double* d_mass = nullptr;
 
     double* h_rec = nullptr;    // pinned staging
@@ -152,12 +161,13 @@ cudaError_t dalloc(lbdem_handle* h, P** p, size_t bytes) {
 }
 
 void release(lbdem_handle* h) {
-    void* dev[] = {h->f, h->vox, h->up, h->cf, h->btab, h->btabf, h->d_rec, h->d_sph, h->d_fast, h->d_xpf, h->d_tag2slot,
-                   h->d_tile_cnt, h->d_bins, h->d_work, h->d_work_n, h->d_ft, h->d_err, h->d_mass, h->scratch, h->d_jobs, h->d_pavg,
+    void* dev[] = {h->f, h->vox, h->up, h->cf, h->btab, h->btabf, h->rec2[0], h->rec2[1], h->d_sph, h->d_fast, h->d_xpf,
+                   h->map2[0], h->map2[1],
+                   h->d_tile_cnt, h->d_bins, h->d_work, h->d_work_n, h->d_err, h->d_mass, h->scratch, h->d_jobs, h->d_pavg,
                    h->d_ppart, h->d_pcount, h->adj_ws};
     for (void* p : dev)
         if (p) cudaFree(p);
-    void* host[] = {h->h_rec, h->h_ft, h->h_err, h->h_pavg};
+    void* host[] = {h->h_rec, h->h_err, h->h_pavg};
     for (void* p : host)
         if (p) cudaFreeHost(p);
     if (h->ev_staged) cudaEventDestroy(h->ev_staged);
@@ -195,8 +205,8 @@ lbdem_status wait_staging(lbdem_handle* h) {
     return LBDEM_OK;
 }
 
-// Voxelization of n records read from src (h->d_rec, or a device table of the
-// caller that the prepare launch copies into h->d_rec as it reads it).
+// Voxelization of n records read from src (the pinned staging table, or a device table of
+// the caller) by the prepare launch, which copies them into the handle's table.
 lbdem_status voxelize(lbdem_handle* h, int n, int init_vel, const double* src) {
     cudaStream_t s = h->stream;
     // defineVelocity reads the velocity a covered cell held before this pass.  The
@@ -210,11 +220,28 @@ lbdem_status voxelize(lbdem_handle* h, int n, int init_vel, const double* src) {
         CK(h, launch_owner_velocity(h->vox, h->d_tag2slot, h->cfg.max_tag, h->n_cur, h->d_xpf, h->g, up_before, s));
         h->launches += 1;
     }
-    CK(h, cudaMemsetAsync(h->d_tag2slot, 0x7F, sizeof(int) * ((size_t)h->cfg.max_tag + 1), s));
+    // A call that is captured into a graph runs again with the same buffers and an unknown
+    // list before it, so it keeps the current pair and clears the whole map; so does an
+    // empty list, which has no prepare launch.
+    cudaStreamCaptureStatus capturing = cudaStreamCaptureStatusNone;
+    CK(h, cudaStreamIsCapturing(s, &capturing));
+    const bool whole = n <= 0 || capturing != cudaStreamCaptureStatusNone;
+    if (whole) CK(h, cudaMemsetAsync(h->d_tag2slot, 0x7F, sizeof(int) * ((size_t)h->cfg.max_tag + 1), s));
     if (n > 0) {
+        int* const old_map = whole ? nullptr : h->d_tag2slot;
+        const double* const old_rec = h->d_rec;
+        if (!whole) {
+            h->cur ^= 1;
+            h->d_tag2slot = h->map2[h->cur];
+            h->d_rec = h->rec2[h->cur];
+        }
         CK(h, launch_prepare_bin(src, n, h->d_sph, h->d_fast, h->d_xpf, h->d_tag2slot, h->d_err, h->g,
                                  h->cfg.max_tag, h->cfg.max_radius, h->d_ft, src == h->d_rec ? nullptr : h->d_rec,
-                                 h->d_tile_cnt, h->d_bins, h->d_work, h->d_work_n, s));
+                                 h->d_tile_cnt, h->d_bins, h->d_work, h->d_work_n, old_map, old_rec, h->n_cur, s));
+        if (src == h->h_rec) {   // the staging table is free again once the launch has read it
+            CK(h, cudaEventRecord(h->ev_staged, s));
+            h->staged_pending = true;
+        }
         h->ft_dirty = false;   // the prepare launch zeroed the 6 n sums
         const int phase = (int)(h->step & 1);
         if (h->prec == LBDEM_PREC_FP64)
@@ -429,23 +456,25 @@ lbdem_status lbdem_create(const lbdem_config* cfg, lbdem_handle** out) {
     TRY(dalloc(h, &h->btab, 126 * sizeof(double)));
     TRY(dalloc(h, &h->btabf, 126 * sizeof(float)));
     const size_t capn = (size_t)(h->cap > 0 ? h->cap : 1);
-    TRY(dalloc(h, &h->d_rec, capn * REC_STRIDE * sizeof(double)));
+    for (auto& r : h->rec2) TRY(dalloc(h, &r, capn * REC_STRIDE * sizeof(double)));
+    h->d_rec = h->rec2[0];
     TRY(dalloc(h, &h->d_sph, capn * sizeof(SphereDev)));
     TRY(dalloc(h, &h->d_fast, capn * sizeof(SphereFast)));
     TRY(dalloc(h, &h->d_xpf, capn * XPF_STRIDE * sizeof(float)));
-    TRY(dalloc(h, &h->d_tag2slot, ((size_t)c.max_tag + 1) * sizeof(int)));
+    for (auto& m : h->map2) TRY(dalloc(h, &m, ((size_t)c.max_tag + 1) * sizeof(int)));
+    h->d_tag2slot = h->map2[0];
     TRY(dalloc(h, &h->d_tile_cnt, (size_t)h->ntiles * sizeof(int)));
     TRY(dalloc(h, &h->d_bins, (size_t)h->ntiles * TILE_BIN * sizeof(int)));
     TRY(cudaMemset(h->d_tile_cnt, 0, (size_t)h->ntiles * sizeof(int)));
     TRY(dalloc(h, &h->d_work, (size_t)h->ntiles * sizeof(int)));
     TRY(dalloc(h, &h->d_work_n, 4 * sizeof(int)));
     TRY(cudaMemset(h->d_work_n, 0, 4 * sizeof(int)));
-    TRY(dalloc(h, &h->d_ft, 6 * capn * sizeof(double)));
-    TRY(dalloc(h, &h->d_err, sizeof(unsigned)));
+    TRY(dalloc(h, &h->d_err, (FT_PAD + 6 * capn) * sizeof(double)));
+    h->d_ft = (double*)h->d_err + FT_PAD;
     TRY(dalloc(h, &h->d_mass, sizeof(double)));
     TRY(halloc(&h->h_rec, capn * REC_STRIDE * sizeof(double)));
-    TRY(halloc(&h->h_ft, 6 * capn * sizeof(double)));
-    TRY(halloc(&h->h_err, sizeof(unsigned)));
+    TRY(halloc(&h->h_err, (FT_PAD + 6 * capn) * sizeof(double)));
+    h->h_ft = (double*)h->h_err + FT_PAD;
     TRY(dalloc(h, &h->d_jobs, 3 * sizeof(PlaneJob)));
     TRY(dalloc(h, &h->d_pavg, 8 * sizeof(double)));
     TRY(dalloc(h, &h->d_ppart, 3 * PLANE_BLOCKS_MAX * sizeof(double)));
@@ -459,9 +488,8 @@ lbdem_status lbdem_create(const lbdem_config* cfg, lbdem_handle** out) {
     TRY(cudaMemset(h->vox, 0, N * sizeof(uint32_t)));
     if (h->up) TRY(cudaMemset(h->up, 0, 3 * N * h->esz));
     if (h->cf) TRY(cudaMemset(h->cf, 0, 3 * N * h->esz));
-    TRY(cudaMemset(h->d_tag2slot, 0x7F, ((size_t)c.max_tag + 1) * sizeof(int)));
-    TRY(cudaMemset(h->d_ft, 0, 6 * capn * sizeof(double)));
-    TRY(cudaMemset(h->d_err, 0, sizeof(unsigned)));
+    for (int* m : h->map2) TRY(cudaMemset(m, 0x7F, ((size_t)c.max_tag + 1) * sizeof(int)));
+    TRY(cudaMemset(h->d_err, 0, (FT_PAD + 6 * capn) * sizeof(double)));
     TRY(cudaDeviceSynchronize());
 #undef TRY
     *out = h;
@@ -550,13 +578,7 @@ lbdem_status lbdem_set_particles(lbdem_handle* h, int32_t n, const double* x, co
         p[10] = (double)tag[i];
         p[11] = 0.0;
     }
-    if (n > 0) {
-        CK(h, cudaMemcpyAsync(h->d_rec, h->h_rec, (size_t)n * REC_STRIDE * sizeof(double), cudaMemcpyHostToDevice,
-                              h->stream));
-        CK(h, cudaEventRecord(h->ev_staged, h->stream));
-        h->staged_pending = true;
-    }
-    return voxelize(h, n, init_vel, h->d_rec);
+    return voxelize(h, n, init_vel, h->h_rec);
 }
 
 lbdem_status lbdem_set_particles_device(lbdem_handle* h, int32_t n, const double* rec, int32_t init_vel) {
@@ -565,10 +587,14 @@ lbdem_status lbdem_set_particles_device(lbdem_handle* h, int32_t n, const double
     if (n > h->cap) return fail(h, LBDEM_ERR_CAPACITY, "set_particles_device: n exceeds max_particles");
     if (n > 0 && !rec) return fail(h, LBDEM_ERR_INVALID_ARG, "set_particles_device: null table");
     DeviceGuard dg(h->device);
-    // a table overlapping the handle's own (other than being it) cannot be read and copied in one pass
-    const uintptr_t a = (uintptr_t)rec, b = (uintptr_t)h->d_rec, len = (uintptr_t)n * REC_STRIDE * sizeof(double);
-    if (n > 0 && a != b && a < b + len && b < a + len)
-        return fail(h, LBDEM_ERR_INVALID_ARG, "set_particles_device: table overlaps the handle's particle table");
+    // a table overlapping the handle's own (other than being the current one) cannot be
+    // read and copied in one pass
+    const uintptr_t a = (uintptr_t)rec, len = (uintptr_t)n * REC_STRIDE * sizeof(double);
+    for (const double* own : h->rec2) {
+        const uintptr_t b = (uintptr_t)own;
+        if (n > 0 && !(a == b && own == h->d_rec) && a < b + len && b < a + len)
+            return fail(h, LBDEM_ERR_INVALID_ARG, "set_particles_device: table overlaps the handle's particle table");
+    }
     return voxelize(h, n, init_vel, rec);
 }
 
@@ -603,9 +629,8 @@ lbdem_status lbdem_get_forces(lbdem_handle* h, int32_t n, double* force, double*
     if (n != h->n_cur) return fail(h, LBDEM_ERR_INVALID_ARG, "get_forces: n differs from the particle list");
     if (n > 0 && (!force || !torque)) return fail(h, LBDEM_ERR_INVALID_ARG, "get_forces: null output");
     DeviceGuard dg(h->device);
-    if (n > 0)
-        CK(h, cudaMemcpyAsync(h->h_ft, h->d_ft, 6 * (size_t)n * sizeof(double), cudaMemcpyDeviceToHost, h->stream));
-    CK(h, cudaMemcpyAsync(h->h_err, h->d_err, sizeof(unsigned), cudaMemcpyDeviceToHost, h->stream));
+    CK(h, cudaMemcpyAsync(h->h_err, h->d_err, (FT_PAD + 6 * (size_t)n) * sizeof(double), cudaMemcpyDeviceToHost,
+                          h->stream));   // the error word and the sums
     CK(h, cudaStreamSynchronize(h->stream));
     h->staged_pending = false;
     if (n > 0) {

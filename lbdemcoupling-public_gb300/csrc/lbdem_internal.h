@@ -20,6 +20,7 @@ constexpr int REC_STRIDE = 12;          // doubles per particle record {x3, v3, 
 constexpr int XPF_STRIDE = 16;          // floats per particle of the float table (xpf, see below)
 constexpr int VOX_NBITS = 7;            // voxel word: sub-cell count n (7 bits) | tag << 7
 constexpr uint32_t VOX_NMASK = (1u << VOX_NBITS) - 1u;
+constexpr int NO_SLOT = 0x7f7f7f7f;     // tag map entry of a tag without a particle (memset with 0x7f)
 constexpr int32_t MAX_TAG_LIMIT = (1 << 25) - 1;
 constexpr int COLLIDE_BLOCK = 128;      // threads per block along z in the collide-stream kernel
 constexpr int COLLIDE_SEGW = 64;        // cells per z-segment of the collide-stream kernel
@@ -309,10 +310,13 @@ cudaError_t launch_collide_batch(const CollideArgs<T>* dargs, const int* seg0, i
 // by launch_voxelize).  ft_zero (may be null): 6 n doubles set to zero by the
 // same launch (the force and torque sums of the next collide-stream step).
 // rec_copy (may be null, never overlapping rec): receives a copy of the n records.
+// rec may be host memory that the device can read (pinned).  old_map (may be null): the
+// tag map of an earlier list of old_n records old_rec, whose entries are set back to "no
+// slot" by the same launch.
 cudaError_t launch_prepare_bin(const double* rec, int n, SphereDev* sph, SphereFast* fast, float* xpf,
                                int* tag2slot, unsigned* err, Geom g, int max_tag, double max_radius,
                                double* ft_zero, double* rec_copy, int* tile_cnt, int* bins, int* work, int* work_n,
-                               cudaStream_t s);
+                               int* old_map, const double* old_rec, int old_n, cudaStream_t s);
 // The tables and the tag map alone (no tile bins), for a list whose voxel words stand.
 cudaError_t launch_prepare(const double* rec, int n, SphereDev* sph, SphereFast* fast, float* xpf, int* tag2slot,
                            unsigned* err, Geom g, int max_tag, double max_radius, double* ft_zero, double* rec_copy,

@@ -96,7 +96,8 @@ extern "C" lbdem_status lbdem_voxelize_static(int32_t nx, int32_t ny, int32_t nz
         return LBDEM_ERR_CUDA;
     if (n == 0) return LBDEM_OK;   // no sphere touches a cell (as in the reference)
     cudaError_t e = launch_prepare_bin(dev_rec, n, sph, fast, xpf, tag2slot, dev_err, g, LBDEM_STATIC_MAX_TAG,
-                                       LBDEM_STATIC_MAX_RADIUS, nullptr, nullptr, tile_cnt, bins, work, work_n, s);
+                                       LBDEM_STATIC_MAX_RADIUS, nullptr, nullptr, tile_cnt, bins, work, work_n, nullptr,
+                                       nullptr, 0, s);
     const OwnerTable ot{xpf, tag2slot, LBDEM_STATIC_MAX_TAG};
     if (e == cudaSuccess) {
         if (precision == LBDEM_PREC_FP64) {
