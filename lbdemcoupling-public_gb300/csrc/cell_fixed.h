@@ -6,7 +6,7 @@
 // an eighth of the memory rate.  Here a cell's doubles are
 // read as 64-bit fixed-point numbers of one common unit, the update is evaluated
 // in those, and every result is rounded once to the nearest double.  A 128^3 suspension
-// (solid fraction 0.26) steps in 0.33 / 0.39 ms (even / odd phase) against 0.93 ms in double.
+// (solid fraction 0.26) steps in 0.32 / 0.36 ms (even / odd phase) against 0.93 ms in double.
 //
 // Unit.  With 2^E above every |f_i| of the cell (E from the largest exponent
 // field emax, E = emax - 1022) the unit is 2^(E - 57) = 2^(emax - 1079): a

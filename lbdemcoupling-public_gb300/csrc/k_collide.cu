@@ -22,9 +22,9 @@
 // shared memory, double-buffered, so the next segment's bytes are in flight while the
 // current one is collided: per-thread 16-byte cp.async with commit groups for
 // the FP32 form, cp.async.bulk on an mbarrier for the FP64 form; rows that are not
-// 16-byte aligned (nz % 4 != 0) are copied in whole 16-byte chunks around the row (FP64),
-// or not staged at all (FP32: k_collide_direct, which also steps FP32 batches).  The staged pre-collision values double as
-// fPre of the PSM update.  The FP32 form collides two cells per thread in packed
+// 16-byte aligned are copied in whole 16-byte chunks around the row (FP64, odd nz), or not
+// staged at all (FP32, nz % 4 != 0: k_collide_direct, which also steps FP32 batches).  The
+// staged pre-collision values double as fPre of the PSM update.  The FP32 form collides two cells per thread in packed
 // f32x2 arithmetic (collide_segment_pairs) and recomputes the particle surface
 // velocity of its solid cells from the owner particle's row of the float table
 // (no per-cell velocity field); the FP64 form one cell per thread, BGK and solid
@@ -858,7 +858,8 @@ struct alignas(16) WarpStage {
     uint32_t vox[2][SEGW + 4];
     T up[2][3][UW];        // particle surface velocity rows of the segment (when staged)
     long long row[2][9];   // element offset of row (x + dx, y + dy) at [3 (dx + 1) + dy + 1]; -1 beyond a wall
-    int geo[2][8];         // x, y, z0, len, domain of the segment held in buffer b
+    T* out[2][sizeof(T) == 8 ? 3 * Q : 1];   // FP64, odd phase: output rows (see issue_segment)
+    int geo[2][8];         // x, y, z0, len, domain, source rows inside, voxel lead of the segment in buffer b
     unsigned long long lead[2];   // unaligned rows: lead elements of row i at bits 2i, voxel row at bits 38,
                                   // surface-velocity row d at bits 40 + 2d
     unsigned long long bar[2];
@@ -914,6 +915,8 @@ __device__ __forceinline__ void bulk_g2s(void* dst, const void* src, uint32_t by
 }
 
 // Directions with c_z != 0 (they need a halo element in the odd phase).
+constexpr uint32_t ZDIRS = 1u << 3 | 1u << 6 | 1u << 7 | 1u << 8 | 1u << 9 | 1u << 12 | 1u << 15 | 1u << 16 | 1u << 17 |
+                           1u << 18;
 __device__ __forceinline__ int zdir(int k) {
     // {3, 6, 7, 8, 9, 12, 15, 16, 17, 18} packed in 5-bit fields
     constexpr unsigned long long D = 3ull | 6ull << 5 | 7ull << 10 | 8ull << 15 | 9ull << 20 | 12ull << 25 |
@@ -952,31 +955,53 @@ __device__ __forceinline__ long long row_off(const Geom& g, const SegGeo& s, int
     return ((long long)X * g.ny + Y) * g.nz;
 }
 
-// Issued by one warp for its segment into buffer b:
+// An 8-byte copy by this thread, counted on an mbarrier whose count has room for one
+// arrival of each lane (cp_arrive).
+__device__ __forceinline__ void cp8(void* dst, const void* src) {
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(smem_addr(dst)), "l"(src) : "memory");
+}
+__device__ __forceinline__ void cp_arrive(unsigned long long* bar) {
+    asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];" ::"r"(smem_addr(bar)) : "memory");
+}
+
+// FP64 form: issued by one warp for its segment into buffer b:
 //   lanes 0..18:  population rows (even: own row, slot i; odd: row x - c_i,
 //                 slot opp i, or own row slot i when that row is beyond a wall);
 //   lanes 19..28: odd phase, aligned rows: the 16-byte chunk holding the halo
-//                 element of the (lane-19)-th c_z != 0 direction (none beyond a z wall);
-//   lane 29:      voxel words of the segment;
+//                 element of the (lane-19)-th c_z != 0 direction;
+//   lane 29:      voxel words of the segment (from the 16-byte boundary below; the lead
+//                 is published);
 //   lanes 29-31:  (second copy) the segment's particle surface-velocity rows.
-// MIS (rows not 16-byte aligned, nz % 4 != 0): each row copy starts at the
+// Odd phase, walls (not PER): what is half-way bounced back is staged where the cell
+// looks for it, one place on along c_z: own rows of c_z != 0 directions whose source
+// row lies beyond a wall, and the halo element at a z wall, with 8-byte copies (about one
+// row in fifteen of a 60 x 60 section).  Telling the cases apart at every read and store
+// instead cost a third more instructions than the even phase: 60x60x180 box with walls,
+// odd phase 117 us, 92 so (even 79); periodic 128^3 suspension, whose stores now take
+// their row from the table st.out, 397 to 359 us (even 322).
+// MIS (rows not 16-byte aligned, odd nz): each row copy starts at the
 // 16-byte boundary below the row and is rounded up to whole chunks (the
 // allocations carry 64 bytes of tail padding); the lead of every row is
 // published in st.lead.  The odd-phase halo elements are then read by lanes
 // 0..9 with plain loads and returned, to be put in place once the copy has
 // landed: the cell that reads and writes such a slot in this step lies in
-// this segment, so no other warp touches it meanwhile.
+// this segment, so no other warp touches it meanwhile.  Rows beyond a wall stay in place.
 // Lanes 0..9 also publish the segment geometry for the compute pass.
-template <typename T, bool ODD, bool MIS, bool STAGE_UP>
-__device__ __forceinline__ T issue_segment(const CollideArgs<T>& a, WarpStage<T, STAGE_UP>& st, int b, long long seg,
-                                           int dom) {
+// Output rows of the odd phase, st.out: the value of direction opp(i) of cell z goes to
+// [i] + z + c_z (the row that direction i was read from), at a z wall to [Q + i] + z (own
+// row), and across the periodic z boundary to [2 Q + i] + the wrapped z + c_z.  For a row
+// beyond a wall all three lead to slot i of the cell itself (MIS: [i] + z).
+template <bool ODD, bool PER, bool MIS, bool STAGE_UP>
+__device__ __forceinline__ double issue_segment(const CollideArgs<double>& a, WarpStage<double, STAGE_UP>& st, int b,
+                                                long long seg, int dom) {
+    using T = double;
     constexpr int V = WarpStage<T>::V;
     const int lane = threadIdx.x & 31;
     const Geom& g = a.g;
-    const SegGeo s = seg_geo(g, seg, a.dz, a.dy);
+    const SegGeo s = seg_geo<PER>(g, seg, a.dz, a.dy);
     const size_t N = g.N;
     const long long own = ((long long)s.x * g.ny + s.y) * g.nz;
-    if (lane < 9) st.row[b][lane] = row_off(g, s, lane / 3 - 1, lane % 3 - 1);
+    if (lane < 9) st.row[b][lane] = row_off<PER>(g, s, lane / 3 - 1, lane % 3 - 1);
 
     if (lane == 9) {
         st.geo[b][0] = s.x; st.geo[b][1] = s.y; st.geo[b][2] = s.z0; st.geo[b][3] = s.len; st.geo[b][4] = dom;
@@ -986,52 +1011,62 @@ __device__ __forceinline__ T issue_segment(const CollideArgs<T>& a, WarpStage<T,
     uint32_t bytes = 0;
     uint32_t lead = 0;
     T halo = T(0);
+    bool in = true;       // the lane's source row lies inside the lattice
+    bool bounce = false;  // the lane's halo element is bounced back at a z wall
     if (lane < Q) {
         const int i = lane;
-        size_t off = (size_t)i * N + (size_t)own + s.z0;
+        const size_t slot = (size_t)i * N + (size_t)own;
+        size_t off = slot;
         if (ODD && i != 0) {
-            const long long r = row_off(g, s, -cx(i), -cy(i));
-            if (r >= 0) off = (size_t)opp(i) * N + (size_t)r + s.z0;
+            const long long r = row_off<PER>(g, s, -cx(i), -cy(i));
+            in = PER || r >= 0;
+            if (in) off = (size_t)opp(i) * N + (size_t)r;
         }
-        src = a.f + off;
+        if (ODD) {
+            const int c = MIS || in ? 0 : cz(i);
+            st.out[b][i] = a.fo + off + c;
+            if (!PER) {
+                st.out[b][Q + i] = a.fo + slot;
+                st.out[b][2 * Q + i] = a.fo + off - c * (g.nz - 1);
+            }
+        }
+        src = a.f + off + s.z0;
         dst = &st.f[b][i][V];
         if (MIS) {
             lead = (uint32_t)(((uintptr_t)src & 15u) / sizeof(T));
             src -= lead;
             bytes = (uint32_t)(((lead + (uint32_t)s.len + V - 1) / V) * 16u);
-        } else {
+        } else if (!ODD || PER || in || cz(i) == 0) {
             bytes = (uint32_t)(s.len * sizeof(T));
         }
     } else if (ODD && !MIS && lane < Q + 10) {
         const int i = zdir(lane - Q);
-        const long long r = row_off(g, s, -cx(i), -cy(i));
-        if (r >= 0) {
+        const long long r = row_off<PER>(g, s, -cx(i), -cy(i));
+        if (PER || r >= 0) {
             int zc;      // first element of the 16-byte chunk (-1: beyond a z wall)
             if (cz(i) > 0) {
                 zc = s.z0 - V;
-                if (zc < 0) zc = g.per[2] ? zc + g.nz : -1;
+                if (zc < 0) zc = PER || g.per[2] ? zc + g.nz : -1;
                 dst = &st.f[b][i][0];
             } else {
                 zc = s.z0 + s.len;
-                if (zc >= g.nz) zc = g.per[2] ? zc - g.nz : -1;
+                if (zc >= g.nz) zc = PER || g.per[2] ? zc - g.nz : -1;
                 dst = &st.f[b][i][V + s.len];
             }
-            if (zc >= 0) {
+            if (PER || zc >= 0) {
                 src = a.f + (size_t)opp(i) * N + (size_t)r + zc;
                 bytes = 16;
+            } else {
+                bounce = true;
             }
         }
     } else if (lane == Q + 10) {
         const uint32_t* vs = a.vox + own + s.z0;
-        if (MIS) {
-            lead = (uint32_t)(((uintptr_t)vs & 15u) / 4u);
-            vs -= lead;
-            bytes = ((lead + (uint32_t)s.len + 3u) / 4u) * 16u;
-        } else {
-            bytes = (uint32_t)(s.len * sizeof(uint32_t));
-        }
-        src = reinterpret_cast<const T*>(vs);
+        const uint32_t vlead = (uint32_t)(((uintptr_t)vs & 15u) / 4u);
+        bytes = ((vlead + (uint32_t)s.len + 3u) / 4u) * 16u;
+        src = reinterpret_cast<const T*>(vs - vlead);
         dst = &st.vox[b][0];
+        st.geo[b][6] = (int)vlead;
     }
     // lanes 29, 30, 31: the surface-velocity rows (components 2, 0, 1) as a second copy
     const T* src2 = nullptr;
@@ -1051,9 +1086,8 @@ __device__ __forceinline__ T issue_segment(const CollideArgs<T>& a, WarpStage<T,
     }
     if (MIS) {
         const uint32_t lo = __reduce_or_sync(FULL, lane < 16 ? lead << (2 * lane) : 0u);
-        const uint32_t hi = __reduce_or_sync(
-            FULL, ((lane >= 16 && lane < Q) ? lead << (2 * (lane - 16)) : (lane == Q + 10 ? lead << 6 : 0u)) |
-                      ((STAGE_UP && lane >= Q + 10) ? lead2 << (8 + 2 * ud) : 0u));
+        const uint32_t hi = __reduce_or_sync(FULL, ((lane >= 16 && lane < Q) ? lead << (2 * (lane - 16)) : 0u) |
+                                                       ((STAGE_UP && lane >= Q + 10) ? lead2 << (8 + 2 * ud) : 0u));
         if (lane == 0) st.lead[b] = (unsigned long long)lo | ((unsigned long long)hi << 32);
         if (ODD && lane < 10) {
             const int i = zdir(lane);
@@ -1069,6 +1103,24 @@ __device__ __forceinline__ T issue_segment(const CollideArgs<T>& a, WarpStage<T,
                                    : a.f[(size_t)i * N + (size_t)own + g.nz - 1];
                 }
             }
+        }
+    }
+    if constexpr (ODD && !PER) {
+        const unsigned rows = __ballot_sync(FULL, in);
+        if constexpr (MIS) {
+            if (lane == 0) st.geo[b][5] = (int)rows;
+        } else {
+            if (bounce) {
+                const int i = zdir(lane - Q);
+                if (cz(i) > 0) cp8(&st.f[b][i][V - 1], a.f + (size_t)i * N + (size_t)own);
+                else cp8(&st.f[b][i][V + s.len], a.f + (size_t)i * N + (size_t)own + (g.nz - 1));
+            }
+            for (unsigned m = ~rows & ZDIRS; m; m &= m - 1u) {
+                const int i = __ffs(m) - 1;
+                const T* p = a.f + (size_t)i * N + (size_t)own + s.z0;
+                for (int j = lane; j < s.len; j += 32) cp8(&st.f[b][i][V - cz(i) + j], p + j);
+            }
+            cp_arrive(&st.bar[b]);
         }
     }
     const uint32_t total = __reduce_add_sync(FULL, bytes + bytes2);
@@ -1777,16 +1829,7 @@ k_collide_direct(const CollideArgs<float> a1, long long nseg, const CollideArgs<
 // (the axes are cycled in between), over values kept in the stage: fully unrolled
 // the update is 5000 instructions, and the warps, each at another place of it, then
 // wait for the instruction cache 80 % of the time.
-// Target row slots of direction q of the three cycles, four bits each.
-__host__ __device__ constexpr unsigned slot_bits(int q) {
-    unsigned v = 0;
-    for (int t = 0; t < 3; ++t) {
-        const int i = fixed::dir_of(t, q);
-        v |= (unsigned)row_slot(cx(i), cy(i)) << (4 * t);
-    }
-    return v;
-}
-
+// MIS: rows not aligned (see issue_segment).
 template <bool ODD, bool PER, bool MIS, bool STAGE_UP>
 struct StagedCell {
     static constexpr int ROW = WarpStage<double, STAGE_UP>::W;
@@ -1797,14 +1840,24 @@ struct StagedCell {
     unsigned N;           // cells (19 N doubles fit the memory, so N < 2^32)
     int b, z;
     size_t c;
-    int zm, zp;           // z - 1 and z + 1 (wrapped; -1 beyond a wall)
-    uint32_t srcrow;
+    int zm, zp;           // z - 1 and z + 1 (wrapped; z itself beyond a wall)
+    int tm, tp;           // and their part of the output rows: 0, Q at a wall, 2 Q wrapped
+    uint32_t rows;        // MIS: bit i: direction i's source row lies inside the lattice
     unsigned long long lead;
 
+    __device__ __forceinline__ StagedCell(const CollideArgs<double>& a, WarpStage<double, STAGE_UP>& stage, int buf,
+                                          int j, int z0, uint32_t inside, unsigned long long leads)
+        : st(stage), base(&stage.f[buf][0][WarpStage<double>::V + j]), fo(a.fo), upf(a.up), N((unsigned)a.g.N), b(buf),
+          z(z0 + j), c((size_t)stage.row[buf][row_slot(0, 0)] + (z0 + j)), zm(z - 1), zp(z + 1), tm(0), tp(0),
+          rows(inside), lead(leads) {
+        const bool wrap = PER || a.g.per[2];
+        if (z == 0) { zm = wrap ? a.g.nz - 1 : z; tm = wrap ? 2 * Q : Q; }
+        if (z == a.g.nz - 1) { zp = wrap ? 0 : z; tp = wrap ? 2 * Q : Q; }
+    }
     // the staged value of direction i (c_z = cz), the cell's own place in the stage
     __device__ __forceinline__ double* at(int i, int cz) const {
         int off = i * ROW;
-        if (ODD) off -= (PER || ((srcrow >> i) & 1u)) ? cz : 0;
+        if (ODD) off -= !MIS || ((rows >> i) & 1u) ? cz : 0;
         if (MIS) off += (int)((lead >> (2 * i)) & 3u);
         return base + off;
     }
@@ -1813,19 +1866,19 @@ struct StagedCell {
         const int m = MIS ? (int)((lead >> (40 + 2 * d)) & 3u) : 0;
         return st.up[b][d][m + j];
     }
-    // where the post-collision value of direction i (opposite o, target row slot rs) goes
-    __device__ __forceinline__ double* slot(int i, int o, int rs, int cz) const {
+    // where the post-collision value of direction i (opposite o, c_z = cz) goes: in both
+    // phases the row that direction o was read from, one cell on in the odd phase
+    __device__ __forceinline__ double* slot(int o, int cz) const {
         if (!ODD) return fo + c + (unsigned long long)(unsigned)o * N;
-        const long long r = st.row[b][rs];
-        const int zd = pick(cz, zm, z, zp);
-        if (PER || (r >= 0 && zd >= 0)) return fo + (unsigned long long)(unsigned)i * N + (size_t)(r + zd);
-        return fo + c + (unsigned long long)(unsigned)o * N;
+        if (MIS && !((rows >> o) & 1u)) return st.out[b][o] + z;
+        const int zd = pick(cz, zm, z, zp), t = PER ? 0 : pick(cz, tm, 0, tp);
+        return st.out[b][o + t] + zd;
     }
 };
 
 // The double routine for a cell outside the fixed-point range, out of line.
-template <bool ODD, bool FORCE, bool PER, bool MIS, bool STAGE_UP>
-__device__ __noinline__ void collide_cell_double(StagedCell<ODD, PER, MIS, STAGE_UP> s, double omega, double g0,
+template <bool FORCE, typename Cell>
+__device__ __noinline__ void collide_cell_double(Cell s, double omega, double g0,
                                                  double g1, double g2, int n, double B, double u0, double u1,
                                                  double u2, double (&F)[3]) {
     double f[Q];
@@ -1835,7 +1888,7 @@ __device__ __noinline__ void collide_cell_double(StagedCell<ODD, PER, MIS, STAGE
     else collide_cell_fp64<true>(f, omega, B, u0, u1, u2, F[0], F[1], F[2]);
     s.fo[s.c] = f[0];
 #pragma unroll
-    for (int i = 1; i < Q; ++i) *s.slot(i, opp(i), row_slot(cx(i), cy(i)), cz(i)) = f[i];
+    for (int i = 1; i < Q; ++i) *s.slot(opp(i), cz(i)) = f[i];
 }
 
 template <bool ODD, bool FORCE, bool PER, bool MIS, bool STAGE_UP>
@@ -1843,20 +1896,7 @@ __device__ __forceinline__ void collide_cell_staged(const CollideArgs<double>& a
                                                     int b, int j, int z0, uint32_t srcrow, unsigned long long lead,
                                                     uint32_t w, bool solid, double (&F)[3]) {
     using fixed::i64;
-    const Geom& g = a.g;
-    const int z = z0 + j;
-    const StagedCell<ODD, PER, MIS, STAGE_UP> s{st,
-                                                &st.f[b][0][WarpStage<double>::V + j],
-                                                a.fo,
-                                                a.up,
-                                                (unsigned)g.N,
-                                                b,
-                                                z,
-                                                (size_t)st.row[b][row_slot(0, 0)] + z,
-                                                wrap_minus(z, g.nz, PER ? 1 : g.per[2]),
-                                                wrap_plus(z, g.nz, PER ? 1 : g.per[2]),
-                                                srcrow,
-                                                lead};
+    const StagedCell<ODD, PER, MIS, STAGE_UP> s(a, st, b, j, z0, srcrow, lead);
     // the cell's unit
     double* const p0 = s.at(0, 0);
     int e = __double2hiint(*p0) & 0x7ff00000;
@@ -1874,7 +1914,7 @@ __device__ __forceinline__ void collide_cell_staged(const CollideArgs<double>& a
     }
     if (FORCE) e = fixed::cell_exponent_up(e, a.g3[0], a.g3[1], a.g3[2]);
     if (!fixed::fits(e)) {
-        collide_cell_double<ODD, FORCE, PER, MIS, STAGE_UP>(s, a.omega, a.g3[0], a.g3[1], a.g3[2], n, B, u0, u1, u2, F);
+        collide_cell_double<FORCE>(s, a.omega, a.g3[0], a.g3[1], a.g3[2], n, B, u0, u1, u2, F);
         return;
     }
     e = max(e, fixed::EMAX_LO);
@@ -1886,10 +1926,6 @@ __device__ __forceinline__ void collide_cell_staged(const CollideArgs<double>& a
     auto dir_z = [](int q, int a) {
         const int zc = q < 2 ? (a == 2 ? 1 : 0) : (a > 0 ? 1 : 0);
         return q == 0 || q == 2 || q == 5 ? zc : -zc;
-    };
-    auto dir_row = [](int q, int a) -> int {   // four bits per cycle
-        constexpr unsigned rows[6] = {slot_bits(0), slot_bits(1), slot_bits(2), slot_bits(3), slot_bits(4), slot_bits(5)};
-        return (int)((rows[q] >> (4 * a)) & 15u);
     };
 #pragma unroll 1
     for (int t = 0, dg = 0; t < 3; dg = t == 0 ? 4 : 2, ++t) {
@@ -1904,13 +1940,13 @@ __device__ __forceinline__ void collide_cell_staged(const CollideArgs<double>& a
     }
     fixed::Cell cell = fixed::cell_setup<FORCE>(solid, sum, e, fixed::relax_of(a.omega), a.g3[0], a.g3[1], a.g3[2],
                                                 n == 125, B, u0, u1, u2, F);
-    a.fo[s.c] = fixed::update_rest<FORCE>(solid, cell, X0, e);
+    *s.slot(0, 0) = fixed::update_rest<FORCE>(solid, cell, X0, e);
 #pragma unroll 1
     for (int t = 0, dg = 0; t < 3; dg = t == 0 ? 4 : 2, ++t) {
         fixed::update_three<FORCE>(
             solid, cell, t == 2,
             [&](int q) { return *reinterpret_cast<const i64*>(s.at(dir(q, t, dg), dir_z(q, t))); }, e,
-            [&](int q, double v) { *s.slot(dir(q, t, dg), dir(q ^ 1, t, dg), dir_row(q, t), dir_z(q, t)) = v; });
+            [&](int q, double v) { *s.slot(dir(q ^ 1, t, dg), dir_z(q, t)) = v; });
     }
 }
 
@@ -1944,6 +1980,8 @@ k_collide_staged(const CollideArgs<T> a1, long long nseg, const CollideArgs<T>* 
     // SW warps share a stage: warp `sub` of group `group`
     constexpr int SW = stage_warps<T>();
     constexpr int GROUPS = WARPS / SW;
+    // a buffer's arrivals: the bytes of its bulk copies, and every lane's own copies
+    constexpr uint32_t ARRIVALS = sizeof(T) == 8 && ODD && !PER && !MIS ? 33 : 1;
     const int group = warp / SW, sub = warp % SW;
     WarpStage<T, STAGE_UP>& st = reinterpret_cast<WarpStage<T, STAGE_UP>*>(smem_raw)[group];
     __shared__ unsigned long long probe[WARPS];   // the test hook's barrier (never completes)
@@ -1951,8 +1989,8 @@ k_collide_staged(const CollideArgs<T> a1, long long nseg, const CollideArgs<T>* 
     __shared__ unsigned long long shared_bar[SW > 1 ? GROUPS : 1][4];
     if (lane == 0) {
         if (sub == 0) {
-            mbar_init(&st.bar[0], 1);
-            mbar_init(&st.bar[1], 1);
+            mbar_init(&st.bar[0], ARRIVALS);
+            mbar_init(&st.bar[1], ARRIVALS);
             if (SW > 1)
                 for (int q = 0; q < 2; ++q) {
                     mbar_init(&shared_bar[group][q], SW);
@@ -1985,8 +2023,7 @@ k_collide_staged(const CollideArgs<T> a1, long long nseg, const CollideArgs<T>* 
         if constexpr (LSU) {
             issue_segment_lsu<T, ODD, PER, STAGE_UP>(a1, st, buf, sg);
             return T(0);
-        }
-        if (BATCH) {
+        } else if constexpr (BATCH) {
             int d, first;
             if (sseg0) {
                 int lo = 0, hi = ndom - 1;
@@ -2002,9 +2039,9 @@ k_collide_staged(const CollideArgs<T> a1, long long nseg, const CollideArgs<T>* 
                 first = __ldg(seg0 + d);
             }
             const CollideArgs<T>& A = dargs[d];
-            return issue_segment<T, ODD, MIS, STAGE_UP>(A, st, buf, sg - first, d);
+            return issue_segment<ODD, PER, MIS, STAGE_UP>(A, st, buf, sg - first, d);
         }
-        return issue_segment<T, ODD, MIS, STAGE_UP>(a1, st, buf, sg, 0);
+        else return issue_segment<ODD, PER, MIS, STAGE_UP>(a1, st, buf, sg, 0);
     };
     // segment k of the stage (buffer b = k & 1) is issued by warp k % SW, one segment
     // ahead; with two warps the same warp takes its first (solid) pass
@@ -2071,7 +2108,7 @@ k_collide_staged(const CollideArgs<T> a1, long long nseg, const CollideArgs<T>* 
         }
         // Odd phase with walls along z, aligned rows: the halo element of an edge
         // cell is its own slot i (half-way bounce-back).
-        if (!MIS && ODD && !PER && !g.per[2] && (z0 == 0 || z0 + len == g.nz)) {
+        if (sizeof(T) == 4 && ODD && !PER && !g.per[2] && (z0 == 0 || z0 + len == g.nz)) {
             if (lane < 10 && lead_warp) {
                 const int i = zdir(lane);
                 if (st.row[b][row_slot(-cx(i), -cy(i))] >= 0) {
@@ -2081,7 +2118,7 @@ k_collide_staged(const CollideArgs<T> a1, long long nseg, const CollideArgs<T>* 
             }
             __syncwarp();
         }
-        if constexpr (SW > 1 && ODD && !PER) {
+        if constexpr (SW > 1 && ODD && MIS) {
             // the other warp's cells read the halo elements that the lead warp put in place
             if (lead_warp) {
                 if (lane == 0) mbar_arrive(&shared_bar[group][2 + b]);
@@ -2095,7 +2132,9 @@ k_collide_staged(const CollideArgs<T> a1, long long nseg, const CollideArgs<T>* 
             }
         }
         uint32_t srcrow = 0;   // bit i: source row of direction i lies inside the lattice
-        if (ODD && !PER) {
+        if (ODD && sizeof(T) == 8) {
+            if (MIS) srcrow = (uint32_t)st.geo[b][5];
+        } else if (ODD && !PER) {
 #pragma unroll
             for (int i = 1; i < Q; ++i)
                 if (cz(i) != 0 && st.row[b][row_slot(-cx(i), -cy(i))] >= 0) srcrow |= 1u << i;
@@ -2110,8 +2149,8 @@ k_collide_staged(const CollideArgs<T> a1, long long nseg, const CollideArgs<T>* 
             // runs the solid terms for every lane, so gathering them leaves more
             // passes on the fluid path.  A cell's result does not depend on
             // its pass.
-            static_assert(SEGW == 64, "two passes of 32 cells per segment");
-            const int vlead = MIS ? (int)((lead >> 38) & 3u) : 0;
+            static_assert(SEGW == 64 && SW == 2, "two passes of 32 cells per segment, one for each warp");
+            const int vlead = st.geo[b][6];
             const uint32_t wl0 = lane < len ? st.vox[b][vlead + lane] : 0u;
             const uint32_t wl1 = lane + 32 < len ? st.vox[b][vlead + lane + 32] : 0u;
             const unsigned sol0 = __ballot_sync(FULL, (wl0 & VOX_NMASK) != 0u);
@@ -2120,24 +2159,26 @@ k_collide_staged(const CollideArgs<T> a1, long long nseg, const CollideArgs<T>* 
             const unsigned flu1 = __ballot_sync(FULL, lane + 32 < len) & ~sol1;
             const int ns0 = __popc(sol0), ns = ns0 + __popc(sol1);
             const int nf0 = __popc(flu0), nf = nf0 + __popc(flu1);
-#pragma unroll 1
-            for (int p = lead_warp ? 0 : 1; p < (lead_warp ? (SW > 1 ? 1 : 2) : 2); ++p) {
-                const int slot = 32 * p + lane;
-                int j = -1;   // the cell this lane takes in pass p
-                if (slot < ns) j = slot < ns0 ? nth_bit(sol0, slot) : 32 + nth_bit(sol1, slot - ns0);
-                else if (slot - ns < nf) j = slot - ns < nf0 ? nth_bit(flu0, slot - ns) : 32 + nth_bit(flu1, slot - ns - nf0);
-                const bool any_solid = ns > 32 * p;   // warp-uniform
-                if (j >= 0) {
-                    const uint32_t w = st.vox[b][vlead + j];
-                    T Fc[3];
-                    collide_cell_staged<ODD, FORCE, PER, MIS, STAGE_UP>(a, st, b, j, z0, srcrow, lead, w, any_solid, Fc);
-                    const size_t c = own + z0 + j;
-                    if (a.cf) { a.cf[c] = Fc[0]; a.cf[N + c] = Fc[1]; a.cf[2 * N + c] = Fc[2]; }
-                    if (any_solid) {
-                        T v[6] = {T(0), T(0), T(0), T(0), T(0), T(0)};
-                        const int key = cell_force_terms(a, w, sx, sy, z0 + j, Fc[0], Fc[1], Fc[2], v);
-                        if (key >= 0) add_cell_force(a, key, v);
-                    }
+            const int p = lead_warp ? 0 : 1;
+            const int slot = 32 * p + lane;
+            int j = -1;   // the cell this lane takes in pass p
+            if (slot < ns) j = slot < ns0 ? nth_bit(sol0, slot) : 32 + nth_bit(sol1, slot - ns0);
+            else if (slot - ns < nf) j = slot - ns < nf0 ? nth_bit(flu0, slot - ns) : 32 + nth_bit(flu1, slot - ns - nf0);
+            const bool any_solid = ns > 32 * p;   // warp-uniform
+            if (j >= 0) {
+                const uint32_t w = st.vox[b][vlead + j];
+                T Fc[3];
+                collide_cell_staged<ODD, FORCE, PER, MIS, STAGE_UP>(a, st, b, j, z0, srcrow, lead, w, any_solid, Fc);
+                // (the segment's data are read again: kept over the update they would spill)
+                if (a.cf) {
+                    const size_t c = (size_t)st.row[b][row_slot(0, 0)] + st.geo[b][2] + j;
+                    a.cf[c] = Fc[0]; a.cf[N + c] = Fc[1]; a.cf[2 * N + c] = Fc[2];
+                }
+                if (any_solid) {
+                    T v[6] = {T(0), T(0), T(0), T(0), T(0), T(0)};
+                    const int key = cell_force_terms(a, st.vox[b][vlead + j], st.geo[b][0], st.geo[b][1], st.geo[b][2] + j, Fc[0],
+                                                     Fc[1], Fc[2], v);
+                    if (key >= 0) add_cell_force(a, key, v);
                 }
             }
         }
@@ -2213,12 +2254,14 @@ cudaError_t launch_direct(const CollideArgs<float>& a, long long nseg, const Col
 template <typename T, bool ODD, bool FORCE>
 cudaError_t launch_one(const CollideArgs<T>& args, cudaStream_t s) {
     CollideArgs<T> a = args;
-    // Aligned rows: every row start and length 16-byte aligned for population rows
-    // (nz * sizeof(T)) and voxel-word rows (nz * 4), i.e. nz % 4 == 0, and 16-byte
-    // aligned arrays (device allocations are; a caller's out-of-place target that is
-    // not takes the other path)
+    // Aligned rows: every population row's start and length 16-byte aligned (nz *
+    // sizeof(T)), and 16-byte aligned arrays (device allocations are; a caller's
+    // out-of-place target that is not takes the other path).  The FP64 form copies
+    // voxel words from the boundary below the row, so an even nz is enough; rows of
+    // 2 (mod 4) cells go 6 / 20 % faster this way (160x48x50 channel, even / odd phase
+    // 72 / 95 us as unaligned rows, 68 / 74 us).
     const bool arrays_aligned = (((uintptr_t)a.f | (uintptr_t)a.fo | (uintptr_t)a.vox | (uintptr_t)a.up) & 15u) == 0;
-    const bool aligned = a.g.nz % 4 == 0 && arrays_aligned;
+    const bool aligned = a.g.nz % (sizeof(T) == 8 ? 2 : 4) == 0 && arrays_aligned;
     const int nzseg = (a.g.nz + SEGW - 1) / SEGW;
     a.dz = div_magic((unsigned)nzseg);
     a.dy = div_magic((unsigned)a.g.ny);
