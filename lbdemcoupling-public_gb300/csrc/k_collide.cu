@@ -857,8 +857,9 @@ struct alignas(16) WarpStage {
     T f[2][Q][W];
     uint32_t vox[2][SEGW + 4];
     T up[2][3][UW];        // particle surface velocity rows of the segment (when staged)
-    long long row[2][9];   // element offset of row (x + dx, y + dy) at [3 (dx + 1) + dy + 1]; -1 beyond a wall
-    T* out[2][sizeof(T) == 8 ? 3 * Q : 1];   // FP64, odd phase: output rows (see issue_segment)
+    long long row[2][sizeof(T) == 8 ? 9 : 1];   // FP64: element offset of row (x + dx, y + dy) at [3 (dx + 1) + dy + 1]; -1 beyond a wall
+    T* out[2][sizeof(T) == 8 ? 3 * Q : Q + 1];   // output rows (see issue_segment, issue_segment_lsu)
+    const T* src[sizeof(T) == 8 ? 1 : Q + 1];    // FP32: source rows of the segment being issued
     int geo[2][8];         // x, y, z0, len, domain, source rows inside, voxel lead of the segment in buffer b
     unsigned long long lead[2];   // unaligned rows: lead elements of row i at bits 2i, voxel row at bits 38,
                                   // surface-velocity row d at bits 40 + 2d
@@ -1153,20 +1154,13 @@ __device__ __forceinline__ void unroll_seq(std::integer_sequence<int, Ts...>, Fn
     (fn(std::integral_constant<int, Ts>{}), ...);
 }
 
-// Element offset of the source row of direction I (even: slot I of the own row;
-// odd: slot opp I of row x - c_I, or slot I of the own row beyond a wall).
-// PER: every axis periodic, the row x - c_I always exists.
-template <bool ODD, bool PER, int I>
-__device__ __forceinline__ size_t src_row(const long long* row, size_t N, size_t own) {
-    if constexpr (!ODD || I == 0) {
-        return (size_t)I * N + own;
-    } else {
-        const long long r = row[row_slot(-cx(I), -cy(I))];
-        if constexpr (PER) return (size_t)opp(I) * N + (size_t)r;
-        else return r >= 0 ? (size_t)opp(I) * N + (size_t)r : (size_t)I * N + own;
-    }
-}
-
+// The rows' addresses are formed once per segment, by one lane each, and kept in shared
+// memory: st.src[i] is the segment's source row of direction i (even: slot i of the own
+// row; odd: slot opp i of row x - c_i, or slot i of the own row beyond a wall), and
+// st.out[b][i] the same row of the output, which is where the value of direction opp(i)
+// goes.  (A copy or store then takes one shared load and one multiply-add.  With the
+// addresses formed at each of them a periodic 256^3 suspension took 445 / 545 us, even /
+// odd phase; so 433 / 530.)
 template <typename T, bool ODD, bool PER, bool STAGE_UP>
 __device__ __forceinline__ void issue_segment_lsu(const CollideArgs<T>& a, WarpStage<T, STAGE_UP>& st, int b,
                                                   long long seg) {
@@ -1179,34 +1173,34 @@ __device__ __forceinline__ void issue_segment_lsu(const CollideArgs<T>& a, WarpS
     const SegGeo s = seg_geo<PER>(g, seg, a.dz, a.dy);
     const size_t N = g.N;
     const size_t own = ((size_t)s.x * g.ny + s.y) * g.nz;
-    if (lane < 9) st.row[b][lane] = row_off<PER>(g, s, lane / 3 - 1, lane % 3 - 1);
-    if (lane == 9) {
-        st.geo[b][0] = s.x; st.geo[b][1] = s.y; st.geo[b][2] = s.z0; st.geo[b][3] = s.len; st.geo[b][4] = 0;
+    bool in = true;   // the lane's source row lies inside the lattice
+    if (lane < Q) {
+        const int i = lane;
+        size_t off = (size_t)i * N + own;
+        if (ODD && i != 0) {
+            const long long r = row_off<PER>(g, s, -cx(i), -cy(i));
+            in = PER || r >= 0;
+            if (in) off = (size_t)opp(i) * N + (size_t)r;
+        }
+        st.src[i] = a.f + off + s.z0;
+        st.out[b][i] = a.fo + off + s.z0;
+    }
+    if (lane == Q) {
+        st.geo[b][0] = s.x; st.geo[b][1] = s.y; st.geo[b][2] = s.z0; st.geo[b][3] = s.len;
+    }
+    if (ODD && !PER) {
+        const unsigned rows = __ballot_sync(FULL, in);
+        if (lane == 0) st.geo[b][5] = (int)rows;
     }
     __syncwarp();
-    const long long* row = st.row[b];
     const int c = lane % CPR, sub = lane / CPR;
     const bool cin = c * V < s.len;   // rows of aligned lattices end on a chunk boundary
-    const T* f = a.f;
     // population rows: pass t covers directions t * RPI + sub
-    unroll_seq(std::make_integer_sequence<int, (Q + RPI - 1) / RPI>{}, [&](auto tc) {
-        constexpr int t = decltype(tc)::value;
-        constexpr int i0 = t * RPI, i1 = t * RPI + 1;
-        if constexpr (RPI == 1 || i1 >= Q) {
-            if (sub == 0 && cin) cp16(&st.f[b][i0][V + c * V], f + src_row<ODD, PER, i0>(row, N, own) + s.z0 + c * V);
-        } else {
-            size_t off;
-            if constexpr (ODD && PER && i0 != 0) {
-                // one row lookup per pass: the lane's direction picks slot and array
-                constexpr int s0 = row_slot(-cx(i0), -cy(i0)), s1 = row_slot(-cx(i1), -cy(i1));
-                const long long r = row[sub == 0 ? s0 : s1];
-                off = (size_t)(sub == 0 ? opp(i0) : opp(i1)) * N + (size_t)r;
-            } else {
-                off = sub == 0 ? src_row<ODD, PER, i0>(row, N, own) : src_row<ODD, PER, i1>(row, N, own);
-            }
-            if (cin) cp16(&st.f[b][sub == 0 ? i0 : i1][V + c * V], f + off + s.z0 + c * V);
-        }
-    });
+#pragma unroll
+    for (int t = 0; t < (Q + RPI - 1) / RPI; ++t) {
+        const int i = t * RPI + sub;
+        if (cin && (RPI * (t + 1) <= Q || i < Q)) cp16(&st.f[b][i][V + c * V], st.src[i] + c * V);
+    }
     // then: voxel row (SEGW / 4 chunks), surface-velocity rows (3 CPR), halo chunks
     // (odd phase, 10) -- in that order, so that only the first pass mixes two kinds
     constexpr int NH = ODD ? 10 : 0, NV = SEGW / 4, NU = STAGE_UP ? 3 * CPR : 0;
@@ -1218,8 +1212,7 @@ __device__ __forceinline__ void issue_segment_lsu(const CollideArgs<T>& a, WarpS
         if (kk >= NX) continue;
         if (k < NH) {
             const int i = zdir(k);
-            const long long r = row[row_slot(-cx(i), -cy(i))];
-            if (!PER && r < 0) continue;
+            if (!PER && row_off(g, s, -cx(i), -cy(i)) < 0) continue;
             int zc;     // first element of the chunk holding the halo (-1: beyond a z wall)
             T* dst;
             if (cz(i) > 0) {
@@ -1231,7 +1224,7 @@ __device__ __forceinline__ void issue_segment_lsu(const CollideArgs<T>& a, WarpS
                 if (zc >= g.nz) zc = (PER || g.per[2]) ? zc - g.nz : -1;
                 dst = &st.f[b][i][V + s.len];
             }
-            if (zc >= 0) cp16(dst, f + (size_t)opp(i) * N + (size_t)r + zc);
+            if (zc >= 0) cp16(dst, st.src[i] + (zc - s.z0));
         } else if (k < NH + NV) {
             const int cv = k - NH;
             if (cv * 4 < s.len) cp16(&st.vox[b][cv * 4], a.vox + own + s.z0 + cv * 4);
@@ -1443,12 +1436,9 @@ __device__ __forceinline__ void collide_segment_pairs(const CollideArgs<float>& 
     const int lane = threadIdx.x & 31;
     const Geom& g = a.g;
     const size_t N = g.N;
-    float* F = a.fo;
-    const size_t own = (size_t)st.row[b][row_slot(0, 0)];
     const int j0 = 2 * lane, j1 = j0 + 1;
     const bool v0 = j0 < len, v1 = j1 < len;
     const int za = z0 + j0, zb = z0 + j1;
-    const size_t ca = own + za, cb = own + zb;
 
     // staged values of direction i for the lane's two cells
     auto at2 = [&](int i) -> F2 {
@@ -1531,61 +1521,52 @@ __device__ __forceinline__ void collide_segment_pairs(const CollideArgs<float>& 
         }
     }
 
-    // Stores.  put(off, x, y, vx, vy): values x, y into slots off, off + 1 (one 64-bit
-    // store when both are valid and the pair is aligned).
-    auto put = [&](size_t off, float x, float y, bool vx, bool vy) {
-        // aligned rows only (the launcher sends arrays that are not 16-byte aligned
-        // to k_collide_direct): an even slot offset is an 8-byte aligned pair
-        if (vx && vy) {
-            *reinterpret_cast<float2*>(F + off) = make_float2(x, y);
-        } else {
-            if (vx) F[off] = x;
-            if (vy) F[off + 1] = y;
-        }
-    };
-    // the lane's two cells into slots (i, base + j0) and (i, base + j1)
-    auto put_cells = [&](size_t base, F2 v) {
+    // Stores (aligned rows only, the launcher sends others to k_collide_direct)
+    // the lane's two cells in place in a row
+    auto put_cells = [&](float* row, F2 v) {
         const float2 t = upk(v);
         // segments hold a multiple of 4 cells, so both cells of a pair are valid together,
         // and every pair of slots is 8-byte aligned
-        if (v0) *reinterpret_cast<float2*>(F + base + j0) = t;
+        if (v0) *reinterpret_cast<float2*>(row + j0) = t;
     };
-    if (!ODD) {
+    const size_t own = ((size_t)sx * g.ny + sy) * g.nz;
+    put_cells(st.out[b][0], f[0]);
+    // Odd phase, c_z != 0: each cell goes to slot z + c_z.  Slots (j0, j0 + 1) receive cells
+    // (j0 - 1, j0) (c_z = +1) or (j0 + 1, j0 + 2) (c_z = -1), one lane over; the first and
+    // the last lane store one value alone: the pair that is cut off by the segment's end, and
+    // the cell whose slot lies outside it (wrapped, or bounced back at a z wall).  Both go out
+    // in one predicated store: as branches of those two lanes they cost a warp one divergence
+    // per direction (256^3 odd phase 530 us, 496 so = 78 % of the copy rate).
+    const int last = len / 2 - 1;
+    const bool pair_p = lane > 0 && v0, pair_m = lane < last, single = lane == 0 || lane == last;
+    const int per_z = PER ? 1 : g.per[2];
+    const int zdp = wrap_plus(z0 + len - 1, g.nz, per_z), zdm = wrap_minus(z0, g.nz, per_z);
+    const int single_p = lane == 0 ? 1 : zdp - z0, single_m = lane == 0 ? zdm - z0 : j0;
 #pragma unroll
-        for (int i = 0; i < Q; ++i) put_cells((size_t)opp(i) * N + own + z0, f[i]);
-    } else {
-        put_cells(own + z0, f[0]);
-        const int per_z = PER ? 1 : g.per[2];
-#pragma unroll
-        for (int i = 1; i < Q; ++i) {
-            const long long r = st.row[b][row_slot(cx(i), cy(i))];
-            if (!PER && r < 0) {            // beyond an x / y wall: bounce back in place
-                put_cells((size_t)opp(i) * N + own + z0, f[i]);
-                continue;
-            }
-            const size_t dst = (size_t)i * N + (size_t)r;   // row x + c_i
-            if (cz(i) == 0) {
-                put_cells(dst + z0, f[i]);
-                continue;
-            }
-            // c_z != 0: each cell to slot z + c_z (wrapped, or bounced back at a z wall)
-            const float2 t = upk(f[i]);
-            // slots (j0, j0 + 1) of this lane receive cells (j0 - 1, j0) (c_z = +1)
-            // or (j0 + 1, j0 + 2) (c_z = -1), one lane over; the cell whose slot
-            // lies outside the segment (je) is stored on its own
-            if (cz(i) > 0) put(dst + z0 + j0, __shfl_up_sync(FULL, t.y, 1), t.x, lane > 0 && v0, v1);
-            else put(dst + z0 + j0, t.y, __shfl_down_sync(FULL, t.x, 1), v1, j0 + 2 < len);
-            const int je = cz(i) > 0 ? len - 1 : 0;
-            const int ze = z0 + je;
-            const int zd = cz(i) > 0 ? wrap_plus(ze, g.nz, per_z) : wrap_minus(ze, g.nz, per_z);
-            const size_t eoff = (PER || zd >= 0) ? dst + zd : (size_t)opp(i) * N + own + ze;
-            const float ev = (je & 1) ? t.y : t.x;
-            if (lane == (je >> 1)) F[eoff] = ev;
+    for (int i = 1; i < Q; ++i) {
+        // row x + c_i; beyond an x / y wall the cell's own (bounce back in place)
+        float* const row = st.out[b][opp(i)];
+        if (!ODD || cz(i) == 0 || (!PER && !((srcrow >> opp(i)) & 1u))) {
+            put_cells(row, f[i]);
+            continue;
         }
+        const float2 t = upk(f[i]);
+        float* q = row + (cz(i) > 0 ? single_p : single_m);
+        if (cz(i) > 0) {
+            const float o = __shfl_up_sync(FULL, t.y, 1);
+            if (pair_p) *reinterpret_cast<float2*>(row + j0) = make_float2(o, t.x);
+            if (!PER && zdp < 0 && lane != 0) q = a.fo + (size_t)opp(i) * N + own + z0 + len - 1;
+        } else {
+            const float o = __shfl_down_sync(FULL, t.x, 1);
+            if (pair_m) *reinterpret_cast<float2*>(row + j0) = make_float2(t.y, o);
+            if (!PER && zdm < 0 && lane == 0) q = a.fo + (size_t)opp(i) * N + own;
+        }
+        if (single) *q = lane == 0 ? t.x : t.y;
     }
 
     const float2 fx = upk(Fx), fy = upk(Fy), fz = upk(Fz);
     if (a.cf) {
+        const size_t ca = own + za, cb = own + zb;
         if (v0) { a.cf[ca] = fx.x; a.cf[N + ca] = fy.x; a.cf[2 * N + ca] = fz.x; }
         if (v1) { a.cf[cb] = fx.y; a.cf[N + cb] = fy.y; a.cf[2 * N + cb] = fz.y; }
     }
@@ -2093,7 +2074,7 @@ k_collide_staged(const CollideArgs<T> a1, long long nseg, const CollideArgs<T>* 
         const Geom& g = a.g;
         const size_t N = g.N;
         const T* Fin = a.f;   // input populations
-        const size_t own = (size_t)st.row[b][row_slot(0, 0)];
+        const size_t own = ((size_t)sx * g.ny + sy) * g.nz;
         const unsigned long long lead = MIS ? st.lead[b] : 0ull;
         if (MIS && ODD) {
             if (lane < 10 && lead_warp) {
@@ -2108,10 +2089,11 @@ k_collide_staged(const CollideArgs<T> a1, long long nseg, const CollideArgs<T>* 
         }
         // Odd phase with walls along z, aligned rows: the halo element of an edge
         // cell is its own slot i (half-way bounce-back).
+        const uint32_t srcrow = ODD && !PER ? (uint32_t)st.geo[b][5] : 0u;   // bit i: direction i's source row is inside
         if (sizeof(T) == 4 && ODD && !PER && !g.per[2] && (z0 == 0 || z0 + len == g.nz)) {
-            if (lane < 10 && lead_warp) {
+            if (lane < 10) {
                 const int i = zdir(lane);
-                if (st.row[b][row_slot(-cx(i), -cy(i))] >= 0) {
+                if ((srcrow >> i) & 1u) {
                     if (cz(i) > 0 && z0 == 0) st.f[b][i][V - 1] = Fin[(size_t)i * N + own];
                     if (cz(i) < 0 && z0 + len == g.nz) st.f[b][i][V + len] = Fin[(size_t)i * N + own + g.nz - 1];
                 }
@@ -2130,14 +2112,6 @@ k_collide_staged(const CollideArgs<T> a1, long long nseg, const CollideArgs<T>* 
                 if (next < nseg) mbar_wait(&st.bar[b ^ 1], (phase >> (b ^ 1)) & 1u);
                 return;
             }
-        }
-        uint32_t srcrow = 0;   // bit i: source row of direction i lies inside the lattice
-        if (ODD && sizeof(T) == 8) {
-            if (MIS) srcrow = (uint32_t)st.geo[b][5];
-        } else if (ODD && !PER) {
-#pragma unroll
-            for (int i = 1; i < Q; ++i)
-                if (cz(i) != 0 && st.row[b][row_slot(-cx(i), -cy(i))] >= 0) srcrow |= 1u << i;
         }
         if constexpr (sizeof(T) == 4) {
             static_assert(LSU, "FP32: aligned rows of a single lattice (others: k_collide_direct)");
