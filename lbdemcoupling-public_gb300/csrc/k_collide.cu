@@ -1607,42 +1607,56 @@ __device__ __forceinline__ void collide_segment_pairs(const CollideArgs<float>& 
 // FP32 form without staging: lattices whose rows are not 16-byte aligned, and
 // every batch.  Lane l takes the cells l and l + 32 of a 64-cell segment and reads and
 // writes global memory directly: every access is a coalesced 32-bit one whatever its
-// alignment, and a cell's source and target slots follow from its own index and its six
-// neighbours' displacements, so a segment needs no set-up.  (Staged, such rows cost a
+// alignment.  (Staged, such rows cost a
 // bulk copy per row with its own lead, and halo elements put in place by hand: even / odd
 // phase of a 71x67x243 channel 34.8 / 54.7 us staged, 32.4 / 35.5 us here = 82 / 75 % of
 // the copy bandwidth; of 512 batched channels, 75.6 M cells, 2.80 / 5.27 and 2.61 /
-// 3.40 ms.)  16 warps per SM at 128 registers; 20 or 24 spill and are slower.
+// 3.19 ms.)  16 warps per SM at 128 registers; 20 or 24 spill and are slower.
+// Odd phase: a cell's source and target rows come from a table of the segment in shared
+// memory, with entries for the cells at a z wall or wrap, so that an access is one
+// shared load and one multiply-add (slots formed from the cell's index, with a test for
+// walls at each: 3.40 ms for the 512 channels, where every row ends at two walls).
 // A segment lies in a z-row, or, in the even phase of a batch, which touches only each
 // cell's own slots, in an x-plane across its z-rows (the plane view: the lanes are filled
 // whatever the row length; force and torque then take per-cell arms).
 struct DirectCell {
     unsigned own;      // index in the domain, also of its voxel word
     int y, z;
-    unsigned dz[2];    // displacement of the neighbour at z - 1, z + 1 (wrapped)
-    unsigned wall;     // bit 0..5: no neighbour at x - 1, x + 1, y - 1, y + 1, z - 1, z + 1
+    int zn[2];         // odd phase: z - 1, z + 1 (wrapped; z itself beyond a wall)
+    int t[2];          // and their part of the row table: 0, Q at a wall, 2 Q wrapped
 };
-// The walls that stand between a cell and its neighbour at (-cx, -cy, -cz).
-__host__ __device__ constexpr unsigned wall_bits(int i) {
-    return (cx(i) > 0 ? 1u : cx(i) < 0 ? 2u : 0u) | (cy(i) > 0 ? 4u : cy(i) < 0 ? 8u : 0u) |
-           (cz(i) > 0 ? 16u : cz(i) < 0 ? 32u : 0u);
+// Odd phase: slot that direction I of the cell is read from: slot opp I of the neighbour at
+// x - c_I, or the cell's own slot I beyond a wall.  The value that streams along I goes to
+// the slot of opp I: in the AA pattern a cell reads and writes the same slots.  T: the
+// segment's row table (direct_rows).
+template <int I>
+__device__ __forceinline__ float* direct_slot(float* const* T, const DirectCell& c) {
+    if constexpr (cz(I) == 0) return T[I] + c.z;
+    else return T[I + c.t[cz(I) > 0 ? 0 : 1]] + c.zn[cz(I) > 0 ? 0 : 1];
 }
-// Slot that direction I of the cell is read from (odd phase): slot opp I of the
-// neighbour at x - c_I, or the cell's own slot I beyond a wall.  The value that streams
-// along I goes to the slot of opp I: in the AA pattern a cell reads and writes the same
-// slots.  dx, dy: displacements of the rows at x - 1, x + 1 and y - 1, y + 1; indices are
-// modulo 2^32.
-template <bool WALLS, int I>
-__device__ __forceinline__ float* direct_slot(float* F, unsigned N, const DirectCell& c, const unsigned (&dx)[2],
-                                              const unsigned (&dy)[2]) {
-    unsigned idx = c.own;
-    if constexpr (cz(I) != 0) idx += c.dz[cz(I) > 0 ? 0 : 1];
-    unsigned d = 0;
-    if constexpr (cx(I) != 0) d += dx[cx(I) > 0 ? 0 : 1];
-    if constexpr (cy(I) != 0) d += dy[cy(I) > 0 ? 0 : 1];
-    float* p = F + (unsigned long long)opp(I) * N + (idx + d);
-    if (WALLS && (c.wall & wall_bits(I))) p = F + (unsigned long long)I * N + c.own;
-    return p;
+// The row table of a segment of row (x, y), made by one warp, one direction a lane:
+// [i] the row that direction i is read from, [Q + i] the cells' own (at a z wall), [2 Q + i]
+// that row again (across the periodic z boundary).  Beyond an x / y wall all three lead to
+// slot i of the cell itself, whatever c_z did to its z.
+__device__ __forceinline__ void direct_rows(float** T, float* F, const Geom& g, int x, int y) {
+    const int i = threadIdx.x & 31;
+    __syncwarp();   // the last segment's reads
+    if (i < Q) {
+        const unsigned own = ((unsigned)x * (unsigned)g.ny + (unsigned)y) * (unsigned)g.nz;
+        float* const slot = F + ((size_t)i * g.N + own);
+        const int X = pick(cx(i), wrap_plus(x, g.nx, g.per[0]), x, wrap_minus(x, g.nx, g.per[0]));
+        const int Y = pick(cy(i), wrap_plus(y, g.ny, g.per[1]), y, wrap_minus(y, g.ny, g.per[1]));
+        if (i != 0 && X >= 0 && Y >= 0) {
+            float* const row = F + ((size_t)opp(i) * g.N + ((unsigned)X * (unsigned)g.ny + (unsigned)Y) * (unsigned)g.nz);
+            T[i] = row;
+            T[2 * Q + i] = row;
+        } else {
+            T[i] = slot + cz(i);
+            T[2 * Q + i] = slot - cz(i) * (g.nz - 1);
+        }
+        T[Q + i] = slot;
+    }
+    __syncwarp();
 }
 
 template <bool ODD, bool FORCE, bool BATCH>
@@ -1652,6 +1666,9 @@ k_collide_direct(const CollideArgs<float> a1, long long nseg, const CollideArgs<
     constexpr bool PLANE = BATCH && !ODD;
     extern __shared__ __align__(16) unsigned char smem_raw[];
     const int lane = threadIdx.x & 31;
+    __shared__ float* rows[ODD ? DIRECT_BLOCK / 32 : 1][2][ODD ? 3 * Q : 1];   // row tables: input, output
+    float** const Tin = rows[ODD ? threadIdx.x >> 5 : 0][0];
+    float** const Tout = rows[ODD ? threadIdx.x >> 5 : 0][1];
     PairTables<BATCH ? NO_TABLES : 0> tb{false};
     const int* sseg0 = nullptr;   // batch: the CTA's copy of seg0 (ndom <= SEG0_SMEM)
     if constexpr (BATCH) {
@@ -1707,14 +1724,9 @@ k_collide_direct(const CollideArgs<float> a1, long long nseg, const CollideArgs<
         const unsigned rowbase = row * (unsigned)a.g.nz;
         float* F = a.fo;
         const float* Fin = a.f;
-        const unsigned unz = (unsigned)g.nz, xs = (unsigned)g.ny * unz;
-        const unsigned dx[2] = {x > 0 ? 0u - xs : (unsigned)(g.nx - 1) * xs,
-                                x < g.nx - 1 ? xs : 0u - (unsigned)(g.nx - 1) * xs};
-        const unsigned dy[2] = {y > 0 ? 0u - unz : xs - unz, y < g.ny - 1 ? unz : unz - xs};
-        unsigned wall = 0u;
-        if (ODD) {
-            if (!g.per[0]) wall |= (x == 0 ? 1u : 0u) | (x == g.nx - 1 ? 2u : 0u);
-            if (!g.per[1]) wall |= (y == 0 ? 4u : 0u) | (y == g.ny - 1 ? 8u : 0u);
+        if constexpr (ODD) {
+            direct_rows(Tin, const_cast<float*>(Fin), g, x, y);
+            if (F != Fin) direct_rows(Tout, F, g, x, y);
         }
         DirectCell c[2];
         bool valid[2];
@@ -1734,15 +1746,14 @@ k_collide_direct(const CollideArgs<float> a1, long long nseg, const CollideArgs<
                 q.z = pc - q.y * g.nz;
             }
             if (ODD) {
-                const bool lo = pc == 0, hi = pc == g.nz - 1;
-                q.dz[0] = lo ? unz - 1u : ~0u;
-                q.dz[1] = hi ? 1u - unz : 1u;
-                q.wall = wall;
-                if (!g.per[2]) q.wall |= (lo ? 16u : 0u) | (hi ? 32u : 0u);
+                q.zn[0] = pc - 1;
+                q.zn[1] = pc + 1;
+                q.t[0] = q.t[1] = 0;
+                if (pc == 0) { q.zn[0] = g.per[2] ? g.nz - 1 : pc; q.t[0] = g.per[2] ? 2 * Q : Q; }
+                if (pc == g.nz - 1) { q.zn[1] = g.per[2] ? 0 : pc; q.t[1] = g.per[2] ? 2 * Q : Q; }
             }
         }
         F2 f[Q];
-        bool walls = false;
         if constexpr (!ODD) {
 #pragma unroll
             for (int i = 0; i < Q; ++i) {
@@ -1750,17 +1761,10 @@ k_collide_direct(const CollideArgs<float> a1, long long nseg, const CollideArgs<
                 f[i] = pk(r[c[0].own], r[c[1].own]);
             }
         } else {
-            walls = __any_sync(FULL, (c[0].wall | c[1].wall) != 0u);
-            float* R = const_cast<float*>(Fin);
-            auto load = [&](auto wc) {
-                constexpr bool WALLS = decltype(wc)::value;
-                unroll_seq(std::make_integer_sequence<int, Q>{}, [&](auto ic) {
-                    constexpr int i = decltype(ic)::value;
-                    f[i] = pk(*direct_slot<WALLS, i>(R, N, c[0], dx, dy), *direct_slot<WALLS, i>(R, N, c[1], dx, dy));
-                });
-            };
-            if (walls) load(std::true_type{});
-            else load(std::false_type{});
+            unroll_seq(std::make_integer_sequence<int, Q>{}, [&](auto ic) {
+                constexpr int i = decltype(ic)::value;
+                f[i] = pk(*direct_slot<i>(Tin, c[0]), *direct_slot<i>(Tin, c[1]));
+            });
         }
         PairForce o;
         collide_pair<FORCE>(a, g, tb, f, valid[0] ? w[0] : 0u, valid[1] ? w[1] : 0u, x, c[0].y, c[0].z, c[1].y, c[1].z,
@@ -1774,17 +1778,13 @@ k_collide_direct(const CollideArgs<float> a1, long long nseg, const CollideArgs<
                 if (valid[1]) r[c[1].own] = t.y;
             }
         } else {
-            auto store = [&](auto wc) {
-                constexpr bool WALLS = decltype(wc)::value;
-                unroll_seq(std::make_integer_sequence<int, Q>{}, [&](auto ic) {
-                    constexpr int i = decltype(ic)::value;
-                    const float2 t = upk(f[i]);
-                    if (valid[0]) *direct_slot<WALLS, opp(i)>(F, N, c[0], dx, dy) = t.x;
-                    if (valid[1]) *direct_slot<WALLS, opp(i)>(F, N, c[1], dx, dy) = t.y;
-                });
-            };
-            if (walls) store(std::true_type{});
-            else store(std::false_type{});
+            float** const T = F != Fin ? Tout : Tin;
+            unroll_seq(std::make_integer_sequence<int, Q>{}, [&](auto ic) {
+                constexpr int i = decltype(ic)::value;
+                const float2 t = upk(f[i]);
+                if (valid[0]) *direct_slot<opp(i)>(T, c[0]) = t.x;
+                if (valid[1]) *direct_slot<opp(i)>(T, c[1]) = t.y;
+            });
         }
         if (a.cf) {
             const float2 fx = upk(o.Fx), fy = upk(o.Fy), fz = upk(o.Fz);
