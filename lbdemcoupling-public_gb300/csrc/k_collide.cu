@@ -670,9 +670,8 @@ __device__ __forceinline__ void arm_terms(T dx, T dy, T dz, const Geom& g, T Fx,
     v[5] = dx * Fy - dy * Fx;
 }
 
-template <typename T>
-__device__ __forceinline__ int cell_force_terms(const CollideArgs<T>& a, uint32_t w, int x, int y, int z, T Fx,
-                                                T Fy, T Fz, T (&v)[6]) {
+__device__ __forceinline__ int cell_force_terms(const CollideArgs<double>& a, uint32_t w, int x, int y, int z,
+                                                double Fx, double Fy, double Fz, double (&v)[6]) {
     if ((w & VOX_NMASK) == 0) return -1;
     const int tag = (int)(w >> VOX_NBITS);
     const int slot = tag <= a.max_tag ? __ldg(a.tag2slot + tag) : -1;
@@ -680,20 +679,8 @@ __device__ __forceinline__ int cell_force_terms(const CollideArgs<T>& a, uint32_
         atomicOr(a.err, 0x8u);   // LBDEM_DEVERR_UNMAPPED_TAG
         return -1;
     }
-    T dx, dy, dz;
-    if (sizeof(T) == 8) {
-        const double* p = a.rec + (size_t)slot * REC_STRIDE;
-        dx = T((double)x - __ldg(p + 0));
-        dy = T((double)y - __ldg(p + 1));
-        dz = T((double)z - __ldg(p + 2));
-    } else {
-        // centre = hi + lo in float: (x - hi) - lo is the arm to ~1 ulp
-        const float4* p = reinterpret_cast<const float4*>(a.xpf + (size_t)slot * XPF_STRIDE);
-        const float4 h = __ldg(p), l = __ldg(p + 1);
-        dx = T(((float)x - h.x) - h.w);
-        dy = T(((float)y - h.y) - l.x);
-        dz = T(((float)z - h.z) - l.y);
-    }
+    const double* p = a.rec + (size_t)slot * REC_STRIDE;
+    const double dx = (double)x - __ldg(p + 0), dy = (double)y - __ldg(p + 1), dz = (double)z - __ldg(p + 2);
     arm_terms(dx, dy, dz, a.g, Fx, Fy, Fz, v);
     return slot;
 }
@@ -1348,7 +1335,7 @@ __device__ __forceinline__ void collide_pair(const CollideArgs<float>& a, const 
 // several rows, or wrap around a periodic row), reduced over the warp per run of equal
 // owner; v0, v1: the lane slots that hold a cell.  Must be reached by all 32 lanes.
 __device__ __forceinline__ void forces_by_cell(const CollideArgs<float>& a, const Geom& g, const PairForce& o,
-                                               int x, int ya, int za, int yb, int zb) {
+                                               int x, int ya, int za, int yb, int zb, bool apart) {
     if (o.unmapped) atomicOr(a.err, 0x8u);   // LBDEM_DEVERR_UNMAPPED_TAG
     const int ka = o.s0, kb = o.s1;
     if (!__any_sync(FULL, ka >= 0 || kb >= 0)) return;
@@ -1369,7 +1356,7 @@ __device__ __forceinline__ void forces_by_cell(const CollideArgs<float>& a, cons
     float va[6] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f}, vb[6] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
     if (ka >= 0) terms(ka, ya, za, fx.x, fy.x, fz.x, va);
     if (kb >= 0) terms(kb, yb, zb, fx.y, fy.y, fz.y, vb);
-    const bool one = __all_sync(FULL, ka < 0 || kb < 0 || ka == kb);   // one reduction for both cells
+    const bool one = !apart && __all_sync(FULL, ka < 0 || kb < 0 || ka == kb);   // one reduction for both cells
     if (one) {
 #pragma unroll
         for (int q = 0; q < 6; ++q) va[q] += vb[q];
@@ -1385,8 +1372,8 @@ __device__ __forceinline__ void forces_by_cell(const CollideArgs<float>& a, cons
 // Force and torque of the two cells of a lane in one row segment, reduced per run of
 // equal owner (finish_run), arms from the segment's middle point zc; the two cells go
 // through one warp reduction when their owners agree.  Must be reached by all 32 lanes.
-__device__ __forceinline__ void forces_by_run(const CollideArgs<float>& a, const PairForce& o, int x, int y, int zc,
-                                              int za, int zb) {
+__device__ __forceinline__ void forces_by_run(const CollideArgs<float>& a, const PairForce& o, int x, int ya, int yb,
+                                              int zc, int za, int zb, bool apart) {
     if (o.unmapped) atomicOr(a.err, 0x8u);   // LBDEM_DEVERR_UNMAPPED_TAG
     const int ka = o.s0, kb = o.s1;
     if (!__any_sync(FULL, ka >= 0 || kb >= 0)) return;
@@ -1399,7 +1386,7 @@ __device__ __forceinline__ void forces_by_run(const CollideArgs<float>& a, const
         if (ka < 0) va[q] = 0.f;
         if (kb < 0) vb[q] = 0.f;
     }
-    const bool one = __all_sync(FULL, ka < 0 || kb < 0 || ka == kb);   // one reduction for both cells
+    const bool one = !apart && __all_sync(FULL, ka < 0 || kb < 0 || ka == kb);   // one reduction for both cells
     if (one) {
 #pragma unroll
         for (int q = 0; q < 5; ++q) va[q] += vb[q];
@@ -1412,13 +1399,13 @@ __device__ __forceinline__ void forces_by_run(const CollideArgs<float>& a, const
 #pragma unroll
         for (int q = 0; q < 5; ++q) v[q] = pass == 0 ? va[q] : vb[q];
         const bool second = pass == 1 || (one && ka < 0);   // the run's cells are the b cells
-        reduce_runs(a, second ? kb : ka, v, second ? zb : za, x, y, zc, o.rh, o.rl0, o.rl1, o.vslot);
+        reduce_runs(a, second ? kb : ka, v, second ? zb : za, x, second ? yb : ya, zc, o.rh, o.rl0, o.rl1, o.vslot);
     }
 }
 // forces_by_cell out of line, for the rare segments of the row kernels.
-__device__ __noinline__ void forces_by_cell_far(const CollideArgs<float>& a, PairForce o, int x, int y, int za,
-                                                int zb) {
-    forces_by_cell(a, a.g, o, x, y, za, y, zb);
+__device__ __noinline__ void forces_by_cell_far(const CollideArgs<float>& a, PairForce o, int x, int ya, int za,
+                                                int yb, int zb, bool apart) {
+    forces_by_cell(a, a.g, o, x, ya, za, yb, zb, apart);
 }
 
 // FP32 compute pass over one staged segment of a lattice with 16-byte aligned rows, two
@@ -1574,7 +1561,7 @@ __device__ __forceinline__ void collide_segment_pairs(const CollideArgs<float>& 
         // the segment is a whole z-periodic row: a particle's chord may wrap
         // around inside it, so the arms are taken per cell
         forces_by_cell_far(a, PairForce{Fx, Fy, Fz, s0, s1, vslot, (n0 > 0 && s0 < 0) || (n1 > 0 && s1 < 0), vrh, vrl0, vrl1},
-                           sx, sy, za, zb);
+                           sx, sy, za, sy, zb, false);
         return;
     }
     // runs of equal owner, arms from the segment's middle point zc
@@ -1611,11 +1598,11 @@ __device__ __forceinline__ void collide_segment_pairs(const CollideArgs<float>& 
 // bulk copy per row with its own lead, and halo elements put in place by hand: even / odd
 // phase of a 71x67x243 channel 34.8 / 54.7 us staged, 32.4 / 35.5 us here = 82 / 75 % of
 // the copy bandwidth; of 512 batched channels, 75.6 M cells, 2.80 / 5.27 and 2.61 /
-// 3.19 ms.)  16 warps per SM at 128 registers; 20 or 24 spill and are slower.
+// 3.08 ms.)  16 warps per SM at 128 registers; 20 or 24 spill and are slower.
 // Odd phase: a cell's source and target rows come from a table of the segment in shared
 // memory, with entries for the cells at a z wall or wrap, so that an access is one
-// shared load and one multiply-add (slots formed from the cell's index, with a test for
-// walls at each: 3.40 ms for the 512 channels, where every row ends at two walls).
+// shared load and one multiply-add (slots formed from the cell's index at each access, and
+// again with tests in warps at a wall: 3.40 ms for the 512 channels).
 // A segment lies in a z-row, or, in the even phase of a batch, which touches only each
 // cell's own slots, in an x-plane across its z-rows (the plane view: the lanes are filled
 // whatever the row length; force and torque then take per-cell arms).
@@ -1664,9 +1651,11 @@ __global__ void __launch_bounds__(DIRECT_BLOCK, DIRECT_BLOCKS_PER_SM)
 k_collide_direct(const CollideArgs<float> a1, long long nseg, const CollideArgs<float>* __restrict__ dargs,
                  const int* __restrict__ seg0, int ndom) {
     constexpr bool PLANE = BATCH && !ODD;
+    constexpr bool ROWS2 = BATCH && ODD;
     extern __shared__ __align__(16) unsigned char smem_raw[];
     const int lane = threadIdx.x & 31;
-    __shared__ float* rows[ODD ? DIRECT_BLOCK / 32 : 1][2][ODD ? 3 * Q : 1];   // row tables: input, output
+    // row tables: input, and output or (batch, in place) the second row's
+    __shared__ float* rows[ODD ? DIRECT_BLOCK / 32 : 1][2][ODD ? 3 * Q : 1];
     float** const Tin = rows[ODD ? threadIdx.x >> 5 : 0][0];
     float** const Tout = rows[ODD ? threadIdx.x >> 5 : 0][1];
     PairTables<BATCH ? NO_TABLES : 0> tb{false};
@@ -1718,28 +1707,57 @@ k_collide_direct(const CollideArgs<float> a1, long long nseg, const CollideArgs<
         const unsigned N = (unsigned)g.N;   // 19 N floats fit the memory, so N < 2^32
         const unsigned sg = seg - (unsigned)first;
         const unsigned row = fast_div(sg, a.dz);
-        const int z0 = (int)(sg - row * a.dz.d) * SEGW;
+        int z0 = (int)(sg - row * a.dz.d) * SEGW;
         const int x = (int)fast_div(row, a.dy);
-        const int y = (int)(row - (unsigned)x * a.dy.d);
-        const unsigned rowbase = row * (unsigned)a.g.nz;
+        int y = (int)(row - (unsigned)x * a.dy.d);
+        unsigned rowbase = row * (unsigned)a.g.nz;
+        bool two = false;    // the lane's second cell lies in the next row
+        bool there = true;   // the segment's row exists
+        if (ROWS2 && tails_paired(g.nz)) {
+            // `row` is a pair of rows, dz divides by the pair's segments: the full ones of each
+            // row, then both tails
+            const int full = g.nz / SEGW;
+            int k = z0 / SEGW;
+            two = k == 2 * full;
+            y *= 2;
+            if (two) k = full;
+            else if (k >= full) { k -= full; ++y; }
+            z0 = k * SEGW;
+            there = y < g.ny;
+            if (!there) --y;
+            rowbase = ((unsigned)x * (unsigned)g.ny + (unsigned)y) * (unsigned)g.nz;
+        }
+        const int hz = two ? 0 : 32;   // z of a lane's second cell, from its first
         float* F = a.fo;
         const float* Fin = a.f;
         if constexpr (ODD) {
             direct_rows(Tin, const_cast<float*>(Fin), g, x, y);
-            if (F != Fin) direct_rows(Tout, F, g, x, y);
+            if (BATCH && two) direct_rows(Tout, F, g, x, min(y + 1, g.ny - 1));
+            if (!BATCH && F != Fin) direct_rows(Tout, F, g, x, y);
         }
         DirectCell c[2];
         bool valid[2];
         uint32_t w[2];
 #pragma unroll
         for (int h = 0; h < 2; ++h) {
-            const int p = z0 + lane + 32 * h;
+            const int p = z0 + lane + hz * h;
             valid[h] = p < a.g.nz;
             const int pc = valid[h] ? p : a.g.nz - 1;   // a lane slot past the row reads its last cell
             DirectCell& q = c[h];
             q.own = rowbase + (unsigned)pc;
-            w[h] = a.vox[q.own];
             q.y = y;
+            if (ROWS2) {
+                valid[h] = valid[h] && there;
+                if (two && h == 1) {
+                    if (y + 1 < g.ny) {
+                        q.y = y + 1;
+                        q.own += (unsigned)g.nz;
+                    } else {
+                        valid[1] = false;
+                    }
+                }
+            }
+            w[h] = a.vox[q.own];
             q.z = pc;
             if (PLANE) {
                 q.y = (int)fast_div((unsigned)pc, a.dnz);
@@ -1753,6 +1771,8 @@ k_collide_direct(const CollideArgs<float> a1, long long nseg, const CollideArgs<
                 if (pc == g.nz - 1) { q.zn[1] = g.per[2] ? 0 : pc; q.t[1] = g.per[2] ? 2 * Q : Q; }
             }
         }
+        // rows of the lane's second cells (a batch steps in place: its output rows too)
+        float* const* const T1 = ROWS2 && two ? Tout : Tin;
         F2 f[Q];
         if constexpr (!ODD) {
 #pragma unroll
@@ -1763,7 +1783,7 @@ k_collide_direct(const CollideArgs<float> a1, long long nseg, const CollideArgs<
         } else {
             unroll_seq(std::make_integer_sequence<int, Q>{}, [&](auto ic) {
                 constexpr int i = decltype(ic)::value;
-                f[i] = pk(*direct_slot<i>(Tin, c[0]), *direct_slot<i>(Tin, c[1]));
+                f[i] = pk(*direct_slot<i>(Tin, c[0]), *direct_slot<i>(T1, c[1]));
             });
         }
         PairForce o;
@@ -1778,12 +1798,13 @@ k_collide_direct(const CollideArgs<float> a1, long long nseg, const CollideArgs<
                 if (valid[1]) r[c[1].own] = t.y;
             }
         } else {
-            float** const T = F != Fin ? Tout : Tin;
+            float* const* const O0 = !BATCH && F != Fin ? Tout : Tin;
+            float* const* const O1 = BATCH ? T1 : O0;
             unroll_seq(std::make_integer_sequence<int, Q>{}, [&](auto ic) {
                 constexpr int i = decltype(ic)::value;
                 const float2 t = upk(f[i]);
-                if (valid[0]) *direct_slot<opp(i)>(T, c[0]) = t.x;
-                if (valid[1]) *direct_slot<opp(i)>(T, c[1]) = t.y;
+                if (valid[0]) *direct_slot<opp(i)>(O0, c[0]) = t.x;
+                if (valid[1]) *direct_slot<opp(i)>(O1, c[1]) = t.y;
             });
         }
         if (a.cf) {
@@ -1792,13 +1813,13 @@ k_collide_direct(const CollideArgs<float> a1, long long nseg, const CollideArgs<
             if (valid[1]) { a.cf[c[1].own] = fx.y; a.cf[N + c[1].own] = fy.y; a.cf[2ull * N + c[1].own] = fz.y; }
         }
         if (PLANE) {
-            forces_by_cell(a, g, o, x, c[0].y, c[0].z, c[1].y, c[1].z);
+            forces_by_cell(a, g, o, x, c[0].y, c[0].z, c[1].y, c[1].z, false);
         } else if (g.per[2] && g.nz <= SEGW) {
             // the segment is a whole z-periodic row: a particle's chord may wrap around inside
             // it, so the arms are taken per cell
-            forces_by_cell_far(a, o, x, y, z0 + lane, z0 + lane + 32);
+            forces_by_cell_far(a, o, x, y, z0 + lane, c[1].y, z0 + lane + hz, two);
         } else {
-            forces_by_run(a, o, x, y, z0 + SEGW / 2, z0 + lane, z0 + lane + 32);
+            forces_by_run(a, o, x, y, c[1].y, z0 + SEGW / 2, z0 + lane, z0 + lane + hz, two);
         }
     }
 }

@@ -189,6 +189,16 @@ long long box_cells(const int32_t* b) {
 template <typename T>
 T* fptr(lbdem_batch* b, int d) { return (T*)b->f + b->views[d].f0; }
 
+// An x-plane's rows (FP32: or pairs of rows, tails_paired) and the segments of each, as the
+// collide-stream kernels number them.
+struct RowSplit {
+    int rows, segs;
+};
+RowSplit row_split(int ny, int nz, size_t esz) {
+    if (esz == 4 && tails_paired(nz)) return {(ny + 1) / 2, 2 * (nz / COLLIDE_SEGW) + 1};
+    return {ny, (nz + COLLIDE_SEGW - 1) / COLLIDE_SEGW};
+}
+
 // out[d]: domain d as rows of nz cells; out[ndom + d]: the same domain as nx rows
 // of ny nz cells (the plane view of the FP32 even phase, whose update touches
 // only each cell's own slots).
@@ -215,8 +225,9 @@ void fill_dargs(lbdem_batch* b, std::vector<CollideArgs<T>>& out, T* f_base, dou
         a.btab = (const T*)b->btab + (size_t)126 * d;
         a.omega = (T)b->dom[d].omega;
         for (int k = 0; k < 3; ++k) a.g3[k] = (T)b->dom[d].body_force[k];
-        a.dz = div_magic((unsigned)((v.g.nz + COLLIDE_SEGW - 1) / COLLIDE_SEGW));
-        a.dy = div_magic((unsigned)v.g.ny);
+        const RowSplit rs = row_split(v.g.ny, v.g.nz, sizeof(T));
+        a.dz = div_magic((unsigned)rs.segs);
+        a.dy = div_magic((unsigned)rs.rows);
         CollideArgs<T>& p = out[b->ndom + d];
         p = a;
         const int plane = v.g.ny * v.g.nz;
@@ -474,7 +485,8 @@ lbdem_status lbdem_batch_create(const lbdem_batch_config* cfg, int32_t ndomains,
         b->cap[d] = dm.max_particles;
         slots += dm.max_particles;
         tiles += (long long)((dm.nx + TILE - 1) / TILE) * ((dm.ny + TILE - 1) / TILE) * ((dm.nz + TILE - 1) / TILE);
-        segs += (long long)dm.nx * dm.ny * ((dm.nz + COLLIDE_SEGW - 1) / COLLIDE_SEGW);
+        const RowSplit rs = row_split(dm.ny, dm.nz, b->esz);
+        segs += (long long)dm.nx * rs.rows * rs.segs;
         psegs += (long long)dm.nx * (((long long)dm.ny * dm.nz + COLLIDE_SEGW - 1) / COLLIDE_SEGW);
         fo += round_up((size_t)Q * v.g.N, 32);
         co += round_up(v.g.N, 32);

@@ -157,6 +157,14 @@ struct CollideArgs {
     DivMagic dnz;
 };
 
+// FP32 batch, odd phase: rows whose last segment holds at most half a segment are taken in
+// pairs (y, y + 1): the full segments of each, then one segment of both tails, a lane's
+// cells in the two rows (each row's forces still summed on its own).  Rows of 64 to 160
+// cells fill 76 % of the lane slots singly, 88 % so: 512 channels, odd phase 3.19 to 3.08 ms.
+__host__ __device__ inline bool tails_paired(int nz) {
+    return nz % COLLIDE_SEGW >= 1 && nz % COLLIDE_SEGW <= COLLIDE_SEGW / 2;
+}
+
 // Float table of a particle list, one row of XPF_STRIDE floats per particle:
 //   {xh0, xh1, xh2, xl0 | xl1, xl2, v0, v1 | v2, w0, w1, w2 | 0, 0, 0, 0},
 // centre = xh + xl (hi/lo split), velocity and angular velocity rounded to float.
