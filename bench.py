@@ -528,19 +528,22 @@ def main():
     ach64 = BYTES_PER_CELL["fp64"] * N / (r64["k1_ms"] * 1e-3) / 1e9 if r64 else None
     # the coupled step against the same bytes: K1's algorithmic bytes per whole step
     step32 = BYTES_PER_CELL["fp32"] * N / (t32 / args.steps * 1e-3) / 1e9
-    # FP64 form against its own ceiling: double-precision lanes per clock per SM (2 on
-    # GB300) x SMs x the median SM clock sampled during its run
+    # FP64 form's use of the FP64 pipe: double-precision lanes per clock per SM (2 on
+    # GB300) x SMs x the median SM clock sampled during its run.  (Its cells are updated in
+    # fixed point on the integer pipe; the double operations left convert the results and
+    # form the torque arms.)
     fp64_pipe = None
     if r64 and traffic.get("fp64_dp_ops") and r64["clocks"].get("sm_mhz"):
         ops = traffic["fp64_dp_ops"]
         rate = ops / (r64["k1_ms"] * 1e-3) / 1e12
         peak_dp = 2.0 * sm_count(device) * r64["clocks"]["sm_mhz"] * 1e6 / 1e12
-        fp64_pipe = {"bound": "fp64", "achieved": rate, "peak": peak_dp, "unit": "T DP lane-ops/s",
+        fp64_pipe = {"bound": "integer issue", "achieved": rate, "peak": peak_dp, "unit": "T DP lane-ops/s",
                      "frac": rate / peak_dp, "dp_ops_per_launch": ops, "dp_ops_per_cell": ops / N,
                      "peak_source": "2 FP64 lanes per clock per SM x SMs x median SM clock of the FP64 run",
                      "pipe_active_frac": (traffic["fp64_pipe_active"] / 100.0) if traffic.get("fp64_pipe_active")
                                          else None,
-                     "pipe_note": "achieved/peak counts add/mul/fma only; pipe_active_frac (ncu) counts every "
+                     "pipe_note": "use of the FP64 pipe, not the kernel's bound; achieved/peak counts add/mul/fma "
+                                  "only; pipe_active_frac (ncu) counts every "
                                   "FP64-pipe instruction (conversions, compares, the reciprocal sequence)",
                      "ops_source": "ncu smsp__sass_thread_inst_executed_op_d{add,mul,fma}_pred_on.sum, "
                                    "profiles/collide_stream_traffic.txt"}
@@ -583,7 +586,7 @@ def main():
             "vs_cpu": (v64 / cpu["value"]) if cpu else None,
             "vs_cpu_note": "FP64 form against the FP64 CPU oracle of cpu_baseline (same precision)",
             "clocks": r64["clocks"],
-            "roofline": fp64_pipe if fp64_pipe else {"bound": "fp64", "achieved": None, "frac": None},
+            "roofline": fp64_pipe if fp64_pipe else {"bound": "integer issue", "achieved": None, "frac": None},
             "hbm": {"achieved": ach64, "peak": peak, "unit": "GB/s", "frac": ach64 / peak,
                     "traffic": traffic.get("fp64"), "kernel": "k_collide_staged<double> (all axes periodic)",
                     "bytes_per_cell": BYTES_PER_CELL["fp64"]},
