@@ -248,7 +248,7 @@ __device__ __forceinline__ CellAdj<T> adjoint_cell(const T (&f)[Q], const T (&mu
 // ---------------------------------------------------------------------------
 // The same reverse in double, built from moments.  GB300 has two double lanes per clock
 // per SM, and the sums above, written per direction, take about 600 double operations
-// for a fluid cell and 1500 for a solid one (553 us a step at 64^3, against 0.29 ms here).  Every sum over the
+// for a fluid cell and 1500 for a solid one (553 us a step at 64^3, against 264 here).  Every sum over the
 // directions is a contraction of
 //   M0 = sum t mu,  M1 = sum t mu c,  M2 = sum t mu c c,  sum mu_k f_k,  sum mu_k f_opp(k)
 // with the cell's vectors (feq and the source are quadratic in c), so those are formed
@@ -474,12 +474,52 @@ __device__ __forceinline__ void reduce6(int key, T (&v)[6], double* __restrict__
         for (int q = 0; q < 6; ++q) atomicAdd(out + 6 * (size_t)key + q, (double)v[q]);
 }
 
+// A run's rows in shared memory, made by one warp, one direction a lane: a load or store
+// then takes one shared load and one multiply-add (FP32 step at 128^3: 155 us with the addresses
+// formed at each, 138 so; FP64 at 64^3, bound by its double operations: 270 and 264).
+// [f + k] the row that f_k is read from (f: even phase the run's own; odd phase slot opp k of
+// row x - c_k), [mu + k] that of mu_k (slot k of row x + c_k), each followed by the entries
+// for a z wall (the own row's slot, index z) and for the periodic z boundary; [out + k] the
+// run's own row of lambda_out.  Beyond an x / y wall all three lead to the cell itself,
+// whatever c_z did to its z.
+constexpr int ROWS_F = 0, ROWS_MU = 3 * Q, ROWS_OUT = 6 * Q, ROWS_ALL = 7 * Q;
+template <typename T, bool PER>
+__device__ __forceinline__ void adjoint_rows(T** rows, const AdjointArgs<T>& A, int x, int y) {
+    const int k = threadIdx.x & 31;
+    const Geom& g = A.g;
+    __syncwarp();   // the last run's reads
+    if (k < Q) {
+        const size_t N = g.N, own = ((size_t)x * g.ny + y) * g.nz;
+        // row (x + dx, y + dy), or -1 beyond a wall
+        auto row = [&](int dx, int dy) -> long long {
+            int X = x + dx, Y = y + dy;
+            if (X < 0 || X >= g.nx) X = PER || g.per[0] ? (X < 0 ? g.nx - 1 : 0) : -1;
+            if (Y < 0 || Y >= g.ny) Y = PER || g.per[1] ? (Y < 0 ? g.ny - 1 : 0) : -1;
+            return PER || (X >= 0 && Y >= 0) ? ((long long)X * g.ny + Y) * g.nz : -1;
+        };
+        auto entries = [&](T** t, T* base, int slot, int back, long long r, int c) {
+            T* const self = base + ((size_t)back * N + own);
+            T* const there = base + ((size_t)slot * N + (size_t)(r >= 0 ? r : 0));
+            t[k] = PER || r >= 0 ? there : self - c;
+            t[Q + k] = self;
+            t[2 * Q + k] = PER || r >= 0 ? there : self + c * (g.nz - 1);
+        };
+        T* const f = const_cast<T*>(A.f);
+        if (A.phase == 0) rows[ROWS_F + k] = f + ((size_t)k * N + own);
+        else entries(rows + ROWS_F, f, opp(k), k, row(-cx(k), -cy(k)), -cz(k));
+        entries(rows + ROWS_MU, const_cast<T*>(A.lam_in), k, opp(k), row(cx(k), cy(k)), cz(k));
+        rows[ROWS_OUT + k] = A.lam_out + ((size_t)k * N + own);
+    }
+    __syncwarp();
+}
+
 // PER: every axis periodic (no wall cases in the neighbour lookups).
 template <typename T, bool PER>
 __global__ void __launch_bounds__(ADJ_THREADS, sizeof(T) == 4 ? 2 : 1) k_adjoint_step(const AdjointArgs<T> A) {
     __shared__ double s_red[ADJ_THREADS / 32][4];
+    __shared__ T* s_rows[ADJ_THREADS / 32][ROWS_ALL];
+    T** const rows = s_rows[threadIdx.x >> 5];
     const Geom g = A.g;
-    const size_t N = g.N;
     T gtau = T(0), gg[3] = {T(0), T(0), T(0)};   // per-thread sums, widened once
     // one warp per 64-cell run of a z-row, in two passes of 32 cells: rows * runs
     // < 2^31 (nx * ny < 2^31 is checked at creation), so all index arithmetic
@@ -496,6 +536,8 @@ __global__ void __launch_bounds__(ADJ_THREADS, sizeof(T) == 4 ? 2 : 1) k_adjoint
         const int row = qi / nzc;
         const int zb = (qi - row * nzc) * 64;
         const int len = min(64, g.nz - zb);
+        const int x = row / g.ny, y = row - x * g.ny;
+        adjoint_rows<T, PER>(rows, A, x, y);
         const size_t rowc = (size_t)row * g.nz + zb;
         const uint32_t wl0 = lane < len ? A.vox[rowc + lane] : 0u;
         const uint32_t wl1 = lane + 32 < len ? A.vox[rowc + lane + 32] : 0u;
@@ -517,46 +559,27 @@ __global__ void __launch_bounds__(ADJ_THREADS, sizeof(T) == 4 ? 2 : 1) k_adjoint
             int key = -1;
             T pv[6] = {T(0), T(0), T(0), T(0), T(0), T(0)};
             if (jr >= 0) {
-                const int x = row / g.ny;
-                const int y = row - x * g.ny;
                 const size_t c = (size_t)row * g.nz + z;
-                // neighbour coordinates (-1 beyond a wall) and the nine row offsets
-                const bool p0 = PER || g.per[0], p1 = PER || g.per[1], p2 = PER || g.per[2];
-                const int xs[3] = {x > 0 ? x - 1 : (p0 ? g.nx - 1 : -1), x, x < g.nx - 1 ? x + 1 : (p0 ? 0 : -1)};
-                const int ys[3] = {y > 0 ? y - 1 : (p1 ? g.ny - 1 : -1), y, y < g.ny - 1 ? y + 1 : (p1 ? 0 : -1)};
-                const int zs[3] = {z > 0 ? z - 1 : (p2 ? g.nz - 1 : -1), z, z < g.nz - 1 ? z + 1 : (p2 ? 0 : -1)};
-                long long rowoff[9];
-#pragma unroll
-                for (int a = 0; a < 3; ++a)
-#pragma unroll
-                    for (int b = 0; b < 3; ++b)
-                        rowoff[3 * a + b] =
-                            (PER || (xs[a] >= 0 && ys[b] >= 0)) ? ((long long)xs[a] * g.ny + ys[b]) * g.nz : -1;
-                // cell x + (dx, dy, dz) as a linear index, or -1 beyond a wall
-                auto nb = [&](int dx, int dy, int dz) -> long long {
-                    const long long r = rowoff[3 * (dx + 1) + dy + 1];
-                    const int zz = zs[dz + 1];
-                    return (PER || (r >= 0 && zz >= 0)) ? r + zz : -1;
+                // z - 1, z, z + 1 (wrapped; z itself beyond a wall) and their part of the row table
+                int zs[3] = {z - 1, z, z + 1}, ts[3] = {0, 0, 0};
+                const bool wrap = PER || g.per[2];
+                if (z == 0) { zs[0] = wrap ? g.nz - 1 : z; ts[0] = wrap ? 2 * Q : Q; }
+                if (z == g.nz - 1) { zs[2] = wrap ? 0 : z; ts[2] = wrap ? 2 * Q : Q; }
+                auto at = [&](int tab, int k, int dz) -> T {
+                    return rows[tab + k + (PER ? 0 : ts[dz + 1])][zs[dz + 1]];
                 };
                 T f[Q], mu[Q];
                 if (A.phase == 0) {
 #pragma unroll
-                    for (int k = 0; k < Q; ++k) f[k] = A.f[(size_t)k * N + c];
+                    for (int k = 0; k < Q; ++k) f[k] = rows[ROWS_F + k][z];
                 } else {
                     // odd layout: f_k(x) in slot (opp k, x - c_k), or (k, x) when x - c_k is beyond a wall
-                    f[0] = A.f[c];
 #pragma unroll
-                    for (int k = 1; k < Q; ++k) {
-                        const long long s2 = nb(-cx(k), -cy(k), -cz(k));
-                        f[k] = s2 >= 0 ? A.f[(size_t)opp(k) * N + (size_t)s2] : A.f[(size_t)k * N + c];
-                    }
+                    for (int k = 0; k < Q; ++k) f[k] = at(ROWS_F, k, -cz(k));
                 }
                 // transpose of push streaming: mu_k = lambda_k(x + c_k), or lambda_opp k(x) beyond a wall
 #pragma unroll
-                for (int k = 0; k < Q; ++k) {
-                    const long long s2 = k == 0 ? (long long)c : nb(cx(k), cy(k), cz(k));
-                    mu[k] = s2 >= 0 ? A.lam_in[(size_t)k * N + (size_t)s2] : A.lam_in[(size_t)opp(k) * N + c];
-                }
+                for (int k = 0; k < Q; ++k) mu[k] = at(ROWS_MU, k, cz(k));
                 const uint32_t w = A.vox[c];
                 int n = min((int)(w & VOX_NMASK), 125);
                 T uP[3] = {T(0), T(0), T(0)}, a[3] = {T(0), T(0), T(0)}, d[3] = {T(0), T(0), T(0)};
@@ -614,14 +637,14 @@ __global__ void __launch_bounds__(ADJ_THREADS, sizeof(T) == 4 ? 2 : 1) k_adjoint
                     const CellAdjD R =
                         adjoint_cell_double(f, mu, n, general, B, dBdtau, uP, a, A.omega, gvec, guP, gtau, gg);
                     // lambda_k = am mu_k + B mu_opp(k) + k0 + c_k.v (a fluid cell has B = 0 and am = 1 - omega)
-                    A.lam_out[c] = fma(R.am, mu[0], fma(R.B, mu[0], R.k0));
+                    rows[ROWS_OUT][z] = fma(R.am, mu[0], fma(R.B, mu[0], R.k0));
 #pragma unroll
                     for (int k = 10; k < Q; ++k) {
                         const int i = k - 9;
                         const double cv = cdotT<double>(k, R.v0, R.v1, R.v2);
                         const double hi = R.k0 + cv, lo = R.k0 - cv;
-                        A.lam_out[(size_t)k * N + c] = fma(R.am, mu[k], general ? fma(R.B, mu[i], hi) : hi);
-                        A.lam_out[(size_t)i * N + c] = fma(R.am, mu[i], general ? fma(R.B, mu[k], lo) : lo);
+                        rows[ROWS_OUT + k][z] = fma(R.am, mu[k], general ? fma(R.B, mu[i], hi) : hi);
+                        rows[ROWS_OUT + i][z] = fma(R.am, mu[i], general ? fma(R.B, mu[k], lo) : lo);
                     }
                 } else {
                     const CellAdj<T> R =
@@ -630,7 +653,7 @@ __global__ void __launch_bounds__(ADJ_THREADS, sizeof(T) == 4 ? 2 : 1) k_adjoint
                     if (!general) {   // fluid cells only: phi = mu, no solid terms
 #pragma unroll
                         for (int k = 0; k < Q; ++k)
-                            A.lam_out[(size_t)k * N + c] = om1 * mu[k] + (R.grb + cdotT<T>(k, R.gJ0, R.gJ1, R.gJ2));
+                            rows[ROWS_OUT + k][z] = om1 * mu[k] + (R.grb + cdotT<T>(k, R.gJ0, R.gJ1, R.gJ2));
                     } else {
                         // the fluid path's expression plus the solid terms (exactly zero for a fluid cell)
 #pragma unroll
@@ -638,7 +661,7 @@ __global__ void __launch_bounds__(ADJ_THREADS, sizeof(T) == 4 ? 2 : 1) k_adjoint
                             const T phi = R.sB * mu[k] + R.grbs + cdotT<T>(k, R.gjs0, R.gjs1, R.gjs2);
                             T l = om1 * phi + (R.grb + cdotT<T>(k, R.gJ0, R.gJ1, R.gJ2));
                             l += R.B * mu[opp(k)] + T(2) * R.B * cdotT<T>(k, a[0], a[1], a[2]);
-                            A.lam_out[(size_t)k * N + c] = l;
+                            rows[ROWS_OUT + k][z] = l;
                         }
                     }
                 }
