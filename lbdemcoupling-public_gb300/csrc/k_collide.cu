@@ -967,20 +967,20 @@ __device__ __forceinline__ void cp_arrive(unsigned long long* bar) {
 // instead cost a third more instructions than the even phase: 60x60x180 box with walls,
 // odd phase 117 us, 92 so (even 79); periodic 128^3 suspension, whose stores now take
 // their row from the table st.out, 397 to 359 us (even 322).
-// MIS (rows not 16-byte aligned, odd nz): each row copy starts at the
-// 16-byte boundary below the row and is rounded up to whole chunks (the
-// allocations carry 64 bytes of tail padding); the lead of every row is
-// published in st.lead.  The odd-phase halo elements are then read by lanes
-// 0..9 with plain loads and returned, to be put in place once the copy has
-// landed: the cell that reads and writes such a slot in this step lies in
-// this segment, so no other warp touches it meanwhile.  Rows beyond a wall stay in place.
+// MIS (rows not 16-byte aligned, odd nz, every batch): a row lies in the stage behind its
+// lead, the elements between it and the 16-byte boundary below; the leads are published in
+// st.lead.  Even phase: the copy starts at that boundary and is rounded up to whole chunks
+// (the allocations carry 64 bytes of tail padding).  Odd phase: the halo elements lie where
+// such chunks would write, so the whole chunks inside the row go out as a bulk copy, and
+// its cut ends and the halo elements as 8-byte copies (put in place by hand after the copy,
+// between the stage's two warps: 60x60x179 box, odd phase 98 us, 88 so).
 // Lanes 0..9 also publish the segment geometry for the compute pass.
 // Output rows of the odd phase, st.out: the value of direction opp(i) of cell z goes to
 // [i] + z + c_z (the row that direction i was read from), at a z wall to [Q + i] + z (own
 // row), and across the periodic z boundary to [2 Q + i] + the wrapped z + c_z.  For a row
-// beyond a wall all three lead to slot i of the cell itself (MIS: [i] + z).
+// beyond a wall all three lead to slot i of the cell itself.
 template <bool ODD, bool PER, bool MIS, bool STAGE_UP>
-__device__ __forceinline__ double issue_segment(const CollideArgs<double>& a, WarpStage<double, STAGE_UP>& st, int b,
+__device__ __forceinline__ void issue_segment(const CollideArgs<double>& a, WarpStage<double, STAGE_UP>& st, int b,
                                                 long long seg, int dom) {
     using T = double;
     constexpr int V = WarpStage<T>::V;
@@ -998,7 +998,6 @@ __device__ __forceinline__ double issue_segment(const CollideArgs<double>& a, Wa
     void* dst = nullptr;
     uint32_t bytes = 0;
     uint32_t lead = 0;
-    T halo = T(0);
     bool in = true;       // the lane's source row lies inside the lattice
     bool bounce = false;  // the lane's halo element is bounced back at a z wall
     if (lane < Q) {
@@ -1011,7 +1010,7 @@ __device__ __forceinline__ double issue_segment(const CollideArgs<double>& a, Wa
             if (in) off = (size_t)opp(i) * N + (size_t)r;
         }
         if (ODD) {
-            const int c = MIS || in ? 0 : cz(i);
+            const int c = in ? 0 : cz(i);
             st.out[b][i] = a.fo + off + c;
             if (!PER) {
                 st.out[b][Q + i] = a.fo + slot;
@@ -1020,11 +1019,27 @@ __device__ __forceinline__ double issue_segment(const CollideArgs<double>& a, Wa
         }
         src = a.f + off + s.z0;
         dst = &st.f[b][i][V];
-        if (MIS) {
+        if (MIS && !ODD) {
             lead = (uint32_t)(((uintptr_t)src & 15u) / sizeof(T));
             src -= lead;
             bytes = (uint32_t)(((lead + (uint32_t)s.len + V - 1) / V) * 16u);
-        } else if (!ODD || PER || in || cz(i) == 0) {
+        } else if (MIS && (in || cz(i) == 0)) {
+            static_assert(V == 2, "a cut end is one element");
+            lead = (uint32_t)(((uintptr_t)src & 15u) / sizeof(T));
+            T* const cells = &st.f[b][i][V + lead];
+            const int rest = s.len - (int)lead;
+            if (lead) cp8(cells, src);
+            if (rest & 1) cp8(cells + s.len - 1, src + s.len - 1);
+            if (cz(i) != 0) {
+                const int e = cz(i) > 0 ? 0 : s.len - 1;   // the cell that reads the halo element
+                int zh = s.z0 + e - cz(i);
+                if (zh < 0 || zh >= g.nz) zh = g.per[2] ? (zh < 0 ? g.nz - 1 : 0) : -1;
+                cp8(cells + e - cz(i), zh >= 0 ? a.f + off + zh : a.f + slot + s.z0 + e);
+            }
+            src += lead;
+            dst = cells + lead;
+            bytes = (uint32_t)(rest / 2) * 16u;
+        } else if (!MIS && (!ODD || PER || in || cz(i) == 0)) {
             bytes = (uint32_t)(s.len * sizeof(T));
         }
     } else if (ODD && !MIS && lane < Q + 10) {
@@ -1077,39 +1092,19 @@ __device__ __forceinline__ double issue_segment(const CollideArgs<double>& a, Wa
         const uint32_t hi = __reduce_or_sync(FULL, ((lane >= 16 && lane < Q) ? lead << (2 * (lane - 16)) : 0u) |
                                                        ((STAGE_UP && lane >= Q + 10) ? lead2 << (8 + 2 * ud) : 0u));
         if (lane == 0) st.lead[b] = (unsigned long long)lo | ((unsigned long long)hi << 32);
-        if (ODD && lane < 10) {
-            const int i = zdir(lane);
-            const long long r = row_off(g, s, -cx(i), -cy(i));
-            if (r >= 0) {
-                if (cz(i) > 0) {
-                    const int zs = s.z0 > 0 ? s.z0 - 1 : (g.per[2] ? g.nz - 1 : -1);
-                    halo = zs >= 0 ? a.f[(size_t)opp(i) * N + (size_t)r + zs] : a.f[(size_t)i * N + (size_t)own];
-                } else {
-                    const int ze = s.z0 + s.len;
-                    const int zs = ze < g.nz ? ze : (g.per[2] ? 0 : -1);
-                    halo = zs >= 0 ? a.f[(size_t)opp(i) * N + (size_t)r + zs]
-                                   : a.f[(size_t)i * N + (size_t)own + g.nz - 1];
-                }
-            }
-        }
     }
     if constexpr (ODD && !PER) {
-        const unsigned rows = __ballot_sync(FULL, in);
-        if constexpr (MIS) {
-            if (lane == 0) st.geo[b][5] = (int)rows;
-        } else {
-            if (bounce) {
-                const int i = zdir(lane - Q);
-                if (cz(i) > 0) cp8(&st.f[b][i][V - 1], a.f + (size_t)i * N + (size_t)own);
-                else cp8(&st.f[b][i][V + s.len], a.f + (size_t)i * N + (size_t)own + (g.nz - 1));
-            }
-            for (unsigned m = ~rows & ZDIRS; m; m &= m - 1u) {
-                const int i = __ffs(m) - 1;
-                const T* p = a.f + (size_t)i * N + (size_t)own + s.z0;
-                for (int j = lane; j < s.len; j += 32) cp8(&st.f[b][i][V - cz(i) + j], p + j);
-            }
-            cp_arrive(&st.bar[b]);
+        if (bounce) {
+            const int i = zdir(lane - Q);
+            if (cz(i) > 0) cp8(&st.f[b][i][V - 1], a.f + (size_t)i * N + (size_t)own);
+            else cp8(&st.f[b][i][V + s.len], a.f + (size_t)i * N + (size_t)own + (g.nz - 1));
         }
+        for (unsigned m = ~__ballot_sync(FULL, in) & ZDIRS; m; m &= m - 1u) {
+            const int i = __ffs(m) - 1;
+            const T* p = a.f + (size_t)i * N + (size_t)own + s.z0;
+            for (int j = lane; j < s.len; j += 32) cp8(&st.f[b][i][V - cz(i) + j], p + j);
+        }
+        cp_arrive(&st.bar[b]);
     }
     const uint32_t total = __reduce_add_sync(FULL, bytes + bytes2);
     __syncwarp();   // the lanes' geometry writes come before lane 0's arrival
@@ -1117,7 +1112,6 @@ __device__ __forceinline__ double issue_segment(const CollideArgs<double>& a, Wa
     __syncwarp();
     if (bytes) bulk_g2s(dst, src, bytes, &st.bar[b]);
     if (bytes2) bulk_g2s(dst2, src2, bytes2, &st.bar[b]);
-    return halo;
 }
 
 // ---------------------------------------------------------------------------
@@ -1844,14 +1838,13 @@ struct StagedCell {
     size_t c;
     int zm, zp;           // z - 1 and z + 1 (wrapped; z itself beyond a wall)
     int tm, tp;           // and their part of the output rows: 0, Q at a wall, 2 Q wrapped
-    uint32_t rows;        // MIS: bit i: direction i's source row lies inside the lattice
     unsigned long long lead;
 
     __device__ __forceinline__ StagedCell(const CollideArgs<double>& a, WarpStage<double, STAGE_UP>& stage, int buf,
-                                          int j, int z0, uint32_t inside, unsigned long long leads)
+                                          int j, int z0, unsigned long long leads)
         : st(stage), base(&stage.f[buf][0][WarpStage<double>::V + j]), fo(a.fo), upf(a.up), N((unsigned)a.g.N), b(buf),
           z(z0 + j), c((size_t)stage.row[buf][row_slot(0, 0)] + (z0 + j)), zm(z - 1), zp(z + 1), tm(0), tp(0),
-          rows(inside), lead(leads) {
+          lead(leads) {
         const bool wrap = PER || a.g.per[2];
         if (z == 0) { zm = wrap ? a.g.nz - 1 : z; tm = wrap ? 2 * Q : Q; }
         if (z == a.g.nz - 1) { zp = wrap ? 0 : z; tp = wrap ? 2 * Q : Q; }
@@ -1859,7 +1852,7 @@ struct StagedCell {
     // the staged value of direction i (c_z = cz), the cell's own place in the stage
     __device__ __forceinline__ double* at(int i, int cz) const {
         int off = i * ROW;
-        if (ODD) off -= !MIS || ((rows >> i) & 1u) ? cz : 0;
+        if (ODD) off -= cz;
         if (MIS) off += (int)((lead >> (2 * i)) & 3u);
         return base + off;
     }
@@ -1872,7 +1865,6 @@ struct StagedCell {
     // phases the row that direction o was read from, one cell on in the odd phase
     __device__ __forceinline__ double* slot(int o, int cz) const {
         if (!ODD) return fo + c + (unsigned long long)(unsigned)o * N;
-        if (MIS && !((rows >> o) & 1u)) return st.out[b][o] + z;
         const int zd = pick(cz, zm, z, zp), t = PER ? 0 : pick(cz, tm, 0, tp);
         return st.out[b][o + t] + zd;
     }
@@ -1895,10 +1887,10 @@ __device__ __noinline__ void collide_cell_double(Cell s, double omega, double g0
 
 template <bool ODD, bool FORCE, bool PER, bool MIS, bool STAGE_UP>
 __device__ __forceinline__ void collide_cell_staged(const CollideArgs<double>& a, WarpStage<double, STAGE_UP>& st,
-                                                    int b, int j, int z0, uint32_t srcrow, unsigned long long lead,
+                                                    int b, int j, int z0, unsigned long long lead,
                                                     uint32_t w, bool solid, double (&F)[3]) {
     using fixed::i64;
-    const StagedCell<ODD, PER, MIS, STAGE_UP> s(a, st, b, j, z0, srcrow, lead);
+    const StagedCell<ODD, PER, MIS, STAGE_UP> s(a, st, b, j, z0, lead);
     // the cell's unit
     double* const p0 = s.at(0, 0);
     int e = __double2hiint(*p0) & 0x7ff00000;
@@ -1983,21 +1975,18 @@ k_collide_staged(const CollideArgs<T> a1, long long nseg, const CollideArgs<T>* 
     constexpr int SW = stage_warps<T>();
     constexpr int GROUPS = WARPS / SW;
     // a buffer's arrivals: the bytes of its bulk copies, and every lane's own copies
-    constexpr uint32_t ARRIVALS = sizeof(T) == 8 && ODD && !PER && !MIS ? 33 : 1;
+    constexpr uint32_t ARRIVALS = sizeof(T) == 8 && ODD && !PER ? 33 : 1;
     const int group = warp / SW, sub = warp % SW;
     WarpStage<T, STAGE_UP>& st = reinterpret_cast<WarpStage<T, STAGE_UP>*>(smem_raw)[group];
     __shared__ unsigned long long probe[WARPS];   // the test hook's barrier (never completes)
-    // a shared stage's barriers: buffer b left by both warps [b]; its halo elements in place [2 + b]
-    __shared__ unsigned long long shared_bar[SW > 1 ? GROUPS : 1][4];
+    // a shared stage's barriers: buffer b left by both warps
+    __shared__ unsigned long long shared_bar[SW > 1 ? GROUPS : 1][2];
     if (lane == 0) {
         if (sub == 0) {
             mbar_init(&st.bar[0], ARRIVALS);
             mbar_init(&st.bar[1], ARRIVALS);
             if (SW > 1)
-                for (int q = 0; q < 2; ++q) {
-                    mbar_init(&shared_bar[group][q], SW);
-                    mbar_init(&shared_bar[group][2 + q], 1);
-                }
+                for (int q = 0; q < 2; ++q) mbar_init(&shared_bar[group][q], SW);
         }
         mbar_init(&probe[warp], 1);
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
@@ -2021,10 +2010,9 @@ k_collide_staged(const CollideArgs<T> a1, long long nseg, const CollideArgs<T>* 
     const long long stride = (long long)gridDim.x * GROUPS;
     long long seg = (long long)blockIdx.x * GROUPS + group;
     if (seg >= nseg) return;   // both warps of a shared stage
-    auto issue = [&](int buf, long long sg) -> T {
+    auto issue = [&](int buf, long long sg) {
         if constexpr (LSU) {
             issue_segment_lsu<T, ODD, PER, STAGE_UP>(a1, st, buf, sg);
-            return T(0);
         } else if constexpr (BATCH) {
             int d, first;
             if (sseg0) {
@@ -2041,14 +2029,14 @@ k_collide_staged(const CollideArgs<T> a1, long long nseg, const CollideArgs<T>* 
                 first = __ldg(seg0 + d);
             }
             const CollideArgs<T>& A = dargs[d];
-            return issue_segment<ODD, PER, MIS, STAGE_UP>(A, st, buf, sg - first, d);
+            issue_segment<ODD, PER, MIS, STAGE_UP>(A, st, buf, sg - first, d);
+        } else {
+            issue_segment<ODD, PER, MIS, STAGE_UP>(a1, st, buf, sg, 0);
         }
-        else return issue_segment<ODD, PER, MIS, STAGE_UP>(a1, st, buf, sg, 0);
     };
     // segment k of the stage (buffer b = k & 1) is issued by warp k % SW, one segment
     // ahead; with two warps the same warp takes its first (solid) pass
-    T hcur = T(0);
-    if (sub == 0) hcur = issue(0, seg);
+    if (sub == 0) issue(0, seg);
     uint32_t phase = 0;   // bit b: parity expected next on buffer b
     uint32_t ephase = 0;  // the same for the barriers that hand a shared buffer back
     bool first = true;
@@ -2056,7 +2044,6 @@ k_collide_staged(const CollideArgs<T> a1, long long nseg, const CollideArgs<T>* 
     for (; seg < nseg; seg += stride, b ^= 1) {
         const long long next = seg + stride;
         const bool lead_warp = SW == 1 || sub == b;
-        T hnext = T(0);
         bool ok = true;
         if (next < nseg && (SW == 1 || !lead_warp)) {
             // both warps have left the buffer's last segment (none before the first two)
@@ -2064,7 +2051,7 @@ k_collide_staged(const CollideArgs<T> a1, long long nseg, const CollideArgs<T>* 
                 ok = mbar_wait(&shared_bar[group][b ^ 1], (ephase >> (b ^ 1)) & 1u);
                 ephase ^= 1u << (b ^ 1);
             }
-            if (SW == 1 || __all_sync(FULL, ok)) hnext = issue(b ^ 1, next);
+            if (SW == 1 || __all_sync(FULL, ok)) issue(b ^ 1, next);
         }
         if constexpr (LSU) {
             // this thread's copies of the current segment (all groups but the newest)
@@ -2097,17 +2084,6 @@ k_collide_staged(const CollideArgs<T> a1, long long nseg, const CollideArgs<T>* 
         const T* Fin = a.f;   // input populations
         const size_t own = ((size_t)sx * g.ny + sy) * g.nz;
         const unsigned long long lead = MIS ? st.lead[b] : 0ull;
-        if (MIS && ODD) {
-            if (lane < 10 && lead_warp) {
-                const int i = zdir(lane);
-                if (st.row[b][row_slot(-cx(i), -cy(i))] >= 0) {
-                    const int m = (int)((lead >> (2 * i)) & 3u);
-                    if (cz(i) > 0) st.f[b][i][V + m - 1] = hcur;
-                    else st.f[b][i][V + m + len] = hcur;
-                }
-            }
-            __syncwarp();
-        }
         // Odd phase with walls along z, aligned rows: the halo element of an edge
         // cell is its own slot i (half-way bounce-back).
         const uint32_t srcrow = ODD && !PER ? (uint32_t)st.geo[b][5] : 0u;   // bit i: direction i's source row is inside
@@ -2120,19 +2096,6 @@ k_collide_staged(const CollideArgs<T> a1, long long nseg, const CollideArgs<T>* 
                 }
             }
             __syncwarp();
-        }
-        if constexpr (SW > 1 && ODD && MIS) {
-            // the other warp's cells read the halo elements that the lead warp put in place
-            if (lead_warp) {
-                if (lane == 0) mbar_arrive(&shared_bar[group][2 + b]);
-            } else {
-                ok = mbar_wait(&shared_bar[group][2 + b], (phase >> b & 1u) ^ 1u);   // phase was flipped above
-            }
-            if (__any_sync(FULL, !ok)) {
-                if (lane == 0) atomicOr(BATCH ? dargs[0].err : a1.err, 0x20u);   // LBDEM_DEVERR_TIMEOUT
-                if (next < nseg) mbar_wait(&st.bar[b ^ 1], (phase >> (b ^ 1)) & 1u);
-                return;
-            }
         }
         if constexpr (sizeof(T) == 4) {
             static_assert(LSU, "FP32: aligned rows of a single lattice (others: k_collide_direct)");
@@ -2163,7 +2126,7 @@ k_collide_staged(const CollideArgs<T> a1, long long nseg, const CollideArgs<T>* 
             if (j >= 0) {
                 const uint32_t w = st.vox[b][vlead + j];
                 T Fc[3];
-                collide_cell_staged<ODD, FORCE, PER, MIS, STAGE_UP>(a, st, b, j, z0, srcrow, lead, w, any_solid, Fc);
+                collide_cell_staged<ODD, FORCE, PER, MIS, STAGE_UP>(a, st, b, j, z0, lead, w, any_solid, Fc);
                 // (the segment's data are read again: kept over the update they would spill)
                 if (a.cf) {
                     const size_t c = (size_t)st.row[b][row_slot(0, 0)] + st.geo[b][2] + j;
@@ -2182,7 +2145,6 @@ k_collide_staged(const CollideArgs<T> a1, long long nseg, const CollideArgs<T>* 
         if constexpr (!LSU) asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
         __syncwarp();
         if (SW > 1 && lane == 0) mbar_arrive(&shared_bar[group][b]);
-        hcur = hnext;
     }
 }
 
