@@ -219,9 +219,6 @@ __device__ __forceinline__ void collide_cell(double (&f)[Q], double omega, doubl
 // n = 125 gives B = 1 (no BGK, alpha = 1), n = 0 gives B = 0 (the BGK result).
 // The moments are those of fPre: without a body force BGK conserves them, and the
 // reference's post-collision recomputation (:146-148) differs by rounding only.
-// SOLID false (a warp without solid cells) leaves out the solid terms; a fluid
-// cell gets the same bits either way, so results do not depend on which cells
-// share a warp.
 template <int AX>
 __device__ __forceinline__ double pair_sum(const double (&d)[9]) {
     // sum_k c_k[AX] d[k - 10] over the directions k = 10..18 with c_k[AX] != 0, in k order
@@ -238,7 +235,6 @@ __device__ __forceinline__ double pair_sum(const double (&d)[9]) {
     return r;
 }
 
-template <bool SOLID>
 __device__ __forceinline__ void collide_cell_fp64(double (&f)[Q], double omega, double B, double up0, double up1,
                                                   double up2, double& Fx, double& Fy, double& Fz) {
     double d[9];
@@ -257,18 +253,15 @@ __device__ __forceinline__ void collide_cell_fp64(double (&f)[Q], double omega, 
     const double jSqr = fma(jz, jz, fma(jy, jy, jx * jx));
     const double m15 = -1.5 * invRho;
     const double base = fma(m15, jSqr, rhoBar);
-    double Px = 0.0, Py = 0.0, Pz = 0.0, dd = 0.0, alpha = omega, om1B = omega;
-    if (SOLID) {
-        const double rho = 1.0 + rhoBar;
-        Px = up0 * rho; Py = up1 * rho; Pz = up2 * rho;
-        const double PSqr = fma(Pz, Pz, fma(Py, Py, Px * Px));
-        dd = m15 * (jSqr - PSqr);
-        alpha = fma(B, 1.0 - omega, omega);
-        om1B = omega * (1.0 - B);
-    }
+    const double rho = 1.0 + rhoBar;
+    const double Px = up0 * rho, Py = up1 * rho, Pz = up2 * rho;
+    const double PSqr = fma(Pz, Pz, fma(Py, Py, Px * Px));
+    const double dd = m15 * (jSqr - PSqr);
+    const double alpha = fma(B, 1.0 - omega, omega);
+    const double om1B = omega * (1.0 - B);
     {
         const double g0 = f[0] - wt(0) * base;
-        f[0] = SOLID ? fma(B, wt(0) * dd, fma(-om1B, g0, f[0])) : fma(-omega, g0, f[0]);
+        f[0] = fma(B, wt(0) * dd, fma(-om1B, g0, f[0]));
     }
     double Ex = 0.0, Ey = 0.0, Ez = 0.0;
     bool fx0 = false, fy0 = false, fz0 = false;
@@ -282,26 +275,21 @@ __device__ __forceinline__ void collide_cell_fp64(double (&f)[Q], double omega, 
         const double Lj = t3 * cj;
         const double gi = (f[i] - C) + Lj;
         const double gk = (f[k] - C) - Lj;
-        if (SOLID) {
-            const double cP = cdot(k, Px, Py, Pz);
-            const double m = cj - cP, p = cj + cP;
-            const double Qd = fma(a45 * m, p, t * dd);
-            const double L = t3 * m;
-            const double e = d[i - 1] - t3 * p;
-            f[i] = fma(B, (gk - Qd) + L, fma(-alpha, gi, f[i]));
-            f[k] = fma(B, (gi - Qd) - L, fma(-alpha, gk, f[k]));
-            if (cx(k) != 0) { Ex = fx0 ? (cx(k) > 0 ? Ex + e : Ex - e) : (cx(k) > 0 ? e : -e); fx0 = true; }
-            if (cy(k) != 0) { Ey = fy0 ? (cy(k) > 0 ? Ey + e : Ey - e) : (cy(k) > 0 ? e : -e); fy0 = true; }
-            if (cz(k) != 0) { Ez = fz0 ? (cz(k) > 0 ? Ez + e : Ez - e) : (cz(k) > 0 ? e : -e); fz0 = true; }
-        } else {
-            f[i] = fma(-omega, gi, f[i]);
-            f[k] = fma(-omega, gk, f[k]);
-        }
+        const double cP = cdot(k, Px, Py, Pz);
+        const double m = cj - cP, p = cj + cP;
+        const double Qd = fma(a45 * m, p, t * dd);
+        const double L = t3 * m;
+        const double e = d[i - 1] - t3 * p;
+        f[i] = fma(B, (gk - Qd) + L, fma(-alpha, gi, f[i]));
+        f[k] = fma(B, (gi - Qd) - L, fma(-alpha, gk, f[k]));
+        if (cx(k) != 0) { Ex = fx0 ? (cx(k) > 0 ? Ex + e : Ex - e) : (cx(k) > 0 ? e : -e); fx0 = true; }
+        if (cy(k) != 0) { Ey = fy0 ? (cy(k) > 0 ? Ey + e : Ey - e) : (cy(k) > 0 ? e : -e); fy0 = true; }
+        if (cz(k) != 0) { Ez = fz0 ? (cz(k) > 0 ? Ez + e : Ez - e) : (cz(k) > 0 ? e : -e); fz0 = true; }
     }
     const double B2 = B + B;
-    Fx = SOLID ? B2 * Ex : 0.0;
-    Fy = SOLID ? B2 * Ey : 0.0;
-    Fz = SOLID ? B2 * Ez : 0.0;
+    Fx = B2 * Ex;
+    Fy = B2 * Ey;
+    Fz = B2 * Ez;
 }
 
 // Per-cell force and torque added to the particle's sums (FP64 form): six
@@ -1879,7 +1867,7 @@ __device__ __noinline__ void collide_cell_double(Cell s, double omega, double g0
 #pragma unroll
     for (int i = 0; i < Q; ++i) f[i] = *s.at(i, cz(i));
     if constexpr (FORCE) collide_cell(f, omega, g0, g1, g2, n, B, u0, u1, u2, [&](int i) { return *s.at(i, cz(i)); }, F);
-    else collide_cell_fp64<true>(f, omega, B, u0, u1, u2, F[0], F[1], F[2]);
+    else collide_cell_fp64(f, omega, B, u0, u1, u2, F[0], F[1], F[2]);
     s.fo[s.c] = f[0];
 #pragma unroll
     for (int i = 1; i < Q; ++i) *s.slot(opp(i), cz(i)) = f[i];
