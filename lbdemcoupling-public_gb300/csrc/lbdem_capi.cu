@@ -66,10 +66,13 @@ struct lbdem_handle {
     // particle records [cap][12] and tag map [max_tag + 1], two of each: a new list goes
     // into the other pair, and its prepare launch clears the entries of the list before it
     // in that list's map, so no memset of the whole map stands before a voxelization.
-    // The map not in use is clear.
+    // The map not in use is clear.  A graph keeps the addresses it was captured with, so
+    // from the first captured list or step on the handle stays with its current pair and
+    // clears the whole map before every list.
     double* rec2[2] = {nullptr, nullptr};
     int* map2[2] = {nullptr, nullptr};
     int cur = 0;
+    bool one_pair = false;      // a list or a step has been captured
     double* d_rec = nullptr;    // rec2[cur]
     SphereDev* d_sph = nullptr; // [cap]
     SphereFast* d_fast = nullptr; // [cap]
@@ -205,6 +208,16 @@ lbdem_status wait_staging(lbdem_handle* h) {
     return LBDEM_OK;
 }
 
+// To be called before a launch that takes the handle's records or tag map: under stream
+// capture their addresses are kept for good.
+lbdem_status note_capture(lbdem_handle* h) {
+    if (h->one_pair) return LBDEM_OK;
+    cudaStreamCaptureStatus capturing = cudaStreamCaptureStatusNone;
+    CK(h, cudaStreamIsCapturing(h->stream, &capturing));
+    h->one_pair = capturing != cudaStreamCaptureStatusNone;
+    return LBDEM_OK;
+}
+
 // Voxelization of n records read from src (the pinned staging table, or a device table of
 // the caller) by the prepare launch, which copies them into the handle's table.
 lbdem_status voxelize(lbdem_handle* h, int n, int init_vel, const double* src) {
@@ -220,12 +233,11 @@ lbdem_status voxelize(lbdem_handle* h, int n, int init_vel, const double* src) {
         CK(h, launch_owner_velocity(h->vox, h->d_tag2slot, h->cfg.max_tag, h->n_cur, h->d_xpf, h->g, up_before, s));
         h->launches += 1;
     }
-    // A call that is captured into a graph runs again with the same buffers and an unknown
-    // list before it, so it keeps the current pair and clears the whole map; so does an
-    // empty list, which has no prepare launch.
-    cudaStreamCaptureStatus capturing = cudaStreamCaptureStatusNone;
-    CK(h, cudaStreamIsCapturing(s, &capturing));
-    const bool whole = n <= 0 || capturing != cudaStreamCaptureStatusNone;
+    // With one pair the list before is unknown (a replay may have left another one), so the
+    // whole map is cleared; so it is for an empty list, which has no prepare launch.
+    const lbdem_status cap = note_capture(h);
+    if (cap != LBDEM_OK) return cap;
+    const bool whole = n <= 0 || h->one_pair;
     if (whole) CK(h, cudaMemsetAsync(h->d_tag2slot, 0x7F, sizeof(int) * ((size_t)h->cfg.max_tag + 1), s));
     if (n > 0) {
         int* const old_map = whole ? nullptr : h->d_tag2slot;
@@ -601,6 +613,8 @@ lbdem_status lbdem_set_particles_device(lbdem_handle* h, int32_t n, const double
 lbdem_status lbdem_collide_and_stream(lbdem_handle* h) {
     if (!h) return LBDEM_ERR_INVALID_ARG;
     DeviceGuard dg(h->device);
+    const lbdem_status cap = note_capture(h);
+    if (cap != LBDEM_OK) return cap;
     const int n = h->n_cur;
     // the sums start from zero: the voxelization of this list zeroed them unless
     // a step has run since
