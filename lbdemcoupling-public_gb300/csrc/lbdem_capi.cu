@@ -1045,24 +1045,32 @@ lbdem_status lbdem_adjoint_window(lbdem_handle* h, int32_t nsteps, int32_t K, in
     CK(h, cudaMemsetAsync(tape + (size_t)K * pop, 0, ALLOC_TAIL, s));
     const int64_t step0 = h->step;
     lbdem_status st;
-    // A step whose particle table equals the one voxelized last needs no new
-    // voxelization: with positions fixed the update is idempotent (every cell's
-    // owner re-sets itself, no other sphere can displace it), so the voxel
-    // words, surface velocities and tag map are already those of the step.
+    // The window's first two steps are voxelized.  The first pass over new places can leave a
+    // shared cell with its owner of before (as long as that sphere held more of the cell than
+    // the others do now), whose own count it then lowers, so that the cell changes hands in
+    // the second.  After two passes no further one changes a word: every owner then holds its
+    // own count, no sphere has a larger one, and equal counts do not displace it.  From the
+    // third step on, and in the recomputation, a step whose table is the one voxelized last
+    // needs nothing.
     int vox_t = -1;   // step whose table the voxel state holds
+    int passes = 0;   // voxelizations of the window
     auto same_table = [&](int a, int b) {
         return a >= 0 && b >= 0 &&
                std::memcmp(rec + (size_t)a * n * REC_STRIDE, rec + (size_t)b * n * REC_STRIDE,
                            (size_t)n * REC_STRIDE * sizeof(double)) == 0;
     };
     auto voxelize_for = [&](int t) -> lbdem_status {
-        if (same_table(vox_t, t)) return LBDEM_OK;
+        const bool settled = passes >= std::min(nsteps, 2);
+        if (settled && same_table(vox_t, t)) return LBDEM_OK;
         const double* src = d_recs + (size_t)t * n * REC_STRIDE;
-        // the FP32 form keeps no surface-velocity field, so a step whose positions are those
-        // of the voxelized list only needs its tables (velocities) renewed
-        const lbdem_status r = vox_t >= 0 && h->prec == LBDEM_PREC_FP32_DEV ? renew_tables(h, n, src)
-                                                                            : lbdem_set_particles_device(h, n, src, 0);
-        if (r == LBDEM_OK) vox_t = t;
+        // the FP32 form keeps no surface-velocity field, so other velocities only need the
+        // tables renewed
+        const bool tables = settled && h->prec == LBDEM_PREC_FP32_DEV;
+        const lbdem_status r = tables ? renew_tables(h, n, src) : lbdem_set_particles_device(h, n, src, 0);
+        if (r == LBDEM_OK) {
+            vox_t = t;
+            if (!tables) ++passes;
+        }
         return r;
     };
 
