@@ -723,7 +723,8 @@ __device__ __forceinline__ void reduce_forces(const CollideArgs<T>& a, int key, 
 // velocity already looked up).  Every cell of a
 // particle lies within its radius of the particle's nearest image, so along a
 // row the minimum-image arm of cell z is arm(zc) + (z - zc) e_z for any point
-// zc of the segment, and
+// zc of the segment (where the cells' nearest images differ, images_differ(), the arms are
+// taken per cell), and
 //   sum_cells arm x F = arm(zc) x sum F + sum (z - zc) e_z x F,
 // with e_z x F = (-F_y, F_x, 0).  Per cell the kernel accumulates
 // v = (F, -(z - zc) F_y, (z - zc) F_x); the lane that ends a run (the last
@@ -1384,6 +1385,46 @@ __device__ __forceinline__ void forces_by_run(const CollideArgs<float>& a, const
         reduce_runs(a, second ? kb : ka, v, second ? zb : za, x, second ? yb : ya, zc, o.rh, o.rl0, o.rl1, o.vslot);
     }
 }
+// Whether a segment of len cells can hold cells of one particle whose arms take the minimum
+// image (integer half extent) differently: across the periodic boundary the two ends of a
+// chord are nz less the chord apart, so there are solid cells that far apart, and between
+// walls an arm has to exceed half the row.  s: an owner slot of the lane (-1: none), whose
+// cells are j = 2 l, 2 l + 1 (ADJ) or l, l + 32.  Must be reached by all 32 lanes.
+// (Registers, launch constants and two votes only: a load from the batch's table here took
+// 1 % of the time of 512 channels.)
+template <bool ADJ>
+__device__ __forceinline__ bool images_can_differ(const Geom& g, int reach, int len, int s) {
+    const int j = ADJ ? 2 * (threadIdx.x & 31) : threadIdx.x & 31;
+    const int apart = g.per[2] ? g.nz - 2 * reach : (g.nz / 2 < reach ? 0 : len);
+    return len > apart && __any_sync(FULL, s >= 0 && j < len - apart) &&
+           __any_sync(FULL, s >= 0 && j >= apart - (ADJ ? 1 : 32));
+}
+// Whether they do.  Out of line; must be reached by all 32 lanes.
+__device__ __noinline__ bool images_differ(const CollideArgs<float>& a, int s0, int s1, int vslot, float zh, float zl,
+                                           int za, int zb) {
+    const float half = (float)(a.g.nz / 2);
+    auto image = [&](int slot, int z) -> int {
+        if (slot < 0) return 0;
+        float h = zh, l = zl;   // the centre's z in the row that the velocity lookup read
+        if (slot != vslot) {
+            const float* p = a.xpf + (size_t)slot * XPF_STRIDE;
+            h = __ldg(p + 2);
+            l = __ldg(p + 5);
+        }
+        const float d = ((float)z - h) - l;
+        return d > half ? 1 : (d < -half ? -1 : 0);
+    };
+    const int i0 = image(s0, za), i1 = image(s1, zb);
+    unsigned m0 = __ballot_sync(FULL, i0 != 0), m1 = __ballot_sync(FULL, i1 != 0);
+    while (m0 | m1) {   // one particle at a time: its cells have the image of its first one
+        const int lead = __ffs(m0 ? m0 : m1) - 1;
+        const int slot = __shfl_sync(FULL, m0 ? s0 : s1, lead), first = __shfl_sync(FULL, m0 ? i0 : i1, lead);
+        if (__any_sync(FULL, (s0 == slot && i0 != first) || (s1 == slot && i1 != first))) return true;
+        m0 &= ~__ballot_sync(FULL, s0 == slot);
+        m1 &= ~__ballot_sync(FULL, s1 == slot);
+    }
+    return false;
+}
 // forces_by_cell out of line, for the rare segments of the row kernels.
 __device__ __noinline__ void forces_by_cell_far(const CollideArgs<float>& a, PairForce o, int x, int ya, int za,
                                                 int yb, int zb, bool apart) {
@@ -1539,9 +1580,11 @@ __device__ __forceinline__ void collide_segment_pairs(const CollideArgs<float>& 
         if (v0) { a.cf[ca] = fx.x; a.cf[N + ca] = fy.x; a.cf[2 * N + ca] = fz.x; }
         if (v1) { a.cf[cb] = fx.y; a.cf[N + cb] = fy.y; a.cf[2 * N + cb] = fz.y; }
     }
-    if ((PER || g.per[2]) && len == g.nz) {
-        // the segment is a whole z-periodic row: a particle's chord may wrap
-        // around inside it, so the arms are taken per cell
+    if (((PER || g.per[2]) && len == g.nz) ||
+        (images_can_differ<true>(g, a.reach, len, max(s0, s1)) &&
+         images_differ(a, s0, s1, vslot, vrh.z, vrl1, za, zb))) {
+        // the segment is a whole z-periodic row, or holds both ends of a chord that wraps
+        // around: the arms are taken per cell
         forces_by_cell_far(a, PairForce{Fx, Fy, Fz, s0, s1, vslot, (n0 > 0 && s0 < 0) || (n1 > 0 && s1 < 0), vrh, vrl0, vrl1},
                            sx, sy, za, sy, zb, false);
         return;
@@ -1796,9 +1839,11 @@ k_collide_direct(const CollideArgs<float> a1, long long nseg, const CollideArgs<
         }
         if (PLANE) {
             forces_by_cell(a, g, o, x, c[0].y, c[0].z, c[1].y, c[1].z, false);
-        } else if (g.per[2] && g.nz <= SEGW) {
-            // the segment is a whole z-periodic row: a particle's chord may wrap around inside
-            // it, so the arms are taken per cell
+        } else if ((g.per[2] && g.nz <= SEGW) ||
+                   (images_can_differ<false>(g, a1.reach, min(g.nz - z0, SEGW), max(o.s0, o.s1)) &&
+                    images_differ(a, o.s0, o.s1, o.vslot, o.rh.z, o.rl1, z0 + lane, z0 + lane + hz))) {
+            // the segment is a whole z-periodic row, or holds both ends of a chord that wraps
+            // around: the arms are taken per cell
             forces_by_cell_far(a, o, x, y, z0 + lane, c[1].y, z0 + lane + hz, two);
         } else {
             forces_by_run(a, o, x, y, c[1].y, z0 + SEGW / 2, z0 + lane, z0 + lane + hz, two);
@@ -2221,9 +2266,10 @@ cudaError_t launch_one(const CollideArgs<T>& args, cudaStream_t s) {
 }
 
 template <typename T, bool ODD, bool FORCE>
-cudaError_t launch_batch(const CollideArgs<T>* dargs, const int* seg0, int ndom, long long nseg, int blocks_per_sm,
-                         cudaStream_t s) {
+cudaError_t launch_batch(const CollideArgs<T>* dargs, const int* seg0, int ndom, long long nseg, short reach,
+                         int blocks_per_sm, cudaStream_t s) {
     CollideArgs<T> none{};
+    none.reach = reach;
     if constexpr (sizeof(T) == 4) return launch_direct<ODD, FORCE, true>(none, nseg, dargs, seg0, ndom, blocks_per_sm, s);
     else return launch_staged<T, ODD, FORCE, false, true, true>(none, nseg, dargs, seg0, ndom, blocks_per_sm, s);
 }
@@ -2237,20 +2283,20 @@ cudaError_t launch_collide_stream(const CollideArgs<T>& a, bool odd, bool force,
 }
 
 template <typename T>
-cudaError_t launch_collide_batch(const CollideArgs<T>* dargs, const int* seg0, int ndom, long long nseg, bool odd,
-                                 bool force, int blocks_per_sm, cudaStream_t s) {
+cudaError_t launch_collide_batch(const CollideArgs<T>* dargs, const int* seg0, int ndom, long long nseg, short reach,
+                                 bool odd, bool force, int blocks_per_sm, cudaStream_t s) {
     if (odd)
-        return force ? launch_batch<T, true, true>(dargs, seg0, ndom, nseg, blocks_per_sm, s)
-                     : launch_batch<T, true, false>(dargs, seg0, ndom, nseg, blocks_per_sm, s);
-    return force ? launch_batch<T, false, true>(dargs, seg0, ndom, nseg, blocks_per_sm, s)
-                 : launch_batch<T, false, false>(dargs, seg0, ndom, nseg, blocks_per_sm, s);
+        return force ? launch_batch<T, true, true>(dargs, seg0, ndom, nseg, reach, blocks_per_sm, s)
+                     : launch_batch<T, true, false>(dargs, seg0, ndom, nseg, reach, blocks_per_sm, s);
+    return force ? launch_batch<T, false, true>(dargs, seg0, ndom, nseg, reach, blocks_per_sm, s)
+                 : launch_batch<T, false, false>(dargs, seg0, ndom, nseg, reach, blocks_per_sm, s);
 }
 
 template cudaError_t launch_collide_stream<float>(const CollideArgs<float>&, bool, bool, cudaStream_t);
 template cudaError_t launch_collide_stream<double>(const CollideArgs<double>&, bool, bool, cudaStream_t);
-template cudaError_t launch_collide_batch<float>(const CollideArgs<float>*, const int*, int, long long, bool, bool,
+template cudaError_t launch_collide_batch<float>(const CollideArgs<float>*, const int*, int, long long, short, bool, bool,
                                                  int, cudaStream_t);
-template cudaError_t launch_collide_batch<double>(const CollideArgs<double>*, const int*, int, long long, bool, bool,
+template cudaError_t launch_collide_batch<double>(const CollideArgs<double>*, const int*, int, long long, short, bool, bool,
                                                   int, cudaStream_t);
 
 }  // namespace lbdem

@@ -250,14 +250,15 @@ bool any_force(const lbdem_batch* b) {
 // dargs: the [2][ndom] table of fill_dargs on the device.
 cudaError_t launch_k1(lbdem_batch* b, const void* dargs, bool odd, int bps) {
     const bool force = any_force(b);
+    const short reach = reach_of(b->cfg.max_radius);
     if (b->prec == LBDEM_PREC_FP64)
-        return launch_collide_batch<double>((const CollideArgs<double>*)dargs, b->d_seg0, b->ndom, b->nseg, odd,
-                                            force, bps, b->stream);
+        return launch_collide_batch<double>((const CollideArgs<double>*)dargs, b->d_seg0, b->ndom, b->nseg, reach,
+                                            odd, force, bps, b->stream);
     if (!odd)   // plane segments
         return launch_collide_batch<float>((const CollideArgs<float>*)dargs + b->ndom, b->d_seg0 + b->ndom, b->ndom,
-                                           b->nseg_plane, false, force, bps, b->stream);
-    return launch_collide_batch<float>((const CollideArgs<float>*)dargs, b->d_seg0, b->ndom, b->nseg, true, force,
-                                       bps, b->stream);
+                                           b->nseg_plane, reach, false, force, bps, b->stream);
+    return launch_collide_batch<float>((const CollideArgs<float>*)dargs, b->d_seg0, b->ndom, b->nseg, reach, true,
+                                       force, bps, b->stream);
 }
 
 cudaError_t launch_planes(lbdem_batch* b, int phase, int rescale, const double* avg_in, double* avg_out) {

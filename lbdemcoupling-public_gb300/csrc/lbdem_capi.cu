@@ -353,6 +353,7 @@ cudaError_t k1_launch(lbdem_handle* h, void* fin, void* fout) {
     a.cf = (float*)h->cf; a.tag2slot = h->d_tag2slot; a.rec = h->d_rec; a.xpf = h->d_xpf; a.nslot = n;
     a.max_tag = h->cfg.max_tag; a.ft = h->d_ft; a.err = h->d_err; a.btab = h->btabf; a.omega = (float)h->cfg.omega;
     a.probe_timeout = (h->cfg.flags & LBDEM_FLAG_PROBE_TIMEOUT) ? 1 : 0;
+    a.reach = reach_of(h->cfg.max_radius);
     for (int d = 0; d < 3; ++d) a.g3[d] = (float)h->cfg.body_force[d];
     return launch_collide_stream<float>(a, odd, force, h->stream);
 }

@@ -149,13 +149,17 @@ struct CollideArgs {
     T omega;                 // BGK relaxation frequency
     T g3[3];                 // Guo body-force acceleration
     DivMagic dz, dy;         // division by the z-segments per row and by ny (set by the launchers)
-    int probe_timeout;       // test hook: the first wait of every warp runs out (LBDEM_FLAG_PROBE_TIMEOUT)
+    short probe_timeout;     // test hook: the first wait of every warp runs out (LBDEM_FLAG_PROBE_TIMEOUT)
+    short reach;             // bound of the distance of a particle's cells from its centre, reach_of()
     // Plane view (FP32 batch, even phase): g describes the domain as nx rows of
     // ny nz cells, so that 64-cell segments run across the z-rows of an x-plane;
     // flat_ny, flat_nz are the true extents and dnz divides by flat_nz.  0: no view.
     int flat_ny, flat_nz;
     DivMagic dnz;
 };
+
+// A cell that a sphere covers lies within max_radius + 1 of the centre (max_radius <= 1024).
+inline short reach_of(double max_radius) { return (short)((int)max_radius + 2); }
 
 // FP32 batch, odd phase: rows whose last segment holds at most half a segment are taken in
 // pairs (y, y + 1): the full segments of each, then one segment of both tails, a lane's
@@ -308,8 +312,8 @@ cudaError_t launch_collide_stream(const CollideArgs<T>& a, bool odd, bool force,
 // The FP32 even phase takes plane views (CollideArgs::flat_nz != 0: rows of
 // ny nz cells, one per x-plane) with their own seg0 and nseg.
 template <typename T>
-cudaError_t launch_collide_batch(const CollideArgs<T>* dargs, const int* seg0, int ndom, long long nseg, bool odd,
-                                 bool force, int blocks_per_sm, cudaStream_t s);
+cudaError_t launch_collide_batch(const CollideArgs<T>* dargs, const int* seg0, int ndom, long long nseg, short reach,
+                                 bool odd, bool force, int blocks_per_sm, cudaStream_t s);
 
 // Sphere tables (sph, fast, xpf), the tag -> lowest slot map (tag2slot must
 // hold "no slot" on entry) and the tile bins, in one launch.  tile_cnt must be
