@@ -219,6 +219,9 @@ __device__ __forceinline__ void collide_cell(double (&f)[Q], double omega, doubl
 // n = 125 gives B = 1 (no BGK, alpha = 1), n = 0 gives B = 0 (the BGK result).
 // The moments are those of fPre: without a body force BGK conserves them, and the
 // reference's post-collision recomputation (:146-148) differs by rounding only.
+// SOLID false (a warp without solid cells) leaves out the solid terms, 150 double operations
+// instead of 270; a fluid cell gets the same bits either way, so results do not depend on
+// which cells share a warp.
 template <int AX>
 __device__ __forceinline__ double pair_sum(const double (&d)[9]) {
     // sum_k c_k[AX] d[k - 10] over the directions k = 10..18 with c_k[AX] != 0, in k order
@@ -235,6 +238,7 @@ __device__ __forceinline__ double pair_sum(const double (&d)[9]) {
     return r;
 }
 
+template <bool SOLID>
 __device__ __forceinline__ void collide_cell_fp64(double (&f)[Q], double omega, double B, double up0, double up1,
                                                   double up2, double& Fx, double& Fy, double& Fz) {
     double d[9];
@@ -253,15 +257,18 @@ __device__ __forceinline__ void collide_cell_fp64(double (&f)[Q], double omega, 
     const double jSqr = fma(jz, jz, fma(jy, jy, jx * jx));
     const double m15 = -1.5 * invRho;
     const double base = fma(m15, jSqr, rhoBar);
-    const double rho = 1.0 + rhoBar;
-    const double Px = up0 * rho, Py = up1 * rho, Pz = up2 * rho;
-    const double PSqr = fma(Pz, Pz, fma(Py, Py, Px * Px));
-    const double dd = m15 * (jSqr - PSqr);
-    const double alpha = fma(B, 1.0 - omega, omega);
-    const double om1B = omega * (1.0 - B);
+    double Px = 0.0, Py = 0.0, Pz = 0.0, dd = 0.0, alpha = omega, om1B = omega;
+    if (SOLID) {
+        const double rho = 1.0 + rhoBar;
+        Px = up0 * rho; Py = up1 * rho; Pz = up2 * rho;
+        const double PSqr = fma(Pz, Pz, fma(Py, Py, Px * Px));
+        dd = m15 * (jSqr - PSqr);
+        alpha = fma(B, 1.0 - omega, omega);
+        om1B = omega * (1.0 - B);
+    }
     {
         const double g0 = f[0] - wt(0) * base;
-        f[0] = fma(B, wt(0) * dd, fma(-om1B, g0, f[0]));
+        f[0] = SOLID ? fma(B, wt(0) * dd, fma(-om1B, g0, f[0])) : fma(-omega, g0, f[0]);
     }
     double Ex = 0.0, Ey = 0.0, Ez = 0.0;
     bool fx0 = false, fy0 = false, fz0 = false;
@@ -275,6 +282,11 @@ __device__ __forceinline__ void collide_cell_fp64(double (&f)[Q], double omega, 
         const double Lj = t3 * cj;
         const double gi = (f[i] - C) + Lj;
         const double gk = (f[k] - C) - Lj;
+        if (!SOLID) {
+            f[i] = fma(-omega, gi, f[i]);
+            f[k] = fma(-omega, gk, f[k]);
+            continue;
+        }
         const double cP = cdot(k, Px, Py, Pz);
         const double m = cj - cP, p = cj + cP;
         const double Qd = fma(a45 * m, p, t * dd);
@@ -287,9 +299,9 @@ __device__ __forceinline__ void collide_cell_fp64(double (&f)[Q], double omega, 
         if (cz(k) != 0) { Ez = fz0 ? (cz(k) > 0 ? Ez + e : Ez - e) : (cz(k) > 0 ? e : -e); fz0 = true; }
     }
     const double B2 = B + B;
-    Fx = B2 * Ex;
-    Fy = B2 * Ey;
-    Fz = B2 * Ez;
+    Fx = SOLID ? B2 * Ex : 0.0;
+    Fy = SOLID ? B2 * Ey : 0.0;
+    Fz = SOLID ? B2 * Ez : 0.0;
 }
 
 // Per-cell force and torque added to the particle's sums (FP64 form): six
@@ -1903,8 +1915,9 @@ struct StagedCell {
     }
 };
 
-// The double routine for a cell outside the fixed-point range, out of line.
-template <bool FORCE, typename Cell>
+// The double routine for a cell outside the fixed-point range, out of line.  SOLID false: for
+// the lanes of a warp without solid cells.
+template <bool FORCE, bool SOLID, typename Cell>
 __device__ __noinline__ void collide_cell_double(Cell s, double omega, double g0,
                                                  double g1, double g2, int n, double B, double u0, double u1,
                                                  double u2, double (&F)[3]) {
@@ -1912,7 +1925,7 @@ __device__ __noinline__ void collide_cell_double(Cell s, double omega, double g0
 #pragma unroll
     for (int i = 0; i < Q; ++i) f[i] = *s.at(i, cz(i));
     if constexpr (FORCE) collide_cell(f, omega, g0, g1, g2, n, B, u0, u1, u2, [&](int i) { return *s.at(i, cz(i)); }, F);
-    else collide_cell_fp64(f, omega, B, u0, u1, u2, F[0], F[1], F[2]);
+    else collide_cell_fp64<SOLID>(f, omega, B, u0, u1, u2, F[0], F[1], F[2]);
     s.fo[s.c] = f[0];
 #pragma unroll
     for (int i = 1; i < Q; ++i) *s.slot(opp(i), cz(i)) = f[i];
@@ -1941,7 +1954,8 @@ __device__ __forceinline__ void collide_cell_staged(const CollideArgs<double>& a
     }
     if (FORCE) e = fixed::cell_exponent_up(e, a.g3[0], a.g3[1], a.g3[2]);
     if (!fixed::fits(e)) {
-        collide_cell_double<FORCE>(s, a.omega, a.g3[0], a.g3[1], a.g3[2], n, B, u0, u1, u2, F);
+        if (FORCE || solid) collide_cell_double<FORCE, true>(s, a.omega, a.g3[0], a.g3[1], a.g3[2], n, B, u0, u1, u2, F);
+        else collide_cell_double<FORCE, FORCE>(s, a.omega, 0.0, 0.0, 0.0, 0, 0.0, 0.0, 0.0, 0.0, F);
         return;
     }
     e = max(e, fixed::EMAX_LO);
