@@ -332,10 +332,16 @@ lbdem_status lbdem_voxelize_static(int32_t nx, int32_t ny, int32_t nz, int32_t p
  *   grad_f0    optional out [19][N] of the lattice type, natural order: dL/d
  *              populations before the window
  * On return the handle holds the state after the window and the forces of its
- * last step.  Not available with a pressure drop set (not differentiated). */
+ * last step.  Not available with a pressure drop set (not differentiated).
+ * The window's device memory (checkpoints, tape, adjoint populations) stays with
+ * the handle for its next window, at most 4 GB over all handles; it is given
+ * back when an allocation of this library on the device would fail without it,
+ * by lbdem_adjoint_release, and with the handle. */
 lbdem_status lbdem_adjoint_window(lbdem_handle* h, int32_t nsteps, int32_t checkpoint_every, int32_t n,
                                   const double* rec, const double* weights, double* loss, double* grad_vel,
                                   double* grad_body_force, double* grad_tau, void* grad_f0);
+/* Frees the device memory kept from the handle's windows, for others on the GPU. */
+lbdem_status lbdem_adjoint_release(lbdem_handle* h);
 /* Device time of the last lbdem_adjoint_window: forward pass and backward
  * pass (segment recomputation + adjoint steps), CUDA events. */
 lbdem_status lbdem_adjoint_timing(lbdem_handle* h, float* forward_ms, float* backward_ms);

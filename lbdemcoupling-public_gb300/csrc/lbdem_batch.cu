@@ -127,7 +127,7 @@ template <typename P>
 cudaError_t dalloc(lbdem_batch* b, P** p, size_t bytes) {
     void* q = nullptr;
     if (alloc_should_fail()) return cudaErrorMemoryAllocation;
-    cudaError_t e = cudaMalloc(&q, bytes == 0 ? 16 : bytes);
+    cudaError_t e = device_malloc(&q, bytes == 0 ? 16 : bytes);
     if (e == cudaSuccess) {
         *p = (P*)q;
         b->dev_bytes += bytes;
@@ -334,9 +334,9 @@ lbdem_status autotune(lbdem_batch* b) {
         if (e0) cudaEventDestroy(e0);
         if (e1) cudaEventDestroy(e1);
     };
-    cudaError_t e = cudaMalloc(&fcopy, fbytes);
-    if (e == cudaSuccess) e = cudaMalloc((void**)&ftcopy, ftbytes);
-    if (e == cudaSuccess) e = cudaMalloc(&dcopy, sizeof(CollideArgs<T>) * 2 * (size_t)b->ndom);
+    cudaError_t e = device_malloc(&fcopy, fbytes);
+    if (e == cudaSuccess) e = device_malloc((void**)&ftcopy, ftbytes);
+    if (e == cudaSuccess) e = device_malloc(&dcopy, sizeof(CollideArgs<T>) * 2 * (size_t)b->ndom);
     if (e == cudaSuccess) e = cudaEventCreate(&e0);
     if (e == cudaSuccess) e = cudaEventCreate(&e1);
     if (e == cudaSuccess) e = cudaMemcpyAsync(fcopy, b->f, fbytes, cudaMemcpyDeviceToDevice, b->stream);

@@ -1,6 +1,7 @@
 // C ABI of liblbdem_gb300: handle life cycle, device memory, staging buffers
 // and the launch sequence of one coupling cycle.  See include/lbdem_gpu.h.
 #include "lbdem_gpu.h"
+#include "kept_memory.h"
 #include "lbdem_internal.h"
 
 #include <sys/mman.h>
@@ -20,6 +21,26 @@ using namespace lbdem;
 
 namespace lbdem {
 std::atomic<int> g_alloc_fail_countdown{0};
+
+namespace {
+// Kept between adjoint windows: allocating and releasing 2.2 GB took 2 ms of a 10 ms window
+// at 128^3.  (Never destroyed: handles may outlive the static objects.)
+KeptMemory& kept() {
+    static KeptMemory* const k = new KeptMemory((size_t)4 << 30);
+    return *k;
+}
+void free_block(void* p) { cudaFree(p); }
+}  // namespace
+
+cudaError_t device_malloc(void** p, size_t bytes) {
+    cudaError_t e = cudaMalloc(p, bytes);
+    if (e == cudaErrorMemoryAllocation) {
+        int device = 0;
+        cudaGetLastError();
+        if (cudaGetDevice(&device) == cudaSuccess && kept().give_back(device, free_block)) e = cudaMalloc(p, bytes);
+    }
+    return e;
+}
 
 void populate_host(void* p, size_t bytes) {
 #ifndef MADV_POPULATE_WRITE
@@ -111,8 +132,6 @@ struct lbdem_handle {
     size_t dev_bytes = 0;
 
     float adj_fwd_ms = 0.f, adj_bwd_ms = 0.f;
-    void* adj_ws = nullptr;     // adjoint window memory kept for the next window
-    size_t adj_bytes = 0;
 
     int n_cur = 0;
     int64_t step = 0;
@@ -155,7 +174,7 @@ template <typename P>
 cudaError_t dalloc(lbdem_handle* h, P** p, size_t bytes) {
     void* q = nullptr;
     if (alloc_should_fail()) return cudaErrorMemoryAllocation;
-    cudaError_t e = cudaMalloc(&q, bytes == 0 ? 16 : bytes);
+    cudaError_t e = device_malloc(&q, bytes == 0 ? 16 : bytes);
     if (e == cudaSuccess) {
         *p = (P*)q;
         h->dev_bytes += bytes;
@@ -167,7 +186,7 @@ void release(lbdem_handle* h) {
     void* dev[] = {h->f, h->vox, h->up, h->cf, h->btab, h->btabf, h->rec2[0], h->rec2[1], h->d_sph, h->d_fast, h->d_xpf,
                    h->map2[0], h->map2[1],
                    h->d_tile_cnt, h->d_bins, h->d_work, h->d_work_n, h->d_err, h->d_mass, h->scratch, h->d_jobs, h->d_pavg,
-                   h->d_ppart, h->d_pcount, h->adj_ws};
+                   h->d_ppart, h->d_pcount, kept().take(h).p};
     for (void* p : dev)
         if (p) cudaFree(p);
     void* host[] = {h->h_rec, h->h_err, h->h_pavg};
@@ -185,17 +204,7 @@ lbdem_status ensure_scratch(lbdem_handle* h, size_t bytes) {
         h->scratch = nullptr;
         h->scratch_bytes = 0;
     }
-    cudaError_t e = dalloc(h, &h->scratch, bytes);
-    if (e == cudaErrorMemoryAllocation && h->adj_ws) {   // give the kept adjoint memory back first
-        cudaGetLastError();
-        cudaStreamSynchronize(h->stream);
-        cudaFree(h->adj_ws);
-        h->dev_bytes -= h->adj_bytes;
-        h->adj_ws = nullptr;
-        h->adj_bytes = 0;
-        e = dalloc(h, &h->scratch, bytes);
-    }
-    CK(h, e);
+    CK(h, dalloc(h, &h->scratch, bytes));
     h->scratch_bytes = bytes;
     return LBDEM_OK;
 }
@@ -786,7 +795,7 @@ lbdem_status lbdem_get_step(lbdem_handle* h, int64_t* step) {
 
 lbdem_status lbdem_device_bytes(lbdem_handle* h, size_t* bytes) {
     if (!h || !bytes) return LBDEM_ERR_INVALID_ARG;
-    *bytes = h->dev_bytes;
+    *bytes = h->dev_bytes + kept().held(h);
     return LBDEM_OK;
 }
 
@@ -914,42 +923,34 @@ lbdem_status lbdem_init_profile(lbdem_handle* h, int32_t kind, double rho_hi, do
 
 namespace {
 
-// One adjoint window's device memory, in one block that the handle keeps for the next
-// window up to ADJ_KEEP_BYTES (allocating and releasing 2.2 GB took 2 ms of a 10 ms
-// window at 128^3); a larger one is released when the window ends.
-constexpr size_t ADJ_KEEP_BYTES = (size_t)4 << 30;
+// One adjoint window's device memory, in one block that stays with the handle for the next
+// window where kept() takes it.
 struct AdjointBuffers {
     lbdem_handle* h;
+    KeptMemory::Block block;
     size_t used = 0;
-    explicit AdjointBuffers(lbdem_handle* handle) : h(handle) {}
+    explicit AdjointBuffers(lbdem_handle* handle) : h(handle), block(kept().take(handle)) {}
     ~AdjointBuffers() {
-        if (h->adj_bytes > ADJ_KEEP_BYTES) drop();
-    }
-    void drop() {
-        if (h->adj_ws) {
-            cudaStreamSynchronize(h->stream);
-            cudaFree(h->adj_ws);
-            h->dev_bytes -= h->adj_bytes;
-        }
-        h->adj_ws = nullptr;
-        h->adj_bytes = 0;
+        if (!block.p) return;
+        cudaStreamSynchronize(h->stream);   // (an early return leaves work queued)
+        if (!kept().keep(block)) cudaFree(block.p);
     }
     static size_t rounded(size_t bytes) { return (bytes + 255) / 256 * 256; }
     cudaError_t reserve(size_t bytes) {
-        if (h->adj_bytes >= bytes) return cudaSuccess;
-        drop();
-        const cudaError_t e = cudaMalloc(&h->adj_ws, bytes);
+        if (block.bytes >= bytes) return cudaSuccess;
+        if (block.p) cudaFree(block.p);
+        block = KeptMemory::Block{};
+        const cudaError_t e = device_malloc(&block.p, bytes);
         if (e != cudaSuccess) {
-            h->adj_ws = nullptr;
+            block.p = nullptr;
             return e;
         }
-        h->adj_bytes = bytes;
-        h->dev_bytes += bytes;
+        block = KeptMemory::Block{block.p, bytes, h->device, h};
         return cudaSuccess;
     }
     template <typename P>
     void get(P** p, size_t bytes) {
-        *p = (P*)((char*)h->adj_ws + used);
+        *p = (P*)((char*)block.p + used);
         used += rounded(bytes);
     }
 };
@@ -1153,6 +1154,14 @@ lbdem_status lbdem_adjoint_window(lbdem_handle* h, int32_t nsteps, int32_t K, in
         std::snprintf(msg, sizeof(msg), "device error word 0x%x", *h->h_err);
         return fail(h, LBDEM_ERR_DEVICE, msg);
     }
+    return LBDEM_OK;
+}
+
+lbdem_status lbdem_adjoint_release(lbdem_handle* h) {
+    if (!h) return LBDEM_ERR_INVALID_ARG;
+    DeviceGuard dg(h->device);
+    const KeptMemory::Block b = kept().take(h);
+    if (b.p) CK(h, cudaFree(b.p));
     return LBDEM_OK;
 }
 

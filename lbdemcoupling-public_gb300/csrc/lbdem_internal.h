@@ -295,6 +295,10 @@ inline bool alloc_should_fail() {
     return false;
 }
 
+// cudaMalloc on the current device; where it runs out of memory, what handles keep there
+// between calls (kept_memory.h) is freed and the allocation tried again.
+cudaError_t device_malloc(void** p, size_t bytes);
+
 // Makes the pages of a host buffer that a device-to-host copy is about to fill present.
 // The GPU reads and writes pageable host memory through the host's page tables, so a copy
 // into memory that was never touched (a fresh numpy array) faults page by page, 39 us

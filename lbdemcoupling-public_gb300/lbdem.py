@@ -114,6 +114,7 @@ SIGNATURES = {
     "lbdem_save_state": (C.c_int, [_P, C.c_char_p]),
     "lbdem_load_state": (C.c_int, [_P, C.c_char_p]),
     "lbdem_adjoint_window": (C.c_int, [_P, _I, _I, _I, _D, _D, _D, _D, _D, _D, _P]),
+    "lbdem_adjoint_release": (C.c_int, [_P]),
     "lbdem_adjoint_timing": (C.c_int, [_P, C.POINTER(C.c_float), C.POINTER(C.c_float)]),
     "lbdem_batch_config_default": (None, [C.POINTER(BatchConfig)]),
     "lbdem_batch_create": (C.c_int, [C.POINTER(BatchConfig), _I, C.POINTER(Domain), C.POINTER(_P)]),
@@ -393,6 +394,10 @@ class Lattice:
         if want_f0:
             out["grad_f0"] = f0
         return out
+
+    def adjoint_release(self):
+        """Frees the device memory kept from the windows, for others on the GPU."""
+        self._check(self.lib.lbdem_adjoint_release(self.h))
 
     def adjoint_timing(self):
         a, b = C.c_float(), C.c_float()
