@@ -9,6 +9,7 @@
 
 #include <cstddef>
 #include <mutex>
+#include <new>
 #include <vector>
 
 namespace lbdem {
@@ -35,13 +36,18 @@ public:
             }
         return Block{};
     }
-    // Keeps a block; false (the caller frees it) when that would be more than `most` in all.
+    // Keeps a block; false (the caller frees it) when that would be more than `most` in all,
+    // or the host has no memory for the entry.
     bool keep(const Block& b) {
         std::lock_guard<std::mutex> lock(mutex_);
         size_t sum = b.bytes;
         for (const Block& k : idle_) sum += k.bytes;
         if (sum > most_) return false;
-        idle_.push_back(b);
+        try {
+            idle_.push_back(b);
+        } catch (const std::bad_alloc&) {
+            return false;
+        }
         return true;
     }
     size_t held(const void* owner) {

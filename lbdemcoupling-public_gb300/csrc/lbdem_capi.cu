@@ -26,7 +26,8 @@ namespace {
 // Kept between adjoint windows: allocating and releasing 2.2 GB took 2 ms of a 10 ms window
 // at 128^3.  (Never destroyed: handles may outlive the static objects.)
 KeptMemory& kept() {
-    static KeptMemory* const k = new KeptMemory((size_t)4 << 30);
+    alignas(KeptMemory) static unsigned char room[sizeof(KeptMemory)];
+    static KeptMemory* const k = new (room) KeptMemory((size_t)4 << 30);
     return *k;
 }
 void free_block(void* p) { cudaFree(p); }
