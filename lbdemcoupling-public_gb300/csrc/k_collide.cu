@@ -1846,8 +1846,8 @@ k_collide_direct(const CollideArgs<float> a1, long long nseg, const CollideArgs<
         }
         if (a.cf) {
             const float2 fx = upk(o.Fx), fy = upk(o.Fy), fz = upk(o.Fz);
-            if (valid[0]) { a.cf[c[0].own] = fx.x; a.cf[N + c[0].own] = fy.x; a.cf[2ull * N + c[0].own] = fz.x; }
-            if (valid[1]) { a.cf[c[1].own] = fx.y; a.cf[N + c[1].own] = fy.y; a.cf[2ull * N + c[1].own] = fz.y; }
+            if (valid[0]) { a.cf[c[0].own] = fx.x; a.cf[(size_t)N + c[0].own] = fy.x; a.cf[2 * (size_t)N + c[0].own] = fz.x; }
+            if (valid[1]) { a.cf[c[1].own] = fx.y; a.cf[(size_t)N + c[1].own] = fy.y; a.cf[2 * (size_t)N + c[1].own] = fz.y; }
         }
         if (PLANE) {
             forces_by_cell(a, g, o, x, c[0].y, c[0].z, c[1].y, c[1].z, false);
