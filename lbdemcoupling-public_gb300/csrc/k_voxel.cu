@@ -645,7 +645,9 @@ __device__ __forceinline__ void voxelize_tile(WarpVox<INIT_VEL>& S, int t, const
     int b = (cnt <= TILE_BIN && lane + 32 < cnt) ? b0 : INT_MAX;
     if (cnt <= 0) return;   // (a listed tile has a sphere)
     // the bins are reused by the next voxelization: the count is zeroed by the last of
-    // the tile's warps to have read it (arrivals in the bits above TILE_CNT_MASK)
+    // the tile's warps to have read it (arrivals in the bits above TILE_CNT_MASK; a warp
+    // arrives when every lane of it has)
+    __syncwarp();
     if (lane == 0) {
         if (parts == 1 || atomicAdd((unsigned*)(tile_cnt + t), TILE_CNT_MASK + 1u) >> TILE_CNT_BITS == parts - 1u)
             tile_cnt[t] = 0;
