@@ -334,7 +334,7 @@ lbdem_status lbdem_voxelize_static(int32_t nx, int32_t ny, int32_t nz, int32_t p
  * On return the handle holds the state after the window and the forces of its
  * last step.  Not available with a pressure drop set (not differentiated).
  * The window's device memory (checkpoints, tape, adjoint populations) stays with
- * the handle for its next window, at most 4 GB over all handles; it is given
+ * the handle for its next window, at most 4 GB, and 16 GB over all handles; it is given
  * back when an allocation of this library on the device would fail without it,
  * by lbdem_adjoint_release, and with the handle. */
 lbdem_status lbdem_adjoint_window(lbdem_handle* h, int32_t nsteps, int32_t checkpoint_every, int32_t n,

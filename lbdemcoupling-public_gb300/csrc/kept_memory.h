@@ -1,6 +1,6 @@
 // Device memory that handles keep between calls (the adjoint window's buffers).
 //
-// At most `most` bytes are kept in the process, a block per owner; a block is out of here
+// A block per owner of at most `each` bytes, `all` bytes in the process; a block is out of here
 // while its owner works in it, and its work has finished when it comes back.  So an idle
 // block can be freed at any time, from any thread: by its owner, or by an allocation of any
 // handle on the device that would fail otherwise.  The freeing stands under the lock, so that
@@ -23,7 +23,7 @@ public:
         const void* owner = nullptr;
     };
 
-    explicit KeptMemory(size_t most) : most_(most) {}
+    KeptMemory(size_t each, size_t all) : each_(each), all_(all) {}
 
     // The owner's idle block, which leaves here (p == nullptr: none).
     Block take(const void* owner) {
@@ -36,13 +36,13 @@ public:
             }
         return Block{};
     }
-    // Keeps a block; false (the caller frees it) when that would be more than `most` in all,
-    // or the host has no memory for the entry.
+    // Keeps a block; false (the caller frees it) when that would be too much, or the host has
+    // no memory for the entry.
     bool keep(const Block& b) {
         std::lock_guard<std::mutex> lock(mutex_);
         size_t sum = b.bytes;
         for (const Block& k : idle_) sum += k.bytes;
-        if (sum > most_) return false;
+        if (b.bytes > each_ || sum > all_) return false;
         try {
             idle_.push_back(b);
         } catch (const std::bad_alloc&) {
@@ -72,7 +72,7 @@ public:
     }
 
 private:
-    const size_t most_;
+    const size_t each_, all_;
     std::mutex mutex_;
     std::vector<Block> idle_;
 };

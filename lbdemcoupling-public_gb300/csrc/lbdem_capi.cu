@@ -24,10 +24,10 @@ std::atomic<int> g_alloc_fail_countdown{0};
 
 namespace {
 // Kept between adjoint windows: allocating and releasing 2.2 GB took 2 ms of a 10 ms window
-// at 128^3.  (Never destroyed: handles may outlive the static objects.)
+// at 128^3.  4 GB a handle, 16 GB for a program that goes through several.  (Never destroyed: handles may outlive the static objects.)
 KeptMemory& kept() {
     alignas(KeptMemory) static unsigned char room[sizeof(KeptMemory)];
-    static KeptMemory* const k = new (room) KeptMemory((size_t)4 << 30);
+    static KeptMemory* const k = new (room) KeptMemory((size_t)4 << 30, (size_t)16 << 30);
     return *k;
 }
 void free_block(void* p) { cudaFree(p); }

@@ -19,10 +19,11 @@ int main() {
     int freed = 0;
     const auto drop = [&](void*) { ++freed; };
     char mem[8];
-    KeptMemory k(100);
+    KeptMemory k(70, 100);
     int a = 0, b = 0, c = 0;
     check(k.take(&a).p == nullptr, "nothing kept at first");
-    check(k.keep({mem, 60, 0, &a}), "a block within the bound");
+    check(!k.keep({mem, 71, 0, &a}), "the bound of one block");
+    check(k.keep({mem, 60, 0, &a}), "a block within the bounds");
     check(!k.keep({mem + 1, 41, 0, &b}), "the bound holds over all owners");
     check(k.keep({mem + 1, 40, 1, &b}), "up to the bound");
     check(k.held(&a) == 60 && k.held(&b) == 40 && k.held(&c) == 0, "held bytes");
@@ -34,7 +35,7 @@ int main() {
     check(k.take(&b).bytes == 40 && !k.give_back(1, drop), "empty again");
     // owners on several threads, and one that gives back: every block is freed once
     static int alive[4] = {0, 0, 0, 0};
-    KeptMemory t(1000);
+    KeptMemory t(1000, 1000);
     std::thread work[5];
     for (int n = 0; n < 4; ++n)
         work[n] = std::thread([n, &t] {
