@@ -12,13 +12,14 @@
 // field emax, E = emax - 1022) the unit is 2^(E - 57) = 2^(emax - 1079): a
 // population is below 2^57 units, the sums of 19 populations are exact and below
 // 2^62, and the largest population's last mantissa bit is 16 units.  Products
-// are rounded to the unit (error at most 1.5 units: the low x low partial product is
-// left out), so that a result carries an error of a few units, an eighth to a
-// quarter of the largest population's last bit, and then its own rounding to
-// double.  Double arithmetic rounds at every one of its operations; both errors
-// are measured against 113-bit arithmetic in tests/test_cell_fixed_cpu.py.
+// are rounded to the unit (mul<S>: error at most 2^(62 - S) units for the low x low
+// partial product that is left out, and half a unit: 1.5 units for S = 62, 2.5 for 61), and a
+// result then once to double.  Double arithmetic rounds at every one of its operations; both
+// errors are measured against 113-bit arithmetic in tests/test_cell_fixed_cpu.py (a result is
+// off by a third of what the double update is).
 //
-// Range.  2^E <= 2^-5 (|f_i| < 1/32, hence |rhoBar| < 0.6) and surface velocities
+// Range.  2^E <= 2^-5 (|f_i| < 1/32, hence |rhoBar| < 0.6; a fluid at rest reaches it at
+// |rhoBar| = 0.094, where f_0 = rhoBar / 3 does) and surface velocities and body forces
 // below 2^(E + 3) (they raise E if need be: below 1/4); non-zero cells below
 // 2^-958 are left out too.  A cell outside the range, or with a NaN or infinity,
 // takes the double routine: fits() tells, from the cell's own values alone.

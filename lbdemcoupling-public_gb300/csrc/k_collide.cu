@@ -1916,7 +1916,8 @@ struct StagedCell {
 };
 
 // The double routine for a cell outside the fixed-point range, out of line.  SOLID false: for
-// the lanes of a warp without solid cells.
+// the lanes of a warp without solid cells (128^3 fluid of density 1.12: 550 us a step, 1076
+// with the solid terms; with a body force both forms run them for solid cells only).
 template <bool FORCE, bool SOLID, typename Cell>
 __device__ __noinline__ void collide_cell_double(Cell s, double omega, double g0,
                                                  double g1, double g2, int n, double B, double u0, double u1,
